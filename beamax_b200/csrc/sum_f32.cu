@@ -40,14 +40,22 @@ constexpr int GS = 16;               // sensors per warp group and maximal run l
 constexpr int NW = 8;                // warps per CTA (forward)
 constexpr int TS = GS * NW;          // sensors per tile
 constexpr int THREADS = NW * 32;
-constexpr int G = THREADS / TT;      // beams per record pass
-static_assert(G % 2 == 0, "beams are evaluated in pairs");
+// Beams per record pass.  Every warp then evaluates only the beams that reach
+// its own sensor group (about a quarter to a half of them), so the pass has to
+// be long enough for the warps' shares to even out between the barriers: 8
+// beams per pass left the warps idle there, 32 is the most that two CTAs' records
+// (80 KB each in 3D) leave room for on an SM.
+constexpr int G = 32;
+static_assert(G == 32, "a warp's share of a pass is one 32-bit mask");
 constexpr float kTwoPi = 6.283185307179586f;
 constexpr float kInvTwoPi = 0.15915494309189535f;
 
-// Reduce an FP32 angle to [-pi, pi] (bounded inputs).
+// Reduce an FP32 angle to [-pi, pi] (bounded inputs, |th| < 2^22 turns).  The
+// nearest integer comes from adding 1.5 * 2^23 on the FMA pipe: rintf runs on
+// the MUFU pipe, which the seeds' sin/cos/exp already fill (a complex
+// exponential measured 25.4 cycles per warp and scheduler instead of 32.8).
 __device__ __forceinline__ float reduce_angle(float th) {
-    const float k = rintf(th * kInvTwoPi);
+    const float k = __fadd_rn(fmaf(th, kInvTwoPi, 12582912.0f), -12582912.0f);
     return fmaf(-k, kTwoPi, th);
 }
 
@@ -68,10 +76,6 @@ __device__ __forceinline__ cf csqrtf_(cf z) {
     if (z.re >= 0.0f) return cf{r, z.im / (2.0f * r)};
     return cf{fabsf(z.im) / (2.0f * r), copysignf(r, z.im)};
 }
-#ifndef MSGB_F32X2
-#define MSGB_F32X2 1
-#endif
-#if MSGB_F32X2
 // Two complex numbers, component-packed, for the paired FP32 instructions of
 // sm_100 (FFMA2 / FMUL2 / FADD2).  Each lane of a paired operation rounds
 // exactly as the scalar instruction, so these produce the same bits as cmul
@@ -90,7 +94,6 @@ __device__ __forceinline__ void kahan_add2(float2 &acc, float2 &cmp, float2 v) {
     acc = t;
 }
 __device__ __forceinline__ cf2 pack2(cf a, cf b) { return cf2{make_float2(a.re, b.re), make_float2(a.im, b.im)}; }
-#endif
 
 // exp(x + i y) with y range-reduced first.
 __device__ __forceinline__ cf cexpf_(float x, float y) {
@@ -297,16 +300,31 @@ constexpr float kRecurrenceEfolds = 60.0f;
 // culling is enabled, cutoff > 0).
 constexpr float kNegligibleEfolds = 40.0f;
 
-enum RunKind { kRunRecurrence = 0, kRunNegligible = 1, kRunDirect = 2 };
+// Margin, in e-folds beyond the cutoff, of the per-group test: a (beam, time
+// tile) whose smallest exponent over a group of GS sensors and the 32 times is
+// larger than cutoff + margin is left out for that group.  The tile test
+// (survives, traj_survives) bounds the exponent with the smallest eigenvalue of
+// Im M and a box around 128 sensors, so most of what it keeps lies far outside the
+// beam: at 1024^2 heterogeneous 67 % of the (beam, group) pairs it kept were
+// beyond 24 e-folds, 33 % at 512^2 homogeneous, 56 % at 128^3.
+constexpr float kGroupMarginEfolds = 8.0f;
 
-// Direct evaluation at a run start (seed): z, and the recurrence factors for
-// the step h to the next sensor.  With `kind`, classifies the run of GS
-// sensors (RunKind): the exponent along it is chi(k) = chi + B k + A k^2 with
-// B = -a1r, A = -a2r.
+// One warp's sensor group: its straight run's start and step.
+template <int D>
+struct Run {
+    float ds[D], h[D];
+};
+
+// Smallest exponent chi(k) = chi + B k + A k^2 over k in [0, GS - 1].
+__device__ __forceinline__ float run_chi_min(float chi, float Bq, float Aq) {
+    constexpr float kl = (float)(GS - 1);
+    const float kv = Aq > 0.0f ? fminf(fmaxf(__fdividef(-0.5f * Bq, Aq), 0.0f), kl) : 0.0f;
+    return fminf(fminf(chi, fmaf(kl, fmaf(Aq, kl, Bq), chi)), fmaf(kv, fmaf(Aq, kv, Bq), chi));
+}
+
+// Direct evaluation at sensor offset ds: z.
 template <int D, bool PERIODIC>
-__device__ __forceinline__ cf seed_eval(const Rec<D> &r, const float *ds, const float *h, bool cont,
-                                        const ProbArgs &P, cf &rr, cf &qq, int *kind = nullptr,
-                                        bool skip_negligible = false) {
+__device__ __forceinline__ cf direct_eval(const Rec<D> &r, const float *ds, const ProbArgs &P) {
     float Dl[D];
     float th = r.th0;
 #pragma unroll
@@ -316,32 +334,38 @@ __device__ __forceinline__ cf seed_eval(const Rec<D> &r, const float *ds, const 
         th = fmaf(r.wp[i], ds[i], th);
     }
     th += quad<D>(r.q, Dl);
+    cf z = cexpf_(-quad<D>(r.p, Dl), th);
+    return cf{z.re * r.amp, z.im * r.amp};
+}
+
+// Run start: z, the ratio f to the next sensor and the ratio's own step q.
+// Returns true when the run has to be evaluated directly (z = f = q = 0 then):
+// its factors would leave FP32's range and some sensor of it is not negligible.
+template <int D>
+__device__ __forceinline__ bool seed_eval(const Rec<D> &r, const Run<D> &g, bool skip_negligible, cf &z, cf &f, cf &q) {
+    float Dl[D];
+    float th = r.th0, wh = 0.0f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+        Dl[i] = g.ds[i] + r.d0[i];
+        th = fmaf(r.wp[i], g.ds[i], th);
+        wh = fmaf(r.wp[i], g.h[i], wh);
+    }
+    th += quad<D>(r.q, Dl);
     const float chi = quad<D>(r.p, Dl);
-    cf z = cexpf_(-chi, th);
+    z = cexpf_(-chi, th);
     z.re *= r.amp;
     z.im *= r.amp;
-    if (cont) {
-        float wh = 0.0f;
-#pragma unroll
-        for (int i = 0; i < D; ++i) wh = fmaf(r.wp[i], h[i], wh);
-        const float a1r = -bilin2<D>(r.p, h, Dl), a1i = wh + bilin2<D>(r.q, h, Dl);
-        const float a2r = -quad<D>(r.p, h), a2i = quad<D>(r.q, h);
-        rr = cexpf_(a1r + a2r, a1i + a2i);
-        qq = cexpf_(2.0f * a2r, 2.0f * a2i);
-        if (kind) {
-            const float Aq = -a2r, Bq = -a1r;
-            const float kv = Aq > 0.0f ? fminf(fmaxf(-Bq / (2.0f * Aq), 0.0f), (float)(GS - 1)) : 0.0f;
-            const float kl = (float)(GS - 1);
-            const float chi_min = fminf(fminf(chi, chi + kl * (Bq + Aq * kl)), chi + kv * (Bq + Aq * kv));
-            if (skip_negligible && chi_min > kNegligibleEfolds)
-                *kind = kRunNegligible;
-            else if (chi > kRecurrenceEfolds || a1r + a2r > kRecurrenceEfolds || -2.0f * a2r > kRecurrenceEfolds)
-                *kind = kRunDirect;
-            else
-                *kind = kRunRecurrence;
-        }
+    const float a1r = -bilin2<D>(r.p, g.h, Dl), a1i = wh + bilin2<D>(r.q, g.h, Dl);
+    const float a2r = -quad<D>(r.p, g.h), a2i = quad<D>(r.q, g.h);
+    f = cexpf_(a1r + a2r, a1i + a2i);
+    q = cexpf_(2.0f * a2r, 2.0f * a2i);
+    bool direct = false;
+    if (chi > kRecurrenceEfolds || a1r + a2r > kRecurrenceEfolds || -2.0f * a2r > kRecurrenceEfolds) {
+        direct = !(skip_negligible && run_chi_min(chi, -a1r, -a2r) > kNegligibleEfolds);
+        z = f = q = cf{0.0f, 0.0f};
     }
-    return z;
+    return direct;
 }
 
 template <int D>
@@ -564,14 +588,155 @@ __device__ __forceinline__ void traj_beam_time(const BeamArgs &B, const TrajSrc<
     bt.ang += atan2f(ai, (ar == 0.0f && ai == 0.0f) ? 1e-12f : ar);
 }
 
-// ------------------------------------------------------------------ forward
+// ------------------------------------------------------------------ record passes
+// A record pass holds up to G beams' records at the tile's 32 times in shared
+// memory, rec[field][beam][time], and per beam an 8-bit mask of the warps (sensor
+// groups) it reaches.  Warp w of the pass writes beams w, w + 8, ...: lane = time.
 template <int D>
-__device__ __forceinline__ void load_rec(const float (*rec)[G][TT], int gl, int lane, Rec<D> &r) {
-    float *rf = reinterpret_cast<float *>(&r);
-#pragma unroll
-    for (int f = 0; f < Rec<D>::NF; ++f) rf[f] = rec[f][gl][lane];
+constexpr size_t rec_bytes() {
+    return sizeof(float) * Rec<D>::NF * G * TT;
 }
 
+// Per group of GS sensors, for the test of the record pass: the run's start
+// and step (fast groups: one straight run), or a ball around the sensors.
+template <int D>
+struct GroupInfo {
+    float ds[D], h[D];  // fast: run start and step; else: centre (ds)
+    float rad;          // not fast: largest distance of a sensor from the centre
+    int kind;           // 0 no sensors, 1 fast, 2 not fast, 3 not fast and never left out (periodic)
+};
+
+// Does a record reach group g within thr e-folds (a lower bound on the exponent)?
+template <int D>
+__device__ __forceinline__ bool group_reached(const Rec<D> &r, const GroupInfo<D> &g, float thr) {
+    float Dl[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) Dl[i] = g.ds[i] + r.d0[i];
+    const float chi = quad<D>(r.p, Dl);
+    if (g.kind == 1) return run_chi_min(chi, bilin2<D>(r.p, g.h, Dl), quad<D>(r.p, g.h)) <= thr;
+    // sqrt(chi) is a norm: over the ball it is at least sqrt(chi(centre)) - sqrt(tr P) rad
+    float tr = 0.0f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) tr += r.p[sym_index<D>(i, i)];
+    return sqrtf(fmaxf(chi, 0.0f)) - sqrtf(fmaxf(tr, 0.0f)) * g.rad <= sqrtf(thr);
+}
+
+// Describe the tile's groups (warp w describes group w; sds / shn loaded).
+template <int D>
+__device__ __forceinline__ void describe_group(const float (*sds)[D], const float (*shn)[D], int s_cnt, bool fast,
+                                               bool periodic, GroupInfo<D> *gi) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gbase = warp * GS;
+    const int cnt = min(GS, s_cnt - gbase);
+    float lo[D], hi[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+        lo[i] = hi[i] = sds[gbase][i];
+        for (int k = 1; k < cnt; ++k) lo[i] = fminf(lo[i], sds[gbase + k][i]), hi[i] = fmaxf(hi[i], sds[gbase + k][i]);
+    }
+    if (lane == 0) {
+        GroupInfo<D> g;
+        float r2 = 0.0f;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            g.ds[i] = fast ? sds[gbase][i] : 0.5f * (lo[i] + hi[i]);
+            g.h[i] = shn[gbase][i];
+            const float e = 0.5f * (hi[i] - lo[i]);
+            r2 = fmaf(e, e, r2);
+        }
+        g.rad = sqrtf(r2) * 1.00001f;
+        g.kind = cnt <= 0 ? 0 : (fast ? 1 : (periodic ? 3 : 2));
+        gi[warp] = g;
+    }
+}
+
+// Write the records of the pass's beams idx[0 .. nb) and their masks alive[].
+// load(b, bt): the tile-independent part of beam b at this lane's time.
+template <int D, typename Load>
+__device__ __forceinline__ void record_pass(const ProbArgs &P, const int32_t *idx, int nb, int t_cnt, const TileInfo<D> &ti,
+                                            const GroupInfo<D> *gi, float thr, float *rec, uint8_t *alive,
+                                            const Load &load) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool tv = lane < t_cnt;
+#pragma unroll 1
+    for (int i = warp; i < nb; i += NW) {
+        Rec<D> r;
+#pragma unroll
+        for (int k = 0; k < D; ++k) r.d0[k] = r.wp[k] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = r.p[q] = 0.0f;
+        r.th0 = r.amp = 0.0f;
+        if (tv) {
+            BeamTime<D> bt;
+            load(idx[i], bt);
+            anchor<D>(P, bt, ti.s0, r);
+        }
+        unsigned m = 0;
+#pragma unroll
+        for (int g = 0; g < NW; ++g) {
+            const GroupInfo<D> &q = gi[g];
+            if (q.kind == 0) continue;
+            const bool in = tv && (thr <= 0.0f || q.kind == 3 || group_reached<D>(r, q, thr));
+            if (__any_sync(0xffffffffu, in)) m |= 1u << g;
+        }
+        if (m) {
+            const float *rf = reinterpret_cast<const float *>(&r);
+#pragma unroll
+            for (int f = 0; f < Rec<D>::NF; ++f) rec[(f * G + i) * TT + lane] = rf[f];
+        }
+        if (lane == 0) alive[i] = (uint8_t)m;
+    }
+}
+
+template <int D>
+__device__ __forceinline__ void load_rec(const float *rec, int i, int lane, Rec<D> &r) {
+    float *rf = reinterpret_cast<float *>(&r);
+#pragma unroll
+    for (int f = 0; f < Rec<D>::NF; ++f) rf[f] = rec[(f * G + i) * TT + lane];
+}
+
+// Seeds of beams i0 and i1 (i1 < 0: none) as one pair; bit 0 / 1 of the
+// result: this lane has to evaluate beam i0 / i1 directly.
+template <int D>
+__device__ __forceinline__ int seed_pair(const float *rec, int i0, int i1, int lane, const Run<D> &g, bool skip, cf2 &z,
+                                         cf2 &f, cf2 &q) {
+    cf za, fa, qa, zb{0.0f, 0.0f}, fb{0.0f, 0.0f}, qb{0.0f, 0.0f};
+    Rec<D> r;
+    load_rec<D>(rec, i0, lane, r);
+    int direct = seed_eval<D>(r, g, skip, za, fa, qa) ? 1 : 0;
+    if (i1 >= 0) {
+        load_rec<D>(rec, i1, lane, r);
+        direct |= seed_eval<D>(r, g, skip, zb, fb, qb) ? 2 : 0;
+    }
+    z = pack2(za, zb);
+    f = pack2(fa, fb);
+    q = pack2(qa, qb);
+    return direct;
+}
+
+__device__ __forceinline__ int take_bit(unsigned &bits) {
+    const int i = __ffs((int)bits) - 1;  // -1 when none is left
+    bits &= bits - 1u;
+    return i;
+}
+
+// Exclusive offset of this warp's entry (row k of NROW) in the CTA-wide order
+// (row, warp), from the per-warp counts cnt[row * NW + warp]; total in tot.
+template <int NROW>
+__device__ __forceinline__ int scan_counts(const int *cnt, int row, int warp, int &tot) {
+    static_assert(NROW * NW <= 32, "one count per lane");
+    const int lane = threadIdx.x & 31;
+    const int v = lane < NROW * NW ? cnt[lane] : 0;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    tot = __shfl_sync(0xffffffffu, x, 31);
+    return __shfl_sync(0xffffffffu, x - v, row * NW + warp);
+}
+
+// ------------------------------------------------------------------ forward
 __device__ __forceinline__ void kahan_add(float &acc, float &cmp, float v) {
     const float y = v - cmp;
     const float t = acc + y;
@@ -579,24 +744,34 @@ __device__ __forceinline__ void kahan_add(float &acc, float &cmp, float v) {
     acc = t;
 }
 
+constexpr int SCAN = 4;  // beams tested per thread and scan
+
 // Persistent CTAs take (time tile, sensor tile) work items from a counter.
 // Warp w owns sensor group w (GS sensors) of the tile; lane l owns time l.
-// Beams are evaluated two at a time (independent recurrence chains).
+// Per item: beams are scanned 1024 at a time against the tile (survives /
+// traj_survives), survivors queue up, and every G of them make a record pass;
+// then each warp evaluates the pass's beams that reach its group, four at a
+// time (two independent paired recurrences; the four values of a sensor are
+// added before one compensated addition).
+//
+// Bound: FP32 pipe (recurrence 8 FMA-pipe operations per triple, seed ~75 per 16
+// triples) with the seeds' MUFU work beside it.
 template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
 fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *tiles, const int32_t *offs,
-             const float *ds_g, const float *hn_g, const uint8_t *seed_g, const uint8_t *gfast_g,
-             const int32_t *perm, float cutoff, float *out, unsigned long long *eval_count, int *work, int n_st,
-             int n_tiles, TrajSrc<D> T) {
-    constexpr int NF = Rec<D>::NF;
-    __shared__ float rec[NF][G][TT];
+             const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const int32_t *perm, float cutoff,
+             float *out, unsigned long long *eval_count, int *work, int n_st, int n_tiles, TrajSrc<D> T) {
+    extern __shared__ float rec[];  // rec_bytes<D>()
     __shared__ float sds[TS][D], shn[TS][D];
-    __shared__ uint8_t sseed[TS + 1];
-    __shared__ int64_t surv[2 * THREADS];
-    __shared__ int warp_cnt[NW];
-    __shared__ int tile_s, nsurv_s;
+    __shared__ GroupInfo<D> ginfo[NW];
+    __shared__ int32_t surv[2 * SCAN * THREADS + G];
+    __shared__ int warp_cnt[SCAN * NW];
+    __shared__ uint8_t alive[G];
+    __shared__ int tile_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float thr = cutoff > 0.0f ? cutoff + kGroupMarginEfolds : 0.0f;
+    const bool skip = cutoff > 0.0f;
     unsigned long long evals = 0;
     while (true) {
         if (tid == 0) tile_s = atomicAdd(work, 1);
@@ -615,12 +790,16 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
                 sds[k][i] = k < s_cnt ? ds_g[(s_first + k) * D + i] : 0.0f;
                 shn[k][i] = k < s_cnt ? hn_g[(s_first + k) * D + i] : 0.0f;
             }
-            sseed[k] = k < s_cnt ? seed_g[s_first + k] : 1;
         }
-        if (tid == 0) sseed[TS] = 1;
+        __syncthreads();
         const bool fast = gfast_g[st * NW + warp] != 0;
         const int gbase = warp * GS;
         const bool active = gbase < s_cnt;
+        describe_group<D>(sds, shn, s_cnt, fast, PERIODIC, ginfo);
+        Run<D> run;
+#pragma unroll
+        for (int i = 0; i < D; ++i) run.ds[i] = sds[gbase][i], run.h[i] = shn[gbase][i];
+        const int g_cnt = max(0, min(GS, s_cnt - gbase));
         // Kahan sums of sensors 2h and 2h + 1 in .x and .y
         float2 acc2[GS / 2], cmp2[GS / 2];
 #pragma unroll
@@ -641,133 +820,133 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
             }
         }
         const int64_t nbeam = TRAJ ? T.nb : B.n;
+        int nq = 0;  // queued survivors (the same in every thread)
 
-        for (int64_t j0 = 0; j0 < nbeam; j0 += THREADS) {
-            const int64_t j = j0 + tid;
-            bool keep_p = false, keep_m = false;
-            if (j < nbeam) {
-                if (TRAJ) {
-                    keep_p = traj_survives<D>(T, j, tt, ti, cutoff);
-                } else {
-                    const Cull<D> cb = cull[j];
-                    keep_p = mode_on(B.modes, 0) && survives<D>(cb, (float)P.c, ta, tb, ti, P, cutoff);
-                    keep_m = mode_on(B.modes, 1) && survives<D>(cb, -(float)P.c, ta, tb, ti, P, cutoff);
-                }
-            }
-            const unsigned bp = __ballot_sync(0xffffffffu, keep_p);
-            const unsigned bm = __ballot_sync(0xffffffffu, keep_m);
-            if (lane == 0) warp_cnt[warp] = __popc(bp) + __popc(bm);
-            __syncthreads();
-            int off = 0, tot = 0;
+        for (int64_t j0 = 0; j0 < nbeam; j0 += SCAN * THREADS) {
+            unsigned bp[SCAN], bm[SCAN];
 #pragma unroll
-            for (int w = 0; w < NW; ++w) {
-                if (w < warp) off += warp_cnt[w];
-                tot += warp_cnt[w];
-            }
-            const unsigned lt = (1u << lane) - 1u;
-            if (keep_p) surv[off + __popc(bp & lt)] = j;
-            if (keep_m) surv[off + __popc(bp) + __popc(bm & lt)] = j + B.n;
-            if (tid == 0) nsurv_s = tot;
-            __syncthreads();
-            const int nsurv = nsurv_s;
-            evals += (unsigned long long)nsurv * (unsigned long long)t_cnt * (unsigned long long)s_cnt;
-            for (int g0 = 0; g0 < nsurv; g0 += G) {
-                {
-                    const int gl = tid / TT, tloc = tid % TT;
-                    Rec<D> r;
-                    if (g0 + gl < nsurv && tloc < t_cnt) {
-                        BeamTime<D> bt;
-                        if (TRAJ)
-                            traj_beam_time<D>(B, T, surv[g0 + gl], t_first + tloc, bt);
-                        else
-                            beam_time<D>(P, B, surv[g0 + gl], P.ts[t_first + tloc], bt);
-                        anchor<D>(P, bt, ti.s0, r);
+            for (int k = 0; k < SCAN; ++k) {
+                const int64_t j = j0 + k * THREADS + tid;
+                bool keep_p = false, keep_m = false;
+                if (j < nbeam) {
+                    if (TRAJ) {
+                        keep_p = traj_survives<D>(T, j, tt, ti, cutoff);
                     } else {
-#pragma unroll
-                        for (int i = 0; i < D; ++i) r.d0[i] = 0.0f, r.wp[i] = 0.0f;
-#pragma unroll
-                        for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = 0.0f, r.p[q] = 0.0f;
-                        r.th0 = 0.0f;
-                        r.amp = 0.0f;
+                        const Cull<D> cb = cull[j];
+                        keep_p = mode_on(B.modes, 0) && survives<D>(cb, (float)P.c, ta, tb, ti, P, cutoff);
+                        keep_m = mode_on(B.modes, 1) && survives<D>(cb, -(float)P.c, ta, tb, ti, P, cutoff);
                     }
-                    const float *rf = reinterpret_cast<const float *>(&r);
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) rec[f][gl][tloc] = rf[f];
                 }
+                bp[k] = __ballot_sync(0xffffffffu, keep_p);
+                bm[k] = TRAJ ? 0u : __ballot_sync(0xffffffffu, keep_m);
+                if (lane == 0) warp_cnt[k * NW + warp] = __popc(bp[k]) + __popc(bm[k]);
+            }
+            __syncthreads();
+            int tot = 0;
+            const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+            for (int k = 0; k < SCAN; ++k) {
+                const int off = nq + scan_counts<SCAN>(warp_cnt, k, warp, tot);
+                const int32_t j = (int32_t)(j0 + k * THREADS + tid);
+                if (bp[k] >> lane & 1u) surv[off + __popc(bp[k] & lt)] = j;
+                if (!TRAJ && (bm[k] >> lane & 1u)) surv[off + __popc(bp[k]) + __popc(bm[k] & lt)] = (int32_t)(j + B.n);
+            }
+            nq += tot;
+            __syncthreads();
+            const bool last_scan = j0 + SCAN * THREADS >= nbeam;
+            int g0 = 0;
+            while (nq - g0 >= G || (last_scan && g0 < nq)) {
+                const int nb = min(G, nq - g0);
+                record_pass<D>(P, surv + g0, nb, t_cnt, ti, ginfo, thr, rec, alive, [&](int32_t b, BeamTime<D> &bt) {
+                    if (TRAJ)
+                        traj_beam_time<D>(B, T, b, t_first + lane, bt);
+                    else
+                        beam_time<D>(P, B, b, P.ts[t_first + lane], bt);
+                });
                 __syncthreads();
-                const int ng = min(G, nsurv - g0);
-                if (active) {
-                    for (int gl = 0; gl < ng; gl += 2) {
-                        Rec<D> ra, rb;
-                        load_rec<D>(rec, gl, lane, ra);
-                        load_rec<D>(rec, gl + 1, lane, rb);  // zero-amplitude record when gl + 1 == ng
-                        cf za, fa, qa, zb, fb, qb;
-                        int ka = kRunRecurrence, kb = kRunRecurrence;
-                        if (fast) {
-                            za = seed_eval<D, false>(ra, sds[gbase], shn[gbase], true, P, fa, qa, &ka, cutoff > 0.0f);
-                            zb = seed_eval<D, false>(rb, sds[gbase], shn[gbase], true, P, fb, qb, &kb, cutoff > 0.0f);
-                            if (ka == kRunNegligible) za = fa = qa = cf{0.0f, 0.0f};
-                            if (kb == kRunNegligible) zb = fb = qb = cf{0.0f, 0.0f};
-                        }
-                        if (fast && ka != kRunDirect && kb != kRunDirect) {
-#if MSGB_F32X2
-                            // z_{k+1} = z_k f_k, f_{k+1} = f_k q for both beams in one
-                            // paired instruction stream; sensors 2h, 2h + 1 share a
-                            // paired Kahan update.
-                            cf2 z = pack2(za, zb), f = pack2(fa, fb);
-                            const cf2 q = pack2(qa, qb);
+                unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
+                evals += (unsigned long long)__popc(bits) * (unsigned)(t_cnt * g_cnt);
+                while (bits) {
+                    if (fast) {
+                        const int i0 = take_bit(bits), i1 = take_bit(bits), i2 = take_bit(bits), i3 = take_bit(bits);
+                        cf2 za, fa, qa, zb, fb, qb;
+                        int direct = seed_pair<D>(rec, i0, i1, lane, run, skip, za, fa, qa);
+                        if (i2 >= 0) {
+                            direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+                            // z_{k+1} = z_k f_k, f_{k+1} = f_k q; sensors 2h, 2h + 1
+                            // share a paired compensated addition
 #pragma unroll
                             for (int h = 0; h < GS / 2; ++h) {
                                 if (h > 0) {
-                                    z = cmul2(z, f);
-                                    f = cmul2(f, q);
+                                    za = cmul2(za, fa);
+                                    zb = cmul2(zb, fb);
+                                    fa = cmul2(fa, qa);
+                                    fb = cmul2(fb, qb);
                                 }
-                                const float v0 = z.re.x + z.re.y;
-                                z = cmul2(z, f);
-                                f = cmul2(f, q);
-                                kahan_add2(acc2[h], cmp2[h], make_float2(v0, z.re.x + z.re.y));
+                                const float2 v0 = __fadd2_rn(za.re, zb.re);
+                                za = cmul2(za, fa);
+                                zb = cmul2(zb, fb);
+                                fa = cmul2(fa, qa);
+                                fb = cmul2(fb, qb);
+                                const float2 v1 = __fadd2_rn(za.re, zb.re);
+                                kahan_add2(acc2[h], cmp2[h], make_float2(v0.x + v0.y, v1.x + v1.y));
                             }
-#else
-                            float v[GS];
-                            v[0] = za.re + zb.re;
-#pragma unroll
-                            for (int k = 1; k < GS; ++k) {
-                                za = cmul(za, fa);
-                                fa = cmul(fa, qa);
-                                zb = cmul(zb, fb);
-                                fb = cmul(fb, qb);
-                                v[k] = za.re + zb.re;
-                            }
-#pragma unroll
-                            for (int h = 0; h < GS / 2; ++h) {
-                                kahan_add(acc2[h].x, cmp2[h].x, v[2 * h]);
-                                kahan_add(acc2[h].y, cmp2[h].y, v[2 * h + 1]);
-                            }
-#endif
                         } else {
-                            // Rare (broken runs, out-of-range recurrences): one copy of
-                            // the direct evaluation in a loop, values staged in a small
-                            // array, instead of GS inlined copies (keeps the hot loop
-                            // inside the instruction cache).
-                            cf dummy_r, dummy_q;
-                            float v[GS];
-#pragma unroll 1
-                            for (int k = 0; k < GS; ++k) {
-                                const int s = gbase + k;
-                                const cf za = seed_eval<D, PERIODIC>(ra, sds[s], shn[s], false, P, dummy_r, dummy_q);
-                                const cf zb = seed_eval<D, PERIODIC>(rb, sds[s], shn[s], false, P, dummy_r, dummy_q);
-                                v[k] = za.re + zb.re;
-                            }
 #pragma unroll
                             for (int h = 0; h < GS / 2; ++h) {
-                                kahan_add(acc2[h].x, cmp2[h].x, v[2 * h]);
-                                kahan_add(acc2[h].y, cmp2[h].y, v[2 * h + 1]);
+                                if (h > 0) {
+                                    za = cmul2(za, fa);
+                                    fa = cmul2(fa, qa);
+                                }
+                                const float v0 = za.re.x + za.re.y;
+                                za = cmul2(za, fa);
+                                fa = cmul2(fa, qa);
+                                kahan_add2(acc2[h], cmp2[h], make_float2(v0, za.re.x + za.re.y));
                             }
                         }
+                        if (!__any_sync(0xffffffffu, direct != 0)) continue;
+                        // rare: recurrences out of FP32's range
+#pragma unroll 1
+                        for (int e = 0; e < 4; ++e) {
+                            if (!__any_sync(0xffffffffu, direct >> e & 1)) continue;
+                            Rec<D> r;
+                            load_rec<D>(rec, e == 0 ? i0 : (e == 1 ? i1 : (e == 2 ? i2 : i3)), lane, r);
+                            float v[GS];
+#pragma unroll 1
+                            for (int k = 0; k < GS; ++k)
+                                v[k] = (direct >> e & 1) ? direct_eval<D, false>(r, sds[gbase + k], P).re : 0.0f;
+#pragma unroll
+                            for (int h = 0; h < GS / 2; ++h)
+                                kahan_add2(acc2[h], cmp2[h], make_float2(v[2 * h], v[2 * h + 1]));
+                        }
+                    } else {
+                        // broken runs (sensors off the grid, periodic domains): every
+                        // sensor directly, values staged in a small array (one copy
+                        // of the evaluation in the instruction cache)
+                        const int i0 = take_bit(bits), i1 = take_bit(bits);
+                        Rec<D> ra, rb;
+                        load_rec<D>(rec, i0, lane, ra);
+                        load_rec<D>(rec, i1 >= 0 ? i1 : i0, lane, rb);
+                        if (i1 < 0) rb.amp = 0.0f;
+                        float v[GS];
+#pragma unroll 1
+                        for (int k = 0; k < GS; ++k)
+                            v[k] = direct_eval<D, PERIODIC>(ra, sds[gbase + k], P).re +
+                                   direct_eval<D, PERIODIC>(rb, sds[gbase + k], P).re;
+#pragma unroll
+                        for (int h = 0; h < GS / 2; ++h)
+                            kahan_add2(acc2[h], cmp2[h], make_float2(v[2 * h], v[2 * h + 1]));
                     }
                 }
+                g0 += nb;
                 __syncthreads();
             }
+            if (g0 > 0 && g0 < nq) {  // fewer than G survivors wait for the next scan
+                const int32_t left = tid < nq - g0 ? surv[g0 + tid] : 0;
+                __syncthreads();
+                if (tid < nq - g0) surv[tid] = left;
+            }
+            nq -= g0;
         }
         if (lane < t_cnt && active) {
             const int64_t t = t_first + lane;
@@ -788,7 +967,7 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
         }
         __syncthreads();
     }
-    if (eval_count && tid == 0 && evals) atomicAdd(eval_count, evals);
+    if (eval_count && lane == 0 && evals) atomicAdd(eval_count, evals);
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -798,21 +977,22 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
 // homogeneous entry point j is a selected coefficient and both of its modes
 // are summed; for trajectories j is a beam of the chunk.  Items run tt-major,
 // so consecutive items read the same time tile of the data.  For each sensor
-// tile in order, the CTA loads the tile's positions (shared memory) and data
-// (registers: warp w holds sensor group w, lane l time l), tests the range's
-// beams for survival, and for every pair of surviving beams runs the
-// forward's recurrence while the lane accumulates sum_s d(t, s) conj(z(t, s)).
-// The pair's partials are reduced over the 32 times (FP32 shuffles) and over
-// the 8 warps (FP64), in fixed orders, into the range's per-beam FP64
-// accumulators in shared memory (one owner thread per beam per pass).  The
-// item then writes every accumulator (zeros included) to part[tt][slot], and
-// reduce_parts_kernel sums part over the time tiles in order.  Each partial
-// has one writer and every sum has a fixed order, so the result is
-// bit-identical between runs; the work counter only hands out items.
-constexpr int NACC = 2048;  // accumulator slots (re, im FP64) per item
-
-template <bool TRAJ>
+// tile in order, the CTA tests the range's beams for survival, loads the tile's
+// data (registers: warp w holds sensor group w, lane l time l) and makes
+// record passes as the forward does; each warp runs the forward's recurrence
+// for the beams that reach its group while the lane accumulates
+// sum_s d(t, s) conj(z(t, s)).  The partials are reduced over the 32 times
+// (FP32 shuffles) and over the 8 warps (FP64), in fixed orders, into the range's
+// per-beam FP64 accumulators in shared memory (one owner thread per value and
+// pass).  The item then writes every accumulator (zeros included) to
+// part[tt][slot], and reduce_parts_kernel sums part over the time tiles in
+// order.  Each partial has one writer and every sum has a fixed order, so the
+// result is bit-identical between runs; the work counter only hands out items.
+template <int D, bool TRAJ>
 struct AdjRange {
+    // accumulator slots (re, im FP64) per item; 3D's larger records leave room
+    // for half as many when two CTAs share an SM
+    static constexpr int NACC = D == 3 ? 1024 : 2048;
     static constexpr int RJ = TRAJ ? NACC : NACC / 2;  // beam indices per item
 };
 
@@ -822,20 +1002,24 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
              const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const float *dataT, float cutoff,
              double *part, unsigned long long *eval_count, int *work, int n_st, int n_ranges, int n_items,
              TrajSrc<D> T) {
-    constexpr int NF = Rec<D>::NF;
-    constexpr int RJ = AdjRange<TRAJ>::RJ;
-    __shared__ float rec[NF][G][TT];
+    constexpr int RJ = AdjRange<D, TRAJ>::RJ, NACC = AdjRange<D, TRAJ>::NACC;
+    extern __shared__ double acc_smem[];  // (NACC, 2), then the records
+    float *rec = reinterpret_cast<float *>(acc_smem + 2 * NACC);
     __shared__ float sds[TS][D], shn[TS][D];
-    __shared__ int32_t surv[2 * THREADS];
+    __shared__ GroupInfo<D> ginfo[NW];
+    __shared__ int32_t surv[NACC];  // a range's survivors in one tile (local slots)
     __shared__ int warp_cnt[NW];
-    __shared__ double wpart[NW][G][2];
-    __shared__ int item_s, nsurv_s;
-    extern __shared__ double acc_smem[];  // (NACC, 2)
+    __shared__ float wpart[NW][G][2];
+    __shared__ uint8_t alive2[2][G];
+    __shared__ int item_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t nbeam = TRAJ ? T.nb : B.n;
     const int64_t nslots = TRAJ ? T.nb : 2 * B.n;
+    const float thr = cutoff > 0.0f ? cutoff + kGroupMarginEfolds : 0.0f;
+    const bool skip = cutoff > 0.0f;
     unsigned long long evals = 0;
+    int flip = 0;
     for (int q = tid; q < 2 * NACC; q += THREADS) acc_smem[q] = 0.0;
     while (true) {
         if (tid == 0) item_s = atomicAdd(work, 1);
@@ -853,23 +1037,8 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
             const int s_cnt = offs[st + 1] - offs[st];
             if (s_cnt <= 0) continue;
             const TileInfo<D> ti = tiles[st];
-            __syncthreads();  // the previous tile's passes are done with sds / shn
-            for (int k = tid; k < TS; k += THREADS) {
-#pragma unroll
-                for (int i = 0; i < D; ++i) {
-                    sds[k][i] = k < s_cnt ? ds_g[(s_first + k) * D + i] : 0.0f;
-                    shn[k][i] = k < s_cnt ? hn_g[(s_first + k) * D + i] : 0.0f;
-                }
-            }
-            const bool fast = gfast_g[st * NW + warp] != 0;
-            const int gbase = warp * GS;
-            const bool active = gbase < s_cnt;
-            const float *dcol = dataT + (int64_t)s_first * P.nt + t_first + lane;
-            float dv[GS];
-#pragma unroll
-            for (int k = 0; k < GS; ++k)
-                dv[k] = (tv && gbase + k < s_cnt) ? __ldg(dcol + (int64_t)(gbase + k) * P.nt) : 0.0f;
-
+            // survivors of the range: local slot j - r0 (mode +1 / trajectories), RJ + j - r0 (mode -1)
+            int nq = 0;
             for (int64_t j0 = r0; j0 < r1; j0 += THREADS) {
                 const int64_t j = j0 + tid;
                 bool keep_p = false, keep_m = false;
@@ -883,139 +1052,157 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
                     }
                 }
                 const unsigned bp = __ballot_sync(0xffffffffu, keep_p);
-                const unsigned bm = __ballot_sync(0xffffffffu, keep_m);
+                const unsigned bm = TRAJ ? 0u : __ballot_sync(0xffffffffu, keep_m);
+                __syncthreads();  // warp_cnt and (first trip) the previous tile's surv are done with
                 if (lane == 0) warp_cnt[warp] = __popc(bp) + __popc(bm);
-                __syncthreads();  // also: sds / shn loaded
-                int off = 0, tot = 0;
-#pragma unroll
-                for (int w = 0; w < NW; ++w) {
-                    if (w < warp) off += warp_cnt[w];
-                    tot += warp_cnt[w];
-                }
-                // local slot: beam j - r0 (mode +1 / trajectories), RJ + j - r0 (mode -1)
+                __syncthreads();
+                int tot;
+                const int off = nq + scan_counts<1>(warp_cnt, 0, warp, tot);
                 const unsigned lt = (1u << lane) - 1u;
                 if (keep_p) surv[off + __popc(bp & lt)] = (int32_t)(j - r0);
                 if (keep_m) surv[off + __popc(bp) + __popc(bm & lt)] = (int32_t)(RJ + j - r0);
-                if (tid == 0) nsurv_s = tot;
+                nq += tot;
+            }
+            if (nq == 0) continue;
+            for (int k = tid; k < TS; k += THREADS) {
+#pragma unroll
+                for (int i = 0; i < D; ++i) {
+                    sds[k][i] = k < s_cnt ? ds_g[(s_first + k) * D + i] : 0.0f;
+                    shn[k][i] = k < s_cnt ? hn_g[(s_first + k) * D + i] : 0.0f;
+                }
+            }
+            __syncthreads();
+            const bool fast = gfast_g[st * NW + warp] != 0;
+            const int gbase = warp * GS;
+            const bool active = gbase < s_cnt;
+            const int g_cnt = max(0, min(GS, s_cnt - gbase));
+            describe_group<D>(sds, shn, s_cnt, fast, PERIODIC, ginfo);
+            Run<D> run;
+#pragma unroll
+            for (int i = 0; i < D; ++i) run.ds[i] = sds[gbase][i], run.h[i] = shn[gbase][i];
+            const float *dcol = dataT + (int64_t)s_first * P.nt + t_first + lane;
+            float dv[GS];
+#pragma unroll
+            for (int k = 0; k < GS; ++k)
+                dv[k] = (tv && gbase + k < s_cnt) ? __ldg(dcol + (int64_t)(gbase + k) * P.nt) : 0.0f;
+            __syncthreads();  // ginfo, surv
+
+            for (int g0 = 0; g0 < nq; g0 += G) {
+                const int nb = min(G, nq - g0);
+                uint8_t *alive = alive2[flip];
+                flip ^= 1;
+                record_pass<D>(P, surv + g0, nb, t_cnt, ti, ginfo, thr, rec, alive, [&](int32_t q, BeamTime<D> &bt) {
+                    if (TRAJ)
+                        traj_beam_time<D>(B, T, r0 + q, t_first + lane, bt);
+                    else
+                        beam_time<D>(P, B, q < RJ ? r0 + q : B.n + r0 + q - RJ, P.ts[t_first + lane], bt);
+                });
                 __syncthreads();
-                const int nsurv = nsurv_s;
-                evals += (unsigned long long)nsurv * (unsigned long long)t_cnt * (unsigned long long)s_cnt;
-                for (int g0 = 0; g0 < nsurv; g0 += G) {
-                    {
-                        const int gl = tid / TT, tloc = tid % TT;
-                        Rec<D> r;
-                        if (g0 + gl < nsurv && tloc < t_cnt) {
-                            const int q = surv[g0 + gl];
-                            const int64_t b = TRAJ ? r0 + q : (q < RJ ? r0 + q : B.n + r0 + q - RJ);
-                            BeamTime<D> bt;
-                            if (TRAJ)
-                                traj_beam_time<D>(B, T, b, t_first + tloc, bt);
-                            else
-                                beam_time<D>(P, B, b, P.ts[t_first + tloc], bt);
-                            anchor<D>(P, bt, ti.s0, r);
+                unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
+                evals += (unsigned long long)__popc(bits) * (unsigned)(t_cnt * g_cnt);
+                while (bits) {
+                    const int i0 = take_bit(bits), i1 = take_bit(bits);
+                    float2 ar = make_float2(0.0f, 0.0f), ai = ar, br = ar, bi = ar;
+                    int i2 = -1, i3 = -1;
+                    if (fast) {
+                        i2 = take_bit(bits);
+                        i3 = take_bit(bits);
+                        cf2 za, fa, qa, zb, fb, qb;
+                        int direct = seed_pair<D>(rec, i0, i1, lane, run, skip, za, fa, qa);
+                        if (i2 >= 0) {
+                            direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+#pragma unroll
+                            for (int k = 0; k < GS; ++k) {
+                                if (k > 0) {
+                                    za = cmul2(za, fa);
+                                    zb = cmul2(zb, fb);
+                                    fa = cmul2(fa, qa);
+                                    fb = cmul2(fb, qb);
+                                }
+                                const float2 dk = make_float2(dv[k], dv[k]);
+                                ar = __ffma2_rn(dk, za.re, ar);
+                                ai = __ffma2_rn(neg2(dk), za.im, ai);
+                                br = __ffma2_rn(dk, zb.re, br);
+                                bi = __ffma2_rn(neg2(dk), zb.im, bi);
+                            }
                         } else {
 #pragma unroll
-                            for (int i = 0; i < D; ++i) r.d0[i] = 0.0f, r.wp[i] = 0.0f;
-#pragma unroll
-                            for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = 0.0f, r.p[q] = 0.0f;
-                            r.th0 = 0.0f;
-                            r.amp = 0.0f;
-                        }
-                        const float *rf = reinterpret_cast<const float *>(&r);
-#pragma unroll
-                        for (int f = 0; f < NF; ++f) rec[f][gl][tloc] = rf[f];
-                    }
-                    __syncthreads();
-                    const int ng = min(G, nsurv - g0);
-                    for (int gl = 0; gl < ng; gl += 2) {
-                        float2 ar = make_float2(0.0f, 0.0f), ai = make_float2(0.0f, 0.0f);
-                        if (active) {
-                            Rec<D> ra, rb;
-                            load_rec<D>(rec, gl, lane, ra);
-                            load_rec<D>(rec, gl + 1, lane, rb);  // zero-amplitude record when gl + 1 == ng
-                            cf za, fa, qa, zb, fb, qb;
-                            int ka = kRunRecurrence, kb = kRunRecurrence;
-                            if (fast) {
-                                za = seed_eval<D, false>(ra, sds[gbase], shn[gbase], true, P, fa, qa, &ka, cutoff > 0.0f);
-                                zb = seed_eval<D, false>(rb, sds[gbase], shn[gbase], true, P, fb, qb, &kb, cutoff > 0.0f);
-                                if (ka == kRunNegligible) za = fa = qa = cf{0.0f, 0.0f};
-                                if (kb == kRunNegligible) zb = fb = qb = cf{0.0f, 0.0f};
+                            for (int k = 0; k < GS; ++k) {
+                                if (k > 0) {
+                                    za = cmul2(za, fa);
+                                    fa = cmul2(fa, qa);
+                                }
+                                const float2 dk = make_float2(dv[k], dv[k]);
+                                ar = __ffma2_rn(dk, za.re, ar);
+                                ai = __ffma2_rn(neg2(dk), za.im, ai);
                             }
-                            if (fast && ka != kRunDirect && kb != kRunDirect) {
-#if MSGB_F32X2
-                                cf2 z = pack2(za, zb), f = pack2(fa, fb);
-                                const cf2 q = pack2(qa, qb);
-#pragma unroll
-                                for (int k = 0; k < GS; ++k) {
-                                    if (k > 0) {
-                                        z = cmul2(z, f);
-                                        f = cmul2(f, q);
-                                    }
-                                    const float2 dk = make_float2(dv[k], dv[k]);
-                                    ar = __ffma2_rn(dk, z.re, ar);
-                                    ai = __ffma2_rn(neg2(dk), z.im, ai);
-                                }
-#else
-#pragma unroll
-                                for (int k = 0; k < GS; ++k) {
-                                    if (k > 0) {
-                                        za = cmul(za, fa);
-                                        fa = cmul(fa, qa);
-                                        zb = cmul(zb, fb);
-                                        fb = cmul(fb, qb);
-                                    }
-                                    ar.x = fmaf(dv[k], za.re, ar.x);
-                                    ai.x = fmaf(-dv[k], za.im, ai.x);
-                                    ar.y = fmaf(dv[k], zb.re, ar.y);
-                                    ai.y = fmaf(-dv[k], zb.im, ai.y);
-                                }
-#endif
-                            } else {
-                                // rare: broken runs, out-of-range recurrences
-                                cf dummy_r, dummy_q;
+                        }
+                        if (__any_sync(0xffffffffu, direct != 0)) {
+                            // rare: recurrences out of FP32's range
+#pragma unroll 1
+                            for (int e = 0; e < 4; ++e) {
+                                if (!(direct >> e & 1)) continue;
+                                Rec<D> r;
+                                load_rec<D>(rec, e == 0 ? i0 : (e == 1 ? i1 : (e == 2 ? i2 : i3)), lane, r);
+                                float sr = 0.0f, si = 0.0f;
 #pragma unroll 1
                                 for (int k = 0; k < GS; ++k) {
-                                    const int s = gbase + k;
-                                    const float d = (tv && s < s_cnt) ? __ldg(dcol + (int64_t)s * P.nt) : 0.0f;
-                                    const cf za = seed_eval<D, PERIODIC>(ra, sds[s], shn[s], false, P, dummy_r, dummy_q);
-                                    const cf zb = seed_eval<D, PERIODIC>(rb, sds[s], shn[s], false, P, dummy_r, dummy_q);
-                                    ar.x = fmaf(d, za.re, ar.x);
-                                    ai.x = fmaf(-d, za.im, ai.x);
-                                    ar.y = fmaf(d, zb.re, ar.y);
-                                    ai.y = fmaf(-d, zb.im, ai.y);
+                                    const float d = tv ? __ldg(dcol + (int64_t)(gbase + k) * P.nt) : 0.0f;
+                                    const cf z = direct_eval<D, false>(r, sds[gbase + k], P);
+                                    sr = fmaf(d, z.re, sr);
+                                    si = fmaf(-d, z.im, si);
                                 }
+                                if (e == 0) ar.x = sr, ai.x = si;
+                                if (e == 1) ar.y = sr, ai.y = si;
+                                if (e == 2) br.x = sr, bi.x = si;
+                                if (e == 3) br.y = sr, bi.y = si;
                             }
                         }
-                        // over the 32 times (the partials are sums of 16 terms): a
-                        // reduce-scatter of the pair's four partials, 6 shuffles
-                        // instead of 20.  Lanes 0, 8, 16, 24 end with the sums of
-                        // ar.x, ar.y, ai.x, ai.y; FP64 from here on.
-                        {
-                            const bool u4 = (lane & 16) != 0, u3 = (lane & 8) != 0;
-                            float k0 = u4 ? ai.x : ar.x, k1 = u4 ? ai.y : ar.y;
-                            k0 += __shfl_xor_sync(0xffffffffu, u4 ? ar.x : ai.x, 16);
-                            k1 += __shfl_xor_sync(0xffffffffu, u4 ? ar.y : ai.y, 16);
-                            float v = u3 ? k1 : k0;
-                            v += __shfl_xor_sync(0xffffffffu, u3 ? k0 : k1, 8);
-                            v += __shfl_xor_sync(0xffffffffu, v, 4);
-                            v += __shfl_xor_sync(0xffffffffu, v, 2);
-                            v += __shfl_xor_sync(0xffffffffu, v, 1);
-                            // beam gl + u3 (gl + 1 < G: gl is even and G is even), re / im by u4
-                            if ((lane & 7) == 0) wpart[warp][gl + (u3 ? 1 : 0)][u4 ? 1 : 0] = (double)v;
+                    } else {
+                        Rec<D> ra, rb;
+                        load_rec<D>(rec, i0, lane, ra);
+                        load_rec<D>(rec, i1 >= 0 ? i1 : i0, lane, rb);
+#pragma unroll 1
+                        for (int k = 0; k < g_cnt; ++k) {
+                            const float d = tv ? __ldg(dcol + (int64_t)(gbase + k) * P.nt) : 0.0f;
+                            const cf z0 = direct_eval<D, PERIODIC>(ra, sds[gbase + k], P);
+                            const cf z1 = direct_eval<D, PERIODIC>(rb, sds[gbase + k], P);
+                            ar.x = fmaf(d, z0.re, ar.x);
+                            ai.x = fmaf(-d, z0.im, ai.x);
+                            ar.y = fmaf(d, z1.re, ar.y);
+                            ai.y = fmaf(-d, z1.im, ai.y);
                         }
                     }
-                    __syncthreads();
-                    if (tid < ng) {
-                        double re = 0.0, im = 0.0;
+                    // over the 32 times (the partials are sums of 16 terms): a
+                    // reduce-scatter of the eight partials (re, im of four beams), 9
+                    // shuffles.  Lane 4 v ends with value v; FP64 from here on.
+                    {
+                        const bool u4 = (lane & 16) != 0, u3 = (lane & 8) != 0, u2 = (lane & 4) != 0;
+                        float k0 = u4 ? br.x : ar.x, k1 = u4 ? bi.x : ai.x, k2 = u4 ? br.y : ar.y, k3 = u4 ? bi.y : ai.y;
+                        k0 += __shfl_xor_sync(0xffffffffu, u4 ? ar.x : br.x, 16);
+                        k1 += __shfl_xor_sync(0xffffffffu, u4 ? ai.x : bi.x, 16);
+                        k2 += __shfl_xor_sync(0xffffffffu, u4 ? ar.y : br.y, 16);
+                        k3 += __shfl_xor_sync(0xffffffffu, u4 ? ai.y : bi.y, 16);
+                        float m0 = u3 ? k2 : k0, m1 = u3 ? k3 : k1;
+                        m0 += __shfl_xor_sync(0xffffffffu, u3 ? k0 : k2, 8);
+                        m1 += __shfl_xor_sync(0xffffffffu, u3 ? k1 : k3, 8);
+                        float v = u2 ? m1 : m0;
+                        v += __shfl_xor_sync(0xffffffffu, u2 ? m0 : m1, 4);
+                        v += __shfl_xor_sync(0xffffffffu, v, 2);
+                        v += __shfl_xor_sync(0xffffffffu, v, 1);
+                        const int i = u4 ? (u3 ? i3 : i2) : (u3 ? i1 : i0);
+                        if ((lane & 3) == 0 && i >= 0) wpart[warp][i][u2 ? 1 : 0] = v;
+                    }
+                }
+                __syncthreads();
+                if (tid < 2 * nb) {
+                    const int i = tid >> 1, c = tid & 1;
+                    const unsigned m = alive[i];
+                    double sum = 0.0;
 #pragma unroll
-                        for (int w = 0; w < NW; ++w) {
-                            re += wpart[w][tid][0];
-                            im += wpart[w][tid][1];
-                        }
-                        const int q = surv[g0 + tid];  // distinct within a pass: one owner per slot
-                        acc_smem[2 * q] += re;
-                        acc_smem[2 * q + 1] += im;
-                    }
+                    for (int w = 0; w < NW; ++w)
+                        if (m >> w & 1u) sum += (double)wpart[w][i][c];
+                    acc_smem[2 * surv[g0 + i] + c] += sum;  // slots are distinct within a pass
                 }
             }
         }
@@ -1034,7 +1221,7 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
             acc_smem[2 * q + 1] = 0.0;
         }
     }
-    if (eval_count && tid == 0 && evals) atomicAdd(eval_count, evals);
+    if (eval_count && lane == 0 && evals) atomicAdd(eval_count, evals);
 }
 
 // g[j] = sum over time tiles, in order, of part[tt][j] (trajectories) or of
@@ -1199,13 +1386,15 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     const int n_tiles = (int)(n_st * n_tt);
     const int64_t want = 2LL * sm_count();
     const unsigned grid = (unsigned)(want < n_tiles ? want : n_tiles);
+    constexpr size_t smem = rec_bytes<D>();
     auto args = [&](auto kern) {
-        kern<<<grid, THREADS, 0, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull), (const TileInfo<D> *)(ws + l.tiles),
-                                       (const int32_t *)(ws + l.offs), (const float *)(ws + l.ds),
-                                       (const float *)(ws + l.hn), (const uint8_t *)(ws + l.seed),
-                                       (const uint8_t *)(ws + l.gfast), (const int32_t *)(ws + l.vals_out),
-                                       o ? (float)o->cutoff : 0.0f, out, o ? o->eval_count : nullptr, work,
-                                       (int)n_st, n_tiles, T);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull),
+                                          (const TileInfo<D> *)(ws + l.tiles), (const int32_t *)(ws + l.offs),
+                                          (const float *)(ws + l.ds), (const float *)(ws + l.hn),
+                                          (const uint8_t *)(ws + l.gfast), (const int32_t *)(ws + l.vals_out),
+                                          o ? (float)o->cutoff : 0.0f, out, o ? o->eval_count : nullptr, work,
+                                          (int)n_st, n_tiles, T);
     };
     if (periodic)
         args(fwd32_kernel<D, true, TRAJ>);
@@ -1229,7 +1418,7 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     for (int i = 0; i < D; ++i) periodic |= (p->periodic[i] != 0);
     const int64_t nw = TRAJ ? T.nb : b->n;  // beam indices j of the items
     const int64_t n_st = l.n_st, n_tt = (p->nt + TT - 1) / TT;
-    const int64_t n_ranges = (nw + AdjRange<TRAJ>::RJ - 1) / AdjRange<TRAJ>::RJ;
+    const int64_t n_ranges = (nw + AdjRange<D, TRAJ>::RJ - 1) / AdjRange<D, TRAJ>::RJ;
     if (n_ranges * n_tt > 0x7fffffffLL || n_st > 0x7fffffffLL)
         return fail(MSGB_ERR_UNSUPPORTED, "msgb_adj_gather_f32: too many work items");
     int *work = (int *)(ws + l.work);
@@ -1237,7 +1426,7 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     const int n_items = (int)(n_ranges * n_tt);
     const int64_t want = 2LL * sm_count();
     const unsigned grid = (unsigned)(want < n_items ? want : n_items);
-    const size_t smem = (size_t)NACC * 2 * sizeof(double);
+    constexpr size_t smem = (size_t)AdjRange<D, TRAJ>::NACC * 2 * sizeof(double) + rec_bytes<D>();
     auto args = [&](auto kern) {
         // static + dynamic shared memory exceed the default 48 KB: opt in
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
