@@ -266,26 +266,119 @@ __device__ __forceinline__ void beam_time(const ProbArgs &P, const BeamArgs &B, 
     r.amp = 2.0f * sqrtf(fmaf(A.re, A.re, A.im * A.im));
 }
 
-// Anchor-dependent completion of a record.
+// What the closed form needs per selected coefficient (mode independent),
+// prepared in FP64 once per call.  With M0 = i diag(beta), u = p0/|p0| and n_j the
+// eigenvectors of diag(beta) restricted to the plane normal to u (eigenvalues d_j),
+// diag(beta) = e u u^T + sum_j d_j nu_j nu_j^T, nu_j = n_j + (n_j.beta u / d_j) u, and
+//   M(t) = i e u u^T + sum_j d_j k_j (x_j + i) nu_j nu_j^T,  x_j = c t d_j / |p0|,
+//   k_j = 1 / (1 + x_j^2),  A(t) = a0 prod_j (1 + i x_j)^(-1/2),
+// the Sherman-Morrison closed form (gb_solvers.py:194-264, :306-353) written as a sum
+// of positive terms: no cancellation in FP32 and one division per transverse axis
+// instead of complex divisions and a complex square root per record.
 template <int D>
-__device__ __forceinline__ void anchor(const ProbArgs &P, const BeamTime<D> &bt, const double *s0, Rec<D> &r) {
-    double lin = 0.0;
+struct alignas(16) HomBeam {
+    static constexpr int NT = D - 1;  // transverse axes
+    double x0[D], v[D], wp[D];        // centre, velocity c u (mode +1), w p0
+    float N[NT > 0 ? NT : 1][Sym<D>::S];  // w/2 d_j nu_j nu_j^T (off-diagonals doubled)
+    float U[Sym<D>::S];                   // w/2 e u u^T (off-diagonals doubled)
+    float td[NT > 0 ? NT : 1];            // c d_j / |p0|
+    float aabs, aarg;                     // a0
+    int ok;                               // 0: M0 not i diag(beta > 0): beam_time is used
+};
+
+template <int D>
+__device__ __forceinline__ HomBeam<D> make_hom_beam(const ProbArgs &P, const BeamArgs &B, int64_t j) {
+    HomBeam<D> h;
+    double p0[D], beta[D], n2 = 0.0;
+    h.ok = 1;
+    const double w = B.omega[j];
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-        double d0 = s0[i] - bt.x[i];
-        if (P.periodic[i]) d0 -= P.L[i] * nearbyint(d0 / P.L[i]);
-        r.d0[i] = (float)d0;
-        r.wp[i] = (float)bt.wp[i];
-        lin = fma(bt.wp[i], d0, lin);
+        p0[i] = B.p0[j * D + i];
+        n2 += p0[i] * p0[i];
+        beta[i] = B.alpha[2 * (j * D + i) + 1];
+        if (B.alpha[2 * (j * D + i)] != 0.0 || !(beta[i] > 0.0)) h.ok = 0;
+    }
+    const double np = sqrt(n2);
+    if (!(np > 0.0)) h.ok = 0;
+    double u[D], n[D][D];  // n[j]: transverse directions, j < D - 1
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+        u[i] = p0[i] / np;
+        h.x0[i] = B.x0[j * D + i];
+        h.v[i] = P.c * u[i];
+        h.wp[i] = w * p0[i];
+    }
+    if (D == 2) {
+        n[0][0] = -u[1 % D];
+        n[0][1 % D] = u[0];
+    } else if (D == 3) {
+        // any orthonormal pair normal to u, then turned onto the eigenvectors
+        const int ax = fabs(u[0]) < 0.6 ? 0 : 1;
+        double e0[3] = {ax == 0 ? 1.0 : 0.0, ax == 1 ? 1.0 : 0.0, 0.0};
+        double a[3], b[3], aa = 0.0;
+        const double eu = e0[0] * u[0] + e0[1] * u[1 % D];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = e0[i] - eu * u[i % D];
+            aa += a[i] * a[i];
+        }
+        const double ia = 1.0 / sqrt(aa);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) a[i] *= ia;
+        b[0] = u[1 % D] * a[2] - u[2 % D] * a[1];
+        b[1] = u[2 % D] * a[0] - u[0] * a[2];
+        b[2] = u[0] * a[1] - u[1 % D] * a[0];
+        double daa = 0.0, dab = 0.0, dbb = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            daa += beta[i % D] * a[i] * a[i];
+            dab += beta[i % D] * a[i] * b[i];
+            dbb += beta[i % D] * b[i] * b[i];
+        }
+        double sn, cs;
+        sincos(0.5 * atan2(2.0 * dab, daa - dbb), &sn, &cs);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            n[0][i % D] = cs * a[i] + sn * b[i];
+            n[1 % D][i % D] = cs * b[i] - sn * a[i];
+        }
+    }
+    double e = 0.0;
+#pragma unroll
+    for (int i = 0; i < D; ++i) e += beta[i] * u[i] * u[i];
+#pragma unroll
+    for (int q = 0; q < D - 1; ++q) {
+        double d = 0.0, b = 0.0, nu[D];
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            d += beta[i] * n[q][i] * n[q][i];
+            b += beta[i] * n[q][i] * u[i];
+        }
+        e -= b * b / d;
+#pragma unroll
+        for (int i = 0; i < D; ++i) nu[i] = n[q][i] + (b / d) * u[i];
+#pragma unroll
+        for (int i = 0; i < D; ++i)
+#pragma unroll
+            for (int k = i; k < D; ++k)
+                h.N[q][sym_index<D>(i, k)] = (float)((i == k ? 0.5 : 1.0) * w * d * nu[i] * nu[k]);
+        h.td[q] = (float)(P.c * d / np);
     }
 #pragma unroll
-    for (int q = 0; q < Sym<D>::S; ++q) {
-        r.q[q] = bt.q[q];
-        r.p[q] = bt.p[q];
-    }
-    const double th = lin + (double)bt.ang;
-    r.th0 = (float)(th - 6.283185307179586 * nearbyint(th * 0.15915494309189535));
-    r.amp = bt.amp;
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int k = i; k < D; ++k) h.U[sym_index<D>(i, k)] = (float)((i == k ? 0.5 : 1.0) * w * e * u[i] * u[k]);
+    const float ar = (float)B.a0[2 * j], ai = (float)B.a0[2 * j + 1];
+    h.aabs = hypotf(ar, ai);
+    h.aarg = atan2f(ai, (ar == 0.0f && ai == 0.0f) ? 1e-12f : ar);
+    return h;
+}
+
+template <int D>
+__global__ void hom_prep_kernel(ProbArgs P, BeamArgs B, HomBeam<D> *out) {
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (j < B.n) out[j] = make_hom_beam<D>(P, B, j);
 }
 
 // Largest e-fold count the run recurrence may meet: at the seed (chi), in the
@@ -307,7 +400,7 @@ constexpr float kNegligibleEfolds = 40.0f;
 // Im M and a box around 128 sensors, so most of what it keeps lies far outside the
 // beam: at 1024^2 heterogeneous 67 % of the (beam, group) pairs it kept were
 // beyond 24 e-folds, 33 % at 512^2 homogeneous, 56 % at 128^3.
-constexpr float kGroupMarginEfolds = 8.0f;
+constexpr float kGroupMarginEfolds = 4.0f;
 
 // One warp's sensor group: its straight run's start and step.
 template <int D>
@@ -572,22 +665,6 @@ __device__ __forceinline__ bool traj_survives(const TrajSrc<D> &T, int64_t bl, i
     return c[2 * D] * d2 * 0.999f <= cutoff;
 }
 
-template <int D>
-__device__ __forceinline__ void traj_beam_time(const BeamArgs &B, const TrajSrc<D> &T, int64_t bl, int64_t k,
-                                               BeamTime<D> &bt) {
-    if (T.pool)
-        bt = T.pool[(int64_t)T.slot[(k / TT) * T.nb + bl] * TT + k % TT];
-    else
-        bt = T.rec[k * T.nb + bl];
-    const int64_t b = T.b_first + bl;
-    const int64_t j = b < B.n ? b : b - B.n;
-    // the coefficient's amplitude and phase join the record's FP32 |A| and
-    // arg A in FP32 (the record already holds them to FP32 precision)
-    const float ar = (float)B.a0[2 * j], ai = (float)B.a0[2 * j + 1];
-    bt.amp *= hypotf(ar, ai);
-    bt.ang += atan2f(ai, (ar == 0.0f && ai == 0.0f) ? 1e-12f : ar);
-}
-
 // ------------------------------------------------------------------ record passes
 // A record pass holds up to G beams' records at the tile's 32 times in shared
 // memory, rec[field][beam][time], and per beam an 8-bit mask of the warps (sensor
@@ -597,13 +674,23 @@ constexpr size_t rec_bytes() {
     return sizeof(float) * Rec<D>::NF * G * TT;
 }
 
-// Per group of GS sensors, for the test of the record pass: the run's start
-// and step (fast groups: one straight run), or a ball around the sensors.
+// One group of GS sensors, for the test of the record pass: the run's start and
+// step (one straight run), or a ball around the sensors.
 template <int D>
 struct GroupInfo {
-    float ds[D], h[D];  // fast: run start and step; else: centre (ds)
-    float rad;          // not fast: largest distance of a sensor from the centre
-    int kind;           // 0 no sensors, 1 fast, 2 not fast, 3 not fast and never left out (periodic)
+    float ds[D], h[D];  // straight run: start and step; else: centre (ds)
+    float rad;          // else: largest distance of a sensor from the centre
+    int kind;           // 0 no sensors, 1 straight run, 2 other, 3 never left out (periodic)
+};
+
+template <int D>
+struct TileGroups {
+    GroupInfo<D> g[NW];
+    // lattice: the n groups are straight runs with one step, starting at
+    // g[0].ds + k e (a 128-sensor line, or rows of a detector plane)
+    float e[D];
+    int lattice, n;
+    unsigned present;  // groups that hold sensors
 };
 
 // Does a record reach group g within thr e-folds (a lower bound on the exponent)?
@@ -624,61 +711,230 @@ __device__ __forceinline__ bool group_reached(const Rec<D> &r, const GroupInfo<D
 // Describe the tile's groups (warp w describes group w; sds / shn loaded).
 template <int D>
 __device__ __forceinline__ void describe_group(const float (*sds)[D], const float (*shn)[D], int s_cnt, bool fast,
-                                               bool periodic, GroupInfo<D> *gi) {
+                                               bool periodic, TileGroups<D> &tg) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gbase = warp * GS;
     const int cnt = min(GS, s_cnt - gbase);
-    float lo[D], hi[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-        lo[i] = hi[i] = sds[gbase][i];
-        for (int k = 1; k < cnt; ++k) lo[i] = fminf(lo[i], sds[gbase + k][i]), hi[i] = fmaxf(hi[i], sds[gbase + k][i]);
-    }
     if (lane == 0) {
         GroupInfo<D> g;
         float r2 = 0.0f;
 #pragma unroll
         for (int i = 0; i < D; ++i) {
-            g.ds[i] = fast ? sds[gbase][i] : 0.5f * (lo[i] + hi[i]);
+            float lo = sds[gbase][i], hi = lo;
+            if (!fast)
+                for (int k = 1; k < cnt; ++k) lo = fminf(lo, sds[gbase + k][i]), hi = fmaxf(hi, sds[gbase + k][i]);
+            g.ds[i] = fast ? lo : 0.5f * (lo + hi);
             g.h[i] = shn[gbase][i];
-            const float e = 0.5f * (hi[i] - lo[i]);
+            const float e = 0.5f * (hi - lo);
             r2 = fmaf(e, e, r2);
         }
         g.rad = sqrtf(r2) * 1.00001f;
         g.kind = cnt <= 0 ? 0 : (fast ? 1 : (periodic ? 3 : 2));
-        gi[warp] = g;
+        tg.g[warp] = g;
     }
 }
 
-// Write the records of the pass's beams idx[0 .. nb) and their masks alive[].
-// load(b, bt): the tile-independent part of beam b at this lane's time.
-template <int D, typename Load>
-__device__ __forceinline__ void record_pass(const ProbArgs &P, const int32_t *idx, int nb, int t_cnt, const TileInfo<D> &ti,
-                                            const GroupInfo<D> *gi, float thr, float *rec, uint8_t *alive,
-                                            const Load &load) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool tv = lane < t_cnt;
-#pragma unroll 1
-    for (int i = warp; i < nb; i += NW) {
-        Rec<D> r;
+template <int D>
+__device__ __forceinline__ void find_lattice(TileGroups<D> &tg) {
+    int n = 0;
+    while (n < NW && tg.g[n].kind == 1) ++n;
+    bool ok = n > 0 && (n == NW || tg.g[n].kind == 0);  // groups without sensors come last
+    float hh = 0.0f;
+    for (int i = 0; i < D; ++i) hh += fabsf(tg.g[0].h[i]);
+    for (int i = 0; i < D; ++i) {
+        const float e = n > 1 ? tg.g[1].ds[i] - tg.g[0].ds[i] : 0.0f;
+        tg.e[i] = e;
+        // a thousandth of a sensor step is far below the test's margin
+        for (int g = 0; g < n; ++g)
+            ok = ok && fabsf(tg.g[g].h[i] - tg.g[0].h[i]) <= 1e-4f * hh &&
+                 fabsf(tg.g[g].ds[i] - fmaf((float)g, e, tg.g[0].ds[i])) <= 1e-3f * hh;
+    }
+    tg.n = n;
+    tg.lattice = ok ? 1 : 0;
+    tg.present = 0;
+    for (int g = 0; g < NW; ++g) tg.present |= tg.g[g].kind ? 1u << g : 0u;
+}
+
+// Mask of the groups of the tile that this lane's record reaches within thr.
+template <int D>
+__device__ __forceinline__ unsigned reached_mask(const Rec<D> &r, const TileGroups<D> &tg, float thr) {
+    unsigned m = 0;
+    if (tg.lattice) {
+        // chi on the lattice: chi(g, k) = c0 + Bg g + Ag g^2 + (Bk + C g) k + Ak k^2
+        const float *h = tg.g[0].h, *e = tg.e;
+        float Dl[D];
 #pragma unroll
-        for (int k = 0; k < D; ++k) r.d0[k] = r.wp[k] = 0.0f;
-#pragma unroll
-        for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = r.p[q] = 0.0f;
-        r.th0 = r.amp = 0.0f;
-        if (tv) {
-            BeamTime<D> bt;
-            load(idx[i], bt);
-            anchor<D>(P, bt, ti.s0, r);
-        }
-        unsigned m = 0;
+        for (int i = 0; i < D; ++i) Dl[i] = tg.g[0].ds[i] + r.d0[i];
+        const float c0 = quad<D>(r.p, Dl), Bk = bilin2<D>(r.p, h, Dl), Ak = quad<D>(r.p, h);
+        const float Bg = bilin2<D>(r.p, e, Dl), Ag = quad<D>(r.p, e), C = bilin2<D>(r.p, h, e);
+        const float im = Ak > 0.0f ? __fdividef(-0.5f, Ak) : 0.0f;
+        const float lim = fmaf(2e-6f, c0, thr);  // round-off of the expansion
+        const int n = tg.n;
 #pragma unroll
         for (int g = 0; g < NW; ++g) {
-            const GroupInfo<D> &q = gi[g];
-            if (q.kind == 0) continue;
-            const bool in = tv && (thr <= 0.0f || q.kind == 3 || group_reached<D>(r, q, thr));
-            if (__any_sync(0xffffffffu, in)) m |= 1u << g;
+            const float gf = (float)g;
+            const float B = fmaf(C, gf, Bk), cg = fmaf(fmaf(Ag, gf, Bg), gf, c0);
+            const float kv = fminf(fmaxf(B * im, 0.0f), (float)(GS - 1));
+            if (fmaf(fmaf(Ak, kv, B), kv, cg) <= lim && g < n) m |= 1u << g;
         }
+        return m;
+    }
+    for (int g = 0; g < NW; ++g) {
+        const GroupInfo<D> &q = tg.g[g];
+        if (q.kind && (q.kind == 3 || group_reached<D>(r, q, thr))) m |= 1u << g;
+    }
+    return m;
+}
+
+// The closed-form beams of a pass, staged per warp (4 beams each).
+template <int D, bool TRAJ>
+struct HomStage {
+    HomBeam<D> b[G];
+};
+template <int D>
+struct HomStage<D, true> {};
+
+template <int D>
+__device__ __noinline__ void general_beam_time(const ProbArgs &P, const BeamArgs &B, int64_t b, double t,
+                                               BeamTime<D> &bt) {
+    beam_time<D>(P, B, b, t, bt);
+}
+
+// Write the records of the pass's beams beam_of(0 .. nb) and their masks alive[].
+// What a record needs beyond the test (the anchor phase, the amplitude) is formed
+// only when the beam reaches some group at some time.
+template <int D, bool TRAJ, typename BeamOf>
+__device__ __forceinline__ void record_pass(const ProbArgs &P, const BeamArgs &B, const TrajSrc<D> &T,
+                                            const HomBeam<D> *hom, HomStage<D, TRAJ> &stage, int64_t t_first, int t_cnt,
+                                            const TileInfo<D> &ti, const TileGroups<D> &tg, float thr, float *rec,
+                                            uint8_t *alive, int nb, const BeamOf &beam_of) {
+    constexpr int PW = G / NW;  // beams per warp and pass
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool tv = lane < t_cnt;
+    const int mine = warp < nb ? (nb - warp + NW - 1) / NW : 0;  // this warp's beams: warp + k NW, k < mine
+    // lane k < PW looks up beam k of the warp
+    int64_t b_lane = 0;
+    int32_t blk_lane = 0;
+    float aabs_lane = 0.0f, aarg_lane = 0.0f;
+    if (lane < mine) {
+        b_lane = beam_of(warp + lane * NW);
+        if constexpr (TRAJ) {
+            if (T.pool) blk_lane = T.slot[(t_first / TT) * T.nb + b_lane];
+            // the coefficient's amplitude and phase join the record's FP32 |A| and
+            // arg A in FP32 (the record already holds them to FP32 precision)
+            const int64_t b = T.b_first + b_lane, j = b < B.n ? b : b - B.n;
+            const float ar = (float)B.a0[2 * j], ai = (float)B.a0[2 * j + 1];
+            aabs_lane = hypotf(ar, ai);
+            aarg_lane = atan2f(ai, (ar == 0.0f && ai == 0.0f) ? 1e-12f : ar);
+        }
+    }
+    if constexpr (!TRAJ) {
+        if (hom) {
+            constexpr int W = sizeof(HomBeam<D>) / 16;
+            __syncwarp();
+#pragma unroll 1
+            for (int q = lane; q < PW * W; q += 32) {
+                const int k = q / W;
+                const int64_t b = k < mine ? beam_of(warp + k * NW) : -1;
+                if (b >= 0)
+                    reinterpret_cast<int4 *>(&stage.b[warp * PW + k])[q % W] =
+                        __ldg(reinterpret_cast<const int4 *>(&hom[b < B.n ? b : b - B.n]) + q % W);
+            }
+        } else if (lane < mine) {  // no table in the caller's scratch
+            stage.b[warp * PW + lane] = make_hom_beam<D>(P, B, b_lane < B.n ? b_lane : b_lane - B.n);
+        }
+        __syncwarp();
+    }
+    const double t = !TRAJ && tv ? P.ts[t_first + lane] : 0.0;
+#pragma unroll 2
+    for (int k = 0; k < PW; ++k) {
+        if (k >= mine) break;
+        const int i = warp + k * NW;
+        const int64_t b = __shfl_sync(0xffffffffu, b_lane, k);
+        Rec<D> r;
+        double dd[D], wpd[D];
+        float ang = 0.0f, xk[D];  // xk: the closed form's x_j
+#pragma unroll
+        for (int a = 0; a < D; ++a) r.d0[a] = 0.0f, wpd[a] = 0.0, dd[a] = 0.0, xk[a] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = r.p[q] = 0.0f;
+        r.amp = 0.0f;
+        bool closed = false;
+        if constexpr (TRAJ) {
+            const int32_t blk = __shfl_sync(0xffffffffu, blk_lane, k);
+            const float aabs = __shfl_sync(0xffffffffu, aabs_lane, k), aarg = __shfl_sync(0xffffffffu, aarg_lane, k);
+            if (tv) {
+                const BeamTime<D> bt = T.pool ? T.pool[(int64_t)blk * TT + lane] : T.rec[(t_first + lane) * T.nb + b];
+#pragma unroll
+                for (int a = 0; a < D; ++a) {
+                    dd[a] = ti.s0[a] - bt.x[a];
+                    wpd[a] = bt.wp[a];
+                }
+#pragma unroll
+                for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = bt.q[q], r.p[q] = bt.p[q];
+                r.amp = bt.amp * aabs;
+                ang = bt.ang + aarg;
+            }
+        } else {
+            const HomBeam<D> &h = stage.b[warp * PW + k];
+            const double tm = b < B.n ? t : -t;
+            if (h.ok) {
+                closed = true;
+                const float tf = (float)tm;
+#pragma unroll
+                for (int a = 0; a < D; ++a) {
+                    dd[a] = fma(-h.v[a], tm, ti.s0[a] - h.x0[a]);
+                    wpd[a] = h.wp[a];
+                }
+#pragma unroll
+                for (int q = 0; q < Sym<D>::S; ++q) r.p[q] = h.U[q];
+                float kk = 1.0f;
+#pragma unroll
+                for (int n = 0; n < D - 1; ++n) {
+                    xk[n] = h.td[n] * tf;
+                    const float kn = __frcp_rn(fmaf(xk[n], xk[n], 1.0f)), xn = xk[n] * kn;
+                    kk *= kn;
+#pragma unroll
+                    for (int q = 0; q < Sym<D>::S; ++q) {
+                        r.p[q] = fmaf(kn, h.N[n][q], r.p[q]);
+                        r.q[q] = fmaf(xn, h.N[n][q], r.q[q]);
+                    }
+                }
+                r.amp = kk;  // to the power 1/4 below
+                ang = h.aarg;
+            } else if (tv) {
+                BeamTime<D> bt;
+                general_beam_time<D>(P, B, b, t, bt);
+#pragma unroll
+                for (int a = 0; a < D; ++a) {
+                    dd[a] = ti.s0[a] - bt.x[a];
+                    wpd[a] = bt.wp[a];
+                }
+#pragma unroll
+                for (int q = 0; q < Sym<D>::S; ++q) r.q[q] = bt.q[q], r.p[q] = bt.p[q];
+                r.amp = bt.amp;
+                ang = bt.ang;
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            if (P.periodic[a]) dd[a] -= P.L[a] * nearbyint(dd[a] / P.L[a]);
+            r.d0[a] = (float)dd[a];
+            r.wp[a] = (float)wpd[a];
+        }
+        const unsigned reach = !tv ? 0u : (thr > 0.0f ? reached_mask<D>(r, tg, thr) : tg.present);
+        const unsigned m = __reduce_or_sync(0xffffffffu, reach);
         if (m) {
+            double lin = 0.0;
+#pragma unroll
+            for (int a = 0; a < D; ++a) lin = fma(wpd[a], dd[a], lin);
+            if (!TRAJ && closed) {
+                if constexpr (!TRAJ) r.amp = 2.0f * stage.b[warp * PW + k].aabs * sqrtf(sqrtf(r.amp));
+#pragma unroll
+                for (int n = 0; n < D - 1; ++n) ang = fmaf(-0.5f, atanf(xk[n]), ang);
+            }
+            const double th = lin + (double)ang;
+            r.th0 = (float)(th - 6.283185307179586 * nearbyint(th * 0.15915494309189535));
+            if (!tv) r.amp = 0.0f;
             const float *rf = reinterpret_cast<const float *>(&r);
 #pragma unroll
             for (int f = 0; f < Rec<D>::NF; ++f) rec[(f * G + i) * TT + lane] = rf[f];
@@ -758,12 +1014,13 @@ constexpr int SCAN = 4;  // beams tested per thread and scan
 // triples) with the seeds' MUFU work beside it.
 template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
-fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *tiles, const int32_t *offs,
+fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
              const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const int32_t *perm, float cutoff,
              float *out, unsigned long long *eval_count, int *work, int n_st, int n_tiles, TrajSrc<D> T) {
     extern __shared__ float rec[];  // rec_bytes<D>()
     __shared__ float sds[TS][D], shn[TS][D];
-    __shared__ GroupInfo<D> ginfo[NW];
+    __shared__ TileGroups<D> ginfo;
+    __shared__ HomStage<D, TRAJ> hstage;
     __shared__ int32_t surv[2 * SCAN * THREADS + G];
     __shared__ int warp_cnt[SCAN * NW];
     __shared__ uint8_t alive[G];
@@ -796,6 +1053,8 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
         const int gbase = warp * GS;
         const bool active = gbase < s_cnt;
         describe_group<D>(sds, shn, s_cnt, fast, PERIODIC, ginfo);
+        __syncthreads();
+        if (tid == 0) find_lattice<D>(ginfo);
         Run<D> run;
 #pragma unroll
         for (int i = 0; i < D; ++i) run.ds[i] = sds[gbase][i], run.h[i] = shn[gbase][i];
@@ -857,12 +1116,8 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
             int g0 = 0;
             while (nq - g0 >= G || (last_scan && g0 < nq)) {
                 const int nb = min(G, nq - g0);
-                record_pass<D>(P, surv + g0, nb, t_cnt, ti, ginfo, thr, rec, alive, [&](int32_t b, BeamTime<D> &bt) {
-                    if (TRAJ)
-                        traj_beam_time<D>(B, T, b, t_first + lane, bt);
-                    else
-                        beam_time<D>(P, B, b, P.ts[t_first + lane], bt);
-                });
+                record_pass<D, TRAJ>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb,
+                                     [&](int i) { return (int64_t)surv[g0 + i]; });
                 __syncthreads();
                 unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
                 evals += (unsigned long long)__popc(bits) * (unsigned)(t_cnt * g_cnt);
@@ -998,7 +1253,7 @@ struct AdjRange {
 
 template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
-adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *tiles, const int32_t *offs,
+adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
              const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const float *dataT, float cutoff,
              double *part, unsigned long long *eval_count, int *work, int n_st, int n_ranges, int n_items,
              TrajSrc<D> T) {
@@ -1006,7 +1261,8 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
     extern __shared__ double acc_smem[];  // (NACC, 2), then the records
     float *rec = reinterpret_cast<float *>(acc_smem + 2 * NACC);
     __shared__ float sds[TS][D], shn[TS][D];
-    __shared__ GroupInfo<D> ginfo[NW];
+    __shared__ TileGroups<D> ginfo;
+    __shared__ HomStage<D, TRAJ> hstage;
     __shared__ int32_t surv[NACC];  // a range's survivors in one tile (local slots)
     __shared__ int warp_cnt[NW];
     __shared__ float wpart[NW][G][2];
@@ -1085,17 +1341,17 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const TileInfo<D> *til
 #pragma unroll
             for (int k = 0; k < GS; ++k)
                 dv[k] = (tv && gbase + k < s_cnt) ? __ldg(dcol + (int64_t)(gbase + k) * P.nt) : 0.0f;
+            __syncthreads();
+            if (tid == 0) find_lattice<D>(ginfo);
             __syncthreads();  // ginfo, surv
 
             for (int g0 = 0; g0 < nq; g0 += G) {
                 const int nb = min(G, nq - g0);
                 uint8_t *alive = alive2[flip];
                 flip ^= 1;
-                record_pass<D>(P, surv + g0, nb, t_cnt, ti, ginfo, thr, rec, alive, [&](int32_t q, BeamTime<D> &bt) {
-                    if (TRAJ)
-                        traj_beam_time<D>(B, T, r0 + q, t_first + lane, bt);
-                    else
-                        beam_time<D>(P, B, q < RJ ? r0 + q : B.n + r0 + q - RJ, P.ts[t_first + lane], bt);
+                record_pass<D, TRAJ>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb, [&](int i) {
+                    const int q = surv[g0 + i];
+                    return TRAJ || q < RJ ? r0 + q : B.n + r0 + q - RJ;
                 });
                 __syncthreads();
                 unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
@@ -1286,10 +1542,27 @@ Layout layout(const msgb_problem *p, int64_t n_beams, bool with_data, int64_t n_
     l.cull = o; o = align256(o + l.cull_cap * sizeof(Cull<3>));
     l.data = o; o = align256(o + (with_data ? p->nt * ns * 4 : 0));
     l.work = o; o = align256(o + 64);
+    // (the closed-form beam table follows when the caller's workspace has room: see hom_bytes)
     // adjoint partials: one complex FP64 per (time tile, beam mode) of the coefficients
     l.part = o; o = align256(o + (with_data ? (size_t)((p->nt + TT - 1) / TT) * 2 * (n_beams > 0 ? n_beams : 0) * 16 : 0));
     l.total = o;
     return l;
+}
+
+// The closed-form beam table (HomBeam), after everything else in a workspace
+// sized by msgb_sum_f32_workspace_size; a smaller scratch (the static one, for
+// many coefficients) goes without and every record pass prepares its beams.
+size_t hom_bytes(int ndim, int64_t n) {
+    const size_t per = ndim == 1 ? sizeof(HomBeam<1>) : (ndim == 2 ? sizeof(HomBeam<2>) : sizeof(HomBeam<3>));
+    return align256(per * (size_t)(n > 0 ? n : 0));
+}
+
+template <int D>
+const HomBeam<D> *prepare_hom(const msgb_problem *p, const msgb_beam_set *b, char *at, size_t spare, cudaStream_t st) {
+    if (b->n == 0 || spare < hom_bytes(D, b->n)) return nullptr;
+    HomBeam<D> *h = (HomBeam<D> *)at;
+    hom_prep_kernel<D><<<(unsigned)((b->n + 127) / 128), 128, 0, st>>>(to_args(p), to_args(b), h);
+    return h;
 }
 
 // Adjoint partials of a trajectory chunk of nb beams: (n_tt, nb) complex FP64.
@@ -1370,7 +1643,7 @@ int sm_count() {
 
 template <int D, bool TRAJ>
 int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, char *ws, const Layout &l,
-            float *out, cudaStream_t st, TrajSrc<D> T) {
+            size_t ws_bytes, float *out, cudaStream_t st, TrajSrc<D> T) {
     // trajectory sums cull with the records' own boxes: the closed-form
     // culling table (sized for no beams in their layout) is not built
     msgb_beam_set none{};
@@ -1387,9 +1660,10 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     const int64_t want = 2LL * sm_count();
     const unsigned grid = (unsigned)(want < n_tiles ? want : n_tiles);
     constexpr size_t smem = rec_bytes<D>();
+    const HomBeam<D> *hom = TRAJ ? nullptr : prepare_hom<D>(p, b, ws + l.total, ws_bytes - l.total, st);
     auto args = [&](auto kern) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull),
+        kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull), hom,
                                           (const TileInfo<D> *)(ws + l.tiles), (const int32_t *)(ws + l.offs),
                                           (const float *)(ws + l.ds), (const float *)(ws + l.hn),
                                           (const uint8_t *)(ws + l.gfast), (const int32_t *)(ws + l.vals_out),
@@ -1405,7 +1679,7 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
 
 template <int D, bool TRAJ>
 int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, char *ws, const Layout &l,
-            const float *data, double *part, double *g, cudaStream_t st, TrajSrc<D> T) {
+            size_t ws_bytes, const float *data, double *part, double *g, cudaStream_t st, TrajSrc<D> T) {
     msgb_beam_set none{};
     if (int e = prep<D>(p, TRAJ ? &none : b, o, l, ws, st)) return e;
     dim3 tg((unsigned)((p->ns + 31) / 32), (unsigned)((p->nt + 31) / 32));
@@ -1427,10 +1701,11 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     const int64_t want = 2LL * sm_count();
     const unsigned grid = (unsigned)(want < n_items ? want : n_items);
     constexpr size_t smem = (size_t)AdjRange<D, TRAJ>::NACC * 2 * sizeof(double) + rec_bytes<D>();
+    const HomBeam<D> *hom = TRAJ ? nullptr : prepare_hom<D>(p, b, ws + l.total, ws_bytes - l.total, st);
     auto args = [&](auto kern) {
         // static + dynamic shared memory exceed the default 48 KB: opt in
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull),
+        kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull), hom,
                                           (const TileInfo<D> *)(ws + l.tiles), (const int32_t *)(ws + l.offs),
                                           (const float *)(ws + l.ds), (const float *)(ws + l.hn),
                                           (const uint8_t *)(ws + l.gfast), (const float *)(ws + l.data),
@@ -1478,7 +1753,7 @@ extern "C" size_t msgb_sum_f32_workspace_size(const msgb_problem *prob, int64_t 
     // The default tiling has the most tiles a valid tiling of ns sensors needs
     // when every tile is full; reserve for one tile per 16 sensors so that
     // caller tilings with partial tiles fit as well.
-    return layout(prob, n, true, (prob->ns + GS - 1) / GS).total;
+    return layout(prob, n, true, (prob->ns + GS - 1) / GS).total + hom_bytes(prob->ndim, n);
 }
 
 static int check_ws(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, bool with_data, void *ws,
@@ -1504,9 +1779,9 @@ extern "C" int msgb_sum_fwd_f32(const msgb_problem *prob, const msgb_beam_set *b
     cudaStream_t st = as_stream(stream);
     char *ws = (char *)workspace;
     switch (prob->ndim) {
-        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
-        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
-        default: return run_fwd<3, false>(prob, beams, opts, ws, l, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
+        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
+        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
+        default: return run_fwd<3, false>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
     }
 }
 
@@ -1526,11 +1801,11 @@ extern "C" int msgb_adj_gather_f32(const msgb_problem *prob, const msgb_beam_set
     cudaStream_t st = as_stream(stream);
     char *ws = (char *)workspace;
     switch (prob->ndim) {
-        case 1: return run_adj<1, false>(prob, beams, opts, ws, l, data, (double *)(ws + l.part), g, st,
+        case 1: return run_adj<1, false>(prob, beams, opts, ws, l, workspace_bytes, data, (double *)(ws + l.part), g, st,
                                          traj_src<1>(nullptr, nullptr, 1, 1));
-        case 2: return run_adj<2, false>(prob, beams, opts, ws, l, data, (double *)(ws + l.part), g, st,
+        case 2: return run_adj<2, false>(prob, beams, opts, ws, l, workspace_bytes, data, (double *)(ws + l.part), g, st,
                                          traj_src<2>(nullptr, nullptr, 1, 1));
-        default: return run_adj<3, false>(prob, beams, opts, ws, l, data, (double *)(ws + l.part), g, st,
+        default: return run_adj<3, false>(prob, beams, opts, ws, l, workspace_bytes, data, (double *)(ws + l.part), g, st,
                                           traj_src<3>(nullptr, nullptr, 1, 1));
     }
 }
@@ -1580,9 +1855,9 @@ extern "C" int msgb_sum_fwd_f32_traj(const msgb_problem *prob, const msgb_beam_s
     float *state = (float *)(ws + traj_state_offset(l));
     const int f = first_chunk != 0, la = last_chunk != 0;
     switch (prob->ndim) {
-        case 1: return run_fwd<1, true>(prob, beams, opts, ws, l, out, st, traj_src<1>(traj, state, f, la));
-        case 2: return run_fwd<2, true>(prob, beams, opts, ws, l, out, st, traj_src<2>(traj, state, f, la));
-        default: return run_fwd<3, true>(prob, beams, opts, ws, l, out, st, traj_src<3>(traj, state, f, la));
+        case 1: return run_fwd<1, true>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<1>(traj, state, f, la));
+        case 2: return run_fwd<2, true>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<2>(traj, state, f, la));
+        default: return run_fwd<3, true>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<3>(traj, state, f, la));
     }
 }
 
@@ -1603,9 +1878,9 @@ extern "C" int msgb_adj_gather_f32_traj(const msgb_problem *prob, const msgb_bea
     char *ws = (char *)workspace;
     double *part = (double *)(ws + traj_state_offset(l) + traj_state_bytes(prob));
     switch (prob->ndim) {
-        case 1: return run_adj<1, true>(prob, beams, opts, ws, l, data, part, g, st, traj_src<1>(traj, nullptr, 1, 1));
-        case 2: return run_adj<2, true>(prob, beams, opts, ws, l, data, part, g, st, traj_src<2>(traj, nullptr, 1, 1));
-        default: return run_adj<3, true>(prob, beams, opts, ws, l, data, part, g, st, traj_src<3>(traj, nullptr, 1, 1));
+        case 1: return run_adj<1, true>(prob, beams, opts, ws, l, workspace_bytes, data, part, g, st, traj_src<1>(traj, nullptr, 1, 1));
+        case 2: return run_adj<2, true>(prob, beams, opts, ws, l, workspace_bytes, data, part, g, st, traj_src<2>(traj, nullptr, 1, 1));
+        default: return run_adj<3, true>(prob, beams, opts, ws, l, workspace_bytes, data, part, g, st, traj_src<3>(traj, nullptr, 1, 1));
     }
 }
 
@@ -1731,8 +2006,8 @@ extern "C" int msgb_sum_fwd_f32_static(const msgb_problem *prob, const msgb_beam
     // scratch is written by this call's preparation kernels before it is read.
     char *ws = (char *)scratch;
     switch (prob->ndim) {
-        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
-        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
-        default: return run_fwd<3, false>(prob, beams, opts, ws, l, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
+        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
+        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
+        default: return run_fwd<3, false>(prob, beams, opts, ws, l, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
     }
 }
