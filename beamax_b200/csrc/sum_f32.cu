@@ -1002,8 +1002,59 @@ __device__ __forceinline__ void kahan_add(float &acc, float &cmp, float v) {
 
 constexpr int SCAN = 4;  // beams tested per thread and scan
 
-// Persistent CTAs take (time tile, sensor tile) work items from a counter.
-// Warp w owns sensor group w (GS sensors) of the tile; lane l owns time l.
+// A tile's beams in n ranges of len, each its own work item with a partial
+// (compensated sum, compensation) per output, added in order by
+// combine_parts_kernel.  n = 1: the item writes the output itself.
+struct Split {
+    int n;
+    int64_t len;
+    float2 *part;  // (n, ns, nt)
+};
+
+// Work items a launch should have: 8 per resident CTA (2 per SM), so that the
+// last, unevenly filled wave is a small part of it.  Fewer tiles than that are
+// split over the beams, in ranges of at least kSplitMin (8 passes of both modes).
+constexpr int64_t kItemsWanted = 8 * 2 * 148;
+constexpr int64_t kSplitMin = 128;
+
+// out (or the chunk state) = sum over the ranges, in order, and over earlier
+// chunks; one 32 x 32 block of (sorted sensor, time) per CTA.
+__global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *perm, int64_t nt, int64_t ns, float *state,
+                                     int first, int last, float *out) {
+    __shared__ float2 tile[32][33];
+    const int64_t s0 = (int64_t)blockIdx.x * 32, t0 = (int64_t)blockIdx.y * 32;
+    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+        const int64_t s = s0 + k, t = t0 + threadIdx.x;
+        float a = 0.0f, c = 0.0f;
+        if (s < ns && t < nt) {
+            for (int q = 0; q < n; ++q) {
+                const float2 v = part[((int64_t)q * ns + s) * nt + t];
+                kahan_add(a, c, v.x);
+                kahan_add(a, c, -v.y);
+            }
+        }
+        tile[k][threadIdx.x] = make_float2(a, c);
+    }
+    __syncthreads();
+    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+        const int64_t s = s0 + threadIdx.x, t = t0 + k;
+        if (s >= ns || t >= nt) continue;
+        float2 v = tile[threadIdx.x][k];
+        if (!first) {
+            kahan_add(v.x, v.y, state[t * ns + s]);
+            kahan_add(v.x, v.y, -state[(nt + t) * ns + s]);
+        }
+        if (last) {
+            out[t * ns + perm[s]] = v.x - v.y;
+        } else {
+            state[t * ns + s] = v.x;
+            state[(nt + t) * ns + s] = v.y;
+        }
+    }
+}
+
+// Persistent CTAs take (time tile, sensor tile, beam range) work items from a
+// counter.  Warp w owns sensor group w (GS sensors) of the tile; lane l owns time l.
 // Per item: beams are scanned 1024 at a time against the tile (survives /
 // traj_survives), survivors queue up, and every G of them make a record pass;
 // then each warp evaluates the pass's beams that reach its group, four at a
@@ -1016,7 +1067,7 @@ template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
 fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
              const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const int32_t *perm, float cutoff,
-             float *out, unsigned long long *eval_count, int *work, int n_st, int n_tiles, TrajSrc<D> T) {
+             float *out, unsigned long long *eval_count, int *work, int n_st, int n_items, Split sp, TrajSrc<D> T) {
     extern __shared__ float rec[];  // rec_bytes<D>()
     __shared__ float sds[TS][D], shn[TS][D];
     __shared__ TileGroups<D> ginfo;
@@ -1033,8 +1084,9 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
     while (true) {
         if (tid == 0) tile_s = atomicAdd(work, 1);
         __syncthreads();
-        const int tile = tile_s;
-        if (tile >= n_tiles) break;
+        const int item = tile_s;
+        if (item >= n_items) break;
+        const int tile = item / sp.n, part = item % sp.n;
         const int64_t st = tile % n_st, tt = tile / n_st;
         const int64_t s_first = offs[st], t_first = tt * TT;
         const int s_cnt = offs[st + 1] - offs[st];
@@ -1063,7 +1115,7 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
         float2 acc2[GS / 2], cmp2[GS / 2];
 #pragma unroll
         for (int h = 0; h < GS / 2; ++h) acc2[h] = make_float2(0.0f, 0.0f), cmp2[h] = make_float2(0.0f, 0.0f);
-        if (TRAJ && !T.first && lane < t_cnt && active) {
+        if (TRAJ && sp.n == 1 && !T.first && lane < t_cnt && active) {
             const int64_t t = t_first + lane;
 #pragma unroll
             for (int k = 0; k < GS; ++k) {
@@ -1078,10 +1130,11 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                 }
             }
         }
-        const int64_t nbeam = TRAJ ? T.nb : B.n;
+        const int64_t jb = part * sp.len;
+        const int64_t nbeam = min(jb + sp.len, TRAJ ? T.nb : B.n);
         int nq = 0;  // queued survivors (the same in every thread)
 
-        for (int64_t j0 = 0; j0 < nbeam; j0 += SCAN * THREADS) {
+        for (int64_t j0 = jb; j0 < nbeam; j0 += SCAN * THREADS) {
             unsigned bp[SCAN], bm[SCAN];
 #pragma unroll
             for (int k = 0; k < SCAN; ++k) {
@@ -1211,7 +1264,9 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                 if (s < s_cnt) {
                     const float a = (k & 1) ? acc2[k / 2].y : acc2[k / 2].x;
                     const float c = (k & 1) ? cmp2[k / 2].y : cmp2[k / 2].x;
-                    if (TRAJ && !T.last) {
+                    if (sp.n > 1) {
+                        sp.part[((int64_t)part * P.ns + s_first + s) * P.nt + t] = make_float2(a, c);
+                    } else if (TRAJ && !T.last) {
                         T.state[t * P.ns + s_first + s] = a;
                         T.state[(P.nt + t) * P.ns + s_first + s] = c;
                     } else {
@@ -1228,7 +1283,8 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
 // ------------------------------------------------------------------ adjoint
 // Deterministic tile-parallel transpose (no floating-point atomics).
 //
-// Work item = (time tile tt, range of RJ consecutive beam indices j): for the
+// Work item = (time tile tt, range of RJ consecutive beam indices j; fewer per
+// range when the launch would have too few items, kItemsWanted): for the
 // homogeneous entry point j is a selected coefficient and both of its modes
 // are summed; for trajectories j is a beam of the chunk.  Items run tt-major,
 // so consecutive items read the same time tile of the data.  For each sensor
@@ -1248,16 +1304,16 @@ struct AdjRange {
     // accumulator slots (re, im FP64) per item; 3D's larger records leave room
     // for half as many when two CTAs share an SM
     static constexpr int NACC = D == 3 ? 1024 : 2048;
-    static constexpr int RJ = TRAJ ? NACC : NACC / 2;  // beam indices per item
+    static constexpr int RJ = TRAJ ? NACC : NACC / 2;  // most beam indices per item
 };
 
 template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
 adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
              const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const float *dataT, float cutoff,
-             double *part, unsigned long long *eval_count, int *work, int n_st, int n_ranges, int n_items,
+             double *part, unsigned long long *eval_count, int *work, int n_st, int RJ, int n_ranges, int n_items,
              TrajSrc<D> T) {
-    constexpr int RJ = AdjRange<D, TRAJ>::RJ, NACC = AdjRange<D, TRAJ>::NACC;
+    constexpr int NACC = AdjRange<D, TRAJ>::NACC;
     extern __shared__ double acc_smem[];  // (NACC, 2), then the records
     float *rec = reinterpret_cast<float *>(acc_smem + 2 * NACC);
     __shared__ float sds[TS][D], shn[TS][D];
@@ -1464,7 +1520,7 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
         }
         __syncthreads();
         // every slot of the item, zeros included, then clear for the next item
-        for (int q = tid; q < NACC; q += THREADS) {
+        for (int q = tid; q < (TRAJ ? RJ : 2 * RJ); q += THREADS) {
             const int64_t jl = TRAJ ? q : (q < RJ ? q : q - RJ);
             const int64_t j = r0 + jl;
             if (j < r1) {
@@ -1565,6 +1621,32 @@ const HomBeam<D> *prepare_hom(const msgb_problem *p, const msgb_beam_set *b, cha
     return h;
 }
 
+// Ranges of the beams per tile for a forward over n_tiles tiles and nbeam beams
+// (2^62: as many as the tiles ask for).
+int split_count(int64_t n_tiles, int64_t nbeam) {
+    if (n_tiles <= 0) return 1;
+    const int64_t want = (kItemsWanted + n_tiles - 1) / n_tiles, most = (nbeam + kSplitMin - 1) / kSplitMin;
+    const int64_t n = want < most ? want : most;
+    return (int)(n < 1 ? 1 : n);
+}
+
+// Partials of the split forward for any tiling of the problem's sensors.
+size_t split_bytes(const msgb_problem *p, int64_t nbeam) {
+    const int64_t n = split_count((p->ns + TS - 1) / TS * ((p->nt + TT - 1) / TT), nbeam);
+    return n > 1 ? align256((size_t)n * (size_t)p->ns * (size_t)p->nt * sizeof(float2)) : 0;
+}
+
+// The ranges that fit in `spare` bytes at `at` (one range needs none).
+Split make_split(const msgb_problem *p, int64_t n_tiles, int64_t nbeam, char *at, size_t spare) {
+    const size_t per = (size_t)p->ns * (size_t)p->nt * sizeof(float2);
+    int64_t n = split_count(n_tiles, nbeam);
+    if (per * (size_t)n > spare) n = (int64_t)(spare / per);
+    if (n < 2) return Split{1, nbeam > 0 ? nbeam : 1, nullptr};
+    const int64_t len = ((nbeam + n - 1) / n + G - 1) / G * G;
+    n = (nbeam + len - 1) / len;
+    return Split{(int)n, len, n > 1 ? (float2 *)at : nullptr};
+}
+
 // Adjoint partials of a trajectory chunk of nb beams: (n_tt, nb) complex FP64.
 size_t traj_part_bytes(const msgb_problem *p, int64_t nb) {
     return align256((size_t)((p->nt + TT - 1) / TT) * (size_t)(nb > 0 ? nb : 0) * 16);
@@ -1643,7 +1725,7 @@ int sm_count() {
 
 template <int D, bool TRAJ>
 int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, char *ws, const Layout &l,
-            size_t ws_bytes, float *out, cudaStream_t st, TrajSrc<D> T) {
+            size_t ws_used, size_t ws_bytes, float *out, cudaStream_t st, TrajSrc<D> T) {
     // trajectory sums cull with the records' own boxes: the closed-form
     // culling table (sized for no beams in their layout) is not built
     msgb_beam_set none{};
@@ -1656,11 +1738,18 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     cudaMemsetAsync(work, 0, sizeof(int), st);
     bool periodic = false;
     for (int i = 0; i < D; ++i) periodic |= (p->periodic[i] != 0);
-    const int n_tiles = (int)(n_st * n_tt);
+    size_t at = ws_used, spare = ws_bytes - ws_used;
+    const HomBeam<D> *hom = nullptr;
+    if (!TRAJ) {
+        hom = prepare_hom<D>(p, b, ws + at, spare, st);
+        if (hom) at += hom_bytes(D, b->n), spare -= hom_bytes(D, b->n);
+    }
+    const Split sp = make_split(p, n_st * n_tt, TRAJ ? T.nb : b->n, ws + at, spare);
+    if (n_st * n_tt * sp.n > 0x7fffffffLL) return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: too many tiles");
+    const int n_items = (int)(n_st * n_tt * sp.n);
     const int64_t want = 2LL * sm_count();
-    const unsigned grid = (unsigned)(want < n_tiles ? want : n_tiles);
+    const unsigned grid = (unsigned)(want < n_items ? want : n_items);
     constexpr size_t smem = rec_bytes<D>();
-    const HomBeam<D> *hom = TRAJ ? nullptr : prepare_hom<D>(p, b, ws + l.total, ws_bytes - l.total, st);
     auto args = [&](auto kern) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull), hom,
@@ -1668,13 +1757,21 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
                                           (const float *)(ws + l.ds), (const float *)(ws + l.hn),
                                           (const uint8_t *)(ws + l.gfast), (const int32_t *)(ws + l.vals_out),
                                           o ? (float)o->cutoff : 0.0f, out, o ? o->eval_count : nullptr, work,
-                                          (int)n_st, n_tiles, T);
+                                          (int)n_st, n_items, sp, T);
     };
     if (periodic)
         args(fwd32_kernel<D, true, TRAJ>);
     else
         args(fwd32_kernel<D, false, TRAJ>);
-    return check_launch("msgb_sum_fwd_f32");
+    if (int e = check_launch("msgb_sum_fwd_f32")) return e;
+    if (sp.n > 1) {
+        const dim3 cg((unsigned)((p->ns + 31) / 32), (unsigned)n_tt);
+        if (cg.y > 65535u) return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: nt too large");
+        combine_parts_kernel<<<cg, dim3(32, 8), 0, st>>>(sp.part, sp.n, (const int32_t *)(ws + l.vals_out), p->nt, p->ns,
+                                                         T.state, T.first, T.last, out);
+        return check_launch("msgb_sum_fwd_f32 combine");
+    }
+    return MSGB_OK;
 }
 
 template <int D, bool TRAJ>
@@ -1692,7 +1789,10 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     for (int i = 0; i < D; ++i) periodic |= (p->periodic[i] != 0);
     const int64_t nw = TRAJ ? T.nb : b->n;  // beam indices j of the items
     const int64_t n_st = l.n_st, n_tt = (p->nt + TT - 1) / TT;
-    const int64_t n_ranges = (nw + AdjRange<D, TRAJ>::RJ - 1) / AdjRange<D, TRAJ>::RJ;
+    constexpr int64_t RJ = AdjRange<D, TRAJ>::RJ;
+    int64_t rj = nw * n_tt / kItemsWanted / G * G;
+    rj = rj > RJ ? RJ : (rj < G ? G : rj);
+    const int64_t n_ranges = (nw + rj - 1) / rj;
     if (n_ranges * n_tt > 0x7fffffffLL || n_st > 0x7fffffffLL)
         return fail(MSGB_ERR_UNSUPPORTED, "msgb_adj_gather_f32: too many work items");
     int *work = (int *)(ws + l.work);
@@ -1710,7 +1810,7 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
                                           (const float *)(ws + l.ds), (const float *)(ws + l.hn),
                                           (const uint8_t *)(ws + l.gfast), (const float *)(ws + l.data),
                                           o ? (float)o->cutoff : 0.0f, part, o ? o->eval_count : nullptr, work,
-                                          (int)n_st, (int)n_ranges, n_items, T);
+                                          (int)n_st, (int)rj, (int)n_ranges, n_items, T);
     };
     if (periodic)
         args(adj32_kernel<D, true, TRAJ>);
@@ -1753,7 +1853,8 @@ extern "C" size_t msgb_sum_f32_workspace_size(const msgb_problem *prob, int64_t 
     // The default tiling has the most tiles a valid tiling of ns sensors needs
     // when every tile is full; reserve for one tile per 16 sensors so that
     // caller tilings with partial tiles fit as well.
-    return layout(prob, n, true, (prob->ns + GS - 1) / GS).total + hom_bytes(prob->ndim, n);
+    return layout(prob, n, true, (prob->ns + GS - 1) / GS).total + hom_bytes(prob->ndim, n) +
+           split_bytes(prob, n);
 }
 
 static int check_ws(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, bool with_data, void *ws,
@@ -1779,9 +1880,9 @@ extern "C" int msgb_sum_fwd_f32(const msgb_problem *prob, const msgb_beam_set *b
     cudaStream_t st = as_stream(stream);
     char *ws = (char *)workspace;
     switch (prob->ndim) {
-        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
-        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
-        default: return run_fwd<3, false>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
+        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, l.total, workspace_bytes, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
+        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, l.total, workspace_bytes, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
+        default: return run_fwd<3, false>(prob, beams, opts, ws, l, l.total, workspace_bytes, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
     }
 }
 
@@ -1818,7 +1919,9 @@ static size_t traj_state_bytes(const msgb_problem *p) { return align256((size_t)
 extern "C" size_t msgb_sum_f32_traj_workspace_size(const msgb_problem *prob, int64_t nb_max) {
     if (validate_problem(prob) || nb_max < 0) return 0;
     const Layout l = layout(prob, 0, true, (prob->ns + GS - 1) / GS);
-    return l.total + traj_state_bytes(prob) + traj_part_bytes(prob, nb_max);
+    // after the Kahan state: the adjoint's partials, or those of the split forward
+    const size_t part = traj_part_bytes(prob, nb_max), split = split_bytes(prob, int64_t(1) << 62);
+    return l.total + traj_state_bytes(prob) + (part > split ? part : split);
 }
 
 // with_part: the adjoint's partials (n_tt, nb) follow the Kahan state.
@@ -1855,9 +1958,9 @@ extern "C" int msgb_sum_fwd_f32_traj(const msgb_problem *prob, const msgb_beam_s
     float *state = (float *)(ws + traj_state_offset(l));
     const int f = first_chunk != 0, la = last_chunk != 0;
     switch (prob->ndim) {
-        case 1: return run_fwd<1, true>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<1>(traj, state, f, la));
-        case 2: return run_fwd<2, true>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<2>(traj, state, f, la));
-        default: return run_fwd<3, true>(prob, beams, opts, ws, l, workspace_bytes, out, st, traj_src<3>(traj, state, f, la));
+        case 1: return run_fwd<1, true>(prob, beams, opts, ws, l, traj_state_offset(l) + traj_state_bytes(prob), workspace_bytes, out, st, traj_src<1>(traj, state, f, la));
+        case 2: return run_fwd<2, true>(prob, beams, opts, ws, l, traj_state_offset(l) + traj_state_bytes(prob), workspace_bytes, out, st, traj_src<2>(traj, state, f, la));
+        default: return run_fwd<3, true>(prob, beams, opts, ws, l, traj_state_offset(l) + traj_state_bytes(prob), workspace_bytes, out, st, traj_src<3>(traj, state, f, la));
     }
 }
 
@@ -2006,8 +2109,8 @@ extern "C" int msgb_sum_fwd_f32_static(const msgb_problem *prob, const msgb_beam
     // scratch is written by this call's preparation kernels before it is read.
     char *ws = (char *)scratch;
     switch (prob->ndim) {
-        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
-        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
-        default: return run_fwd<3, false>(prob, beams, opts, ws, l, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
+        case 1: return run_fwd<1, false>(prob, beams, opts, ws, l, l.total, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<1>(nullptr, nullptr, 1, 1));
+        case 2: return run_fwd<2, false>(prob, beams, opts, ws, l, l.total, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<2>(nullptr, nullptr, 1, 1));
+        default: return run_fwd<3, false>(prob, beams, opts, ws, l, l.total, (size_t)MSGB_SUM_F32_STATIC_SCRATCH_BYTES, out, st, traj_src<3>(nullptr, nullptr, 1, 1));
     }
 }
