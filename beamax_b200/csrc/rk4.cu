@@ -331,6 +331,59 @@ constexpr size_t dopri_mix_smem_bytes(int blk) {
 }
 constexpr int kMixBlocks = 6;  // default blocks per SM of the mixed-precision integrator (measured best at config 3)
 
+// A lane's stages in shared memory, every integrator block having 64 lanes:
+// stage j holds its N values as N / 2 pairs (FP64) or as quads and a pair (FP32),
+// each vector strided by the block, so that a stage moves with 16-byte accesses at
+// immediate offsets and without bank conflicts.
+constexpr int kOdeBlock = 64;
+
+template <int N>
+struct Stages64 {
+    static_assert(N % 2 == 0, "pairs");
+    double2 *at;
+    __device__ __forceinline__ void get(int j, double *v) const {
+#pragma unroll
+        for (int c = 0; c < N / 2; ++c) {
+            const double2 q = at[(j * (N / 2) + c) * kOdeBlock];
+            v[2 * c] = q.x;
+            v[2 * c + 1] = q.y;
+        }
+    }
+    __device__ __forceinline__ double one(int j, int c) const {
+        const double2 &q = at[(j * (N / 2) + c / 2) * kOdeBlock];
+        return c % 2 ? q.y : q.x;
+    }
+    __device__ __forceinline__ void put(int j, const double *v) const {
+#pragma unroll
+        for (int c = 0; c < N / 2; ++c) at[(j * (N / 2) + c) * kOdeBlock] = make_double2(v[2 * c], v[2 * c + 1]);
+    }
+};
+
+template <int N>
+struct Stages32 {
+    static_assert(N % 2 == 0, "quads and at most one pair");
+    static constexpr int Q = N / 4, R = N % 4 ? 1 : 0;  // quads, pairs
+    float4 *at;
+    float2 *at2;
+    __device__ __forceinline__ void get(int j, float *v) const {
+#pragma unroll
+        for (int c = 0; c < Q; ++c) {
+            const float4 q = at[(j * Q + c) * kOdeBlock];
+            v[4 * c] = q.x, v[4 * c + 1] = q.y, v[4 * c + 2] = q.z, v[4 * c + 3] = q.w;
+        }
+        if (R) {
+            const float2 q = at2[j * kOdeBlock];
+            v[N - 2] = q.x, v[N - 1] = q.y;
+        }
+    }
+    __device__ __forceinline__ void put(int j, const float *v) const {
+#pragma unroll
+        for (int c = 0; c < Q; ++c)
+            at[(j * Q + c) * kOdeBlock] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        if (R) at2[j * kOdeBlock] = make_float2(v[N - 2], v[N - 1]);
+    }
+};
+
 // DENSE: save times may fall inside a step (msgb_ode_opts.dense_output);
 // without it every step ends on a save time and the continuous extension is
 // not compiled (it is what pushed the kernel past 255 registers).
@@ -341,8 +394,8 @@ struct DopriBeam {
     int64_t steps, k;
     bool rejected;
     int code;  // 0 running or done, 1 non-finite, 2 step budget exhausted
-    double *ks;  // this lane's stages in shared memory: stage j, entry c at ks[(j N + c) kst]
-    int kst;
+    Stages64<NVS<D>::value> ks;  // this lane's stages
+    __device__ DopriBeam() { ks.at = reinterpret_cast<double2 *>(dopri_stage_smem) + threadIdx.x; }
 
     __device__ void init(const MediumArgs &med, const ProbArgs &P, const OdeArgs &o, double mode_) {
         mode = mode_;
@@ -354,9 +407,7 @@ struct DopriBeam {
         code = 0;
         SState<D> f0;
         rhs_sym<D, KIND, F32M>(med, mode, y, f0);
-        const double *fv = vals(f0);
-#pragma unroll
-        for (int c = 0; c < NVS<D>::value; ++c) ks[c * kst] = fv[c];
+        ks.put(0, vals(f0));
     }
 
     // One attempt; returns true when the beam is finished (all save times
@@ -397,8 +448,10 @@ struct DopriBeam {
             for (int j = 0; j < s; ++j) {
                 const double a = DP_A[s][j];
                 if (a != 0.0) {
+                    double kj[N];
+                    ks.get(j, kj);
 #pragma unroll
-                    for (int c = 0; c < N; ++c) acc[c] += a * ks[(j * N + c) * kst];
+                    for (int c = 0; c < N; ++c) acc[c] += a * kj[c];
                 }
             }
             double *tv = vals(yt);
@@ -406,22 +459,24 @@ struct DopriBeam {
             for (int c = 0; c < N; ++c) tv[c] = yv[c] + hh * acc[c];
             SState<D> kn;
             rhs_sym<D, KIND, F32M>(med, mode, yt, kn);
-            const double *kv = vals(kn);
-#pragma unroll
-            for (int c = 0; c < N; ++c) ks[(s * N + c) * kst] = kv[c];
+            ks.put(s, vals(kn));
         }
-#define KSV(j, c) ks[((j) * N + (c)) * kst]
         // yt now holds the 5th-order solution (stage 7's input).
         const double *nv = vals(yt);
         double err;
         {
             double ev[N];
 #pragma unroll
-            for (int c = 0; c < N; ++c) {
-                double acc = 0.0;
-                for (int j = 0; j < 7; ++j) acc += DP_E[j] * KSV(j, c);
-                ev[c] = hh * acc;
+            for (int c = 0; c < N; ++c) ev[c] = 0.0;
+#pragma unroll
+            for (int j = 0; j < 7; ++j) {
+                double kj[N];
+                ks.get(j, kj);
+#pragma unroll
+                for (int c = 0; c < N; ++c) ev[c] += DP_E[j] * kj[c];
             }
+#pragma unroll
+            for (int c = 0; c < N; ++c) ev[c] = hh * ev[c];
             // (|e| / (atol + rtol max(|y0|, |y1|)))^2 from squared magnitudes:
             // one square root per entry instead of three.  The FP32 path
             // forms the norm, a step-size heuristic, in FP32.
@@ -470,12 +525,12 @@ struct DopriBeam {
                         double r5 = 0.0;
                         for (int j = 0; j < 7; ++j) {
                             const double dj = DP_D[j];
-                            if (dj != 0.0) r5 += dj * KSV(j, c);
+                            if (dj != 0.0) r5 += dj * ks.one(j, c);
                         }
                         r5 *= hh;
                         const double r2 = nv[c] - yv[c];
-                        const double r3 = hh * KSV(0, c) - r2;
-                        const double r4 = r2 - hh * KSV(6, c) - r3;
+                        const double r3 = hh * ks.one(0, c) - r2;
+                        const double r4 = r2 - hh * ks.one(6, c) - r3;
                         dv[c] = yv[c] + th * (r2 + (1.0 - th) * (r3 + th * (r4 + (1.0 - th) * r5)));
                     }
                     State<D> yf;
@@ -486,9 +541,9 @@ struct DopriBeam {
             }
             t = t_new;
             y = yt;
-#pragma unroll
-            for (int c = 0; c < N; ++c) KSV(0, c) = KSV(6, c);  // first same as last
-#undef KSV
+            double k6[N];
+            ks.get(6, k6);  // first same as last
+            ks.put(0, k6);
             h = (last && !o.dense_output) ? fmax(hh * fac, h) : hh * fac;
         } else {
             h = hh * fmin(1.0, fac);
@@ -674,11 +729,15 @@ struct DopriMix {
     int64_t steps, k;
     bool rejected;
     int code;
-    double *k64;  // stage j, entry c at k64[(j ND + c) kst]
-    float *k32;   // stage j, entry c at k32[(j NF + c) kst]
-    // the block size (every integrator launch has 64 lanes): a compile-time
-    // stride turns the stage addresses into immediate offsets
-    static constexpr int kst = 64;
+    Stages64<ND> k64;
+    Stages32<NF> k32;
+    __device__ DopriMix() {
+        // 7 FP64 stages, then 7 FP32 ones: quads, then pairs
+        k64.at = reinterpret_cast<double2 *>(dopri_stage_smem) + threadIdx.x;
+        float4 *q = reinterpret_cast<float4 *>(dopri_stage_smem + 7 * ND * kOdeBlock);
+        k32.at = q + threadIdx.x;
+        k32.at2 = reinterpret_cast<float2 *>(q + 7 * Stages32<NF>::Q * kOdeBlock) + threadIdx.x;
+    }
 
     __device__ void init(const MediumArgs &med, const ProbArgs &P, const OdeArgs &o, double mode_) {
         mode = mode_;
@@ -690,10 +749,8 @@ struct DopriMix {
         code = 0;
         MState<D> f0;
         rhs_mix<D, KIND>(med, mode, y, f0);
-#pragma unroll
-        for (int c = 0; c < ND; ++c) k64[c * kst] = f0.r[c];
-#pragma unroll
-        for (int c = 0; c < NF; ++c) k32[c * kst] = f0.f[c];
+        k64.put(0, f0.r);
+        k32.put(0, f0.f);
     }
 
     __device__ bool attempt(const MediumArgs &med, const ProbArgs &P, const OdeArgs &o, RecordWriter<D> &rw) {
@@ -712,7 +769,7 @@ struct DopriMix {
             last = true;
         }
         const float hf = (float)hh;
-        MState<D> yt;
+        MState<D> yt, kn;
 #pragma unroll 1
         for (int s = 1; s < 7; ++s) {
             double a64[ND];
@@ -724,47 +781,60 @@ struct DopriMix {
 #pragma unroll 1
             for (int j = 0; j < s; ++j) {
                 const double a = DP_A[s][j];
-                if (a != 0.0) {
-                    const float af = DP_A32[s][j];
+                const float af = DP_A32[s][j];
+                double r[ND];
+                float f[NF];
+                k64.get(j, r);
+                k32.get(j, f);
 #pragma unroll
-                    for (int c = 0; c < ND; ++c) a64[c] += a * k64[(j * ND + c) * kst];
+                for (int c = 0; c < ND; ++c) a64[c] += a * r[c];
 #pragma unroll
-                    for (int c = 0; c < NF; ++c) a32[c] = fmaf(af, k32[(j * NF + c) * kst], a32[c]);
-                }
+                for (int c = 0; c < NF; ++c) a32[c] = fmaf(af, f[c], a32[c]);
             }
 #pragma unroll
             for (int c = 0; c < ND; ++c) yt.r[c] = y.r[c] + hh * a64[c];
 #pragma unroll
             for (int c = 0; c < NF; ++c) yt.f[c] = fmaf(hf, a32[c], y.f[c]);
-            MState<D> kn;
             rhs_mix<D, KIND>(med, mode, yt, kn);
-#pragma unroll
-            for (int c = 0; c < ND; ++c) k64[(s * ND + c) * kst] = kn.r[c];
-#pragma unroll
-            for (int c = 0; c < NF; ++c) k32[(s * NF + c) * kst] = kn.f[c];
+            if (s < 6) {  // the last stage stays in registers
+                k64.put(s, kn.r);
+                k32.put(s, kn.f);
+            }
         }
         // yt holds the 5th-order solution.  Error norm in FP32, as DopriBeam's
         // FP32-path variant forms it.
         float s32 = 0.0f;
         {
+            double e64[ND];
+            float e32[NF];
+#pragma unroll
+            for (int c = 0; c < ND; ++c) e64[c] = 0.0;
+#pragma unroll
+            for (int c = 0; c < NF; ++c) e32[c] = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 7; ++j) {
+                double r[ND];
+                float f[NF];
+                if (j == 1) continue;  // weight 0
+                if (j < 6) {
+                    k64.get(j, r);
+                    k32.get(j, f);
+                }
+#pragma unroll
+                for (int c = 0; c < ND; ++c) e64[c] += DP_E[j] * (j < 6 ? r[c] : kn.r[c]);
+#pragma unroll
+                for (int c = 0; c < NF; ++c) e32[c] = fmaf(DP_E32[j], j < 6 ? f[c] : kn.f[c], e32[c]);
+            }
             const float at = (float)o.atol, rt = (float)o.rtol;
 #pragma unroll
             for (int c = 0; c < ND; ++c) {
-                double acc = 0.0;
-                for (int j = 0; j < 7; ++j) acc += DP_E[j] * k64[(j * ND + c) * kst];
-                const float e = (float)(hh * acc);
+                const float e = (float)(hh * e64[c]);
                 const float sc = fmaf(rt, (float)fmax(fabs(y.r[c]), fabs(yt.r[c])), at);
                 s32 = fmaf(e, __fdividef(e, sc * sc), s32);
             }
 #pragma unroll
             for (int q = 0; q < S + 1; ++q) {
-                float er = 0.0f, ei = 0.0f;
-                for (int j = 0; j < 7; ++j) {
-                    er = fmaf(DP_E32[j], k32[(j * NF + 2 * q) * kst], er);
-                    ei = fmaf(DP_E32[j], k32[(j * NF + 2 * q + 1) * kst], ei);
-                }
-                er *= hf;
-                ei *= hf;
+                const float er = e32[2 * q] * hf, ei = e32[2 * q + 1] * hf;
                 const float y0 = fmaf(y.f[2 * q], y.f[2 * q], y.f[2 * q + 1] * y.f[2 * q + 1]);
                 const float y1 = fmaf(yt.f[2 * q], yt.f[2 * q], yt.f[2 * q + 1] * yt.f[2 * q + 1]);
                 const float sc = fmaf(rt, sqrtf(fmaxf(y0, y1)), at);
@@ -792,10 +862,8 @@ struct DopriMix {
             }
             t = t_new;
             y = yt;
-#pragma unroll
-            for (int c = 0; c < ND; ++c) k64[c * kst] = k64[(6 * ND + c) * kst];  // first same as last
-#pragma unroll
-            for (int c = 0; c < NF; ++c) k32[c * kst] = k32[(6 * NF + c) * kst];
+            k64.put(0, kn.r);  // first same as last
+            k32.put(0, kn.f);
             h = last ? fmax(hh * fac, h) : hh * fac;
         } else {
             h = hh * fmin(1.0, fac);
@@ -830,14 +898,12 @@ __device__ void launch_state(const BeamArgs &B, const TrajArgs &T, int64_t bl, S
 // (the stages take 43 KB of shared memory per block in 2D, so at most 5 fit).
 template <int D, int KIND, int MINB, bool F32M, bool DENSE>
 __global__ void __launch_bounds__(64, MINB)
-dopri_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o, int tt_len) {
+dopri_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t bl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - stride;
     bool active = false;
     DopriBeam<D, KIND, F32M, DENSE> s;
-    s.ks = dopri_stage_smem + threadIdx.x;
-    s.kst = blockDim.x;
-    RecordWriter<D> rw(P, T, 0, 0.0, tt_len);
+    RecordWriter<D> rw(P, T, 0, 0.0);
     unsigned long long lane_steps = 0;
     for (;;) {
         if (!active) {
@@ -880,15 +946,13 @@ dopri_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o, int 
 // dopri_kernel with the FP32 path's mixed-precision state (DopriMix).
 template <int D, int KIND, int MINB>
 __global__ void __launch_bounds__(64, MINB)
-dopri_mix_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o, int tt_len) {
+dopri_mix_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) {
     constexpr int ND = MState<D>::ND;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t bl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - stride;
     bool active = false;
     DopriMix<D, KIND> s;
-    s.k64 = dopri_stage_smem + threadIdx.x;
-    s.k32 = reinterpret_cast<float *>(dopri_stage_smem + 7 * ND * DopriMix<D, KIND>::kst) + threadIdx.x;
-    RecordWriter<D> rw(P, T, 0, 0.0, tt_len);
+    RecordWriter<D> rw(P, T, 0, 0.0);
     unsigned long long lane_steps = 0;
     for (;;) {
         if (!active) {
@@ -931,7 +995,7 @@ dopri_mix_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o, 
 
 // Fixed-step RK4, one thread per beam.
 template <int D>
-__global__ void rk4_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o, int tt_len) {
+__global__ void rk4_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) {
     const int64_t bl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (bl >= T.nb) return;
     if (o.only_flagged && T.status[bl] == 0) return;  // records already accepted
@@ -950,8 +1014,7 @@ __global__ void rk4_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, O
     y.A = cd{1.0, 0.0};
     const double w = B.omega[j];
     int code = 0;
-    RecordWriter<D> rw(P, T, bl, w, tt_len);
-    const int64_t n_tt = (P.nt + tt_len - 1) / tt_len;
+    RecordWriter<D> rw(P, T, bl, w);
     for (int64_t k = 0; k < P.nt; ++k) {
         if (k > 0 && code == 0) {
             const double hs = (P.ts[k] - P.ts[k - 1]) / o.substeps;
@@ -963,7 +1026,6 @@ __global__ void rk4_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, O
         if (!fin && code == 0) code = 1;
         rw.put(k, y, code != 0);
     }
-    (void)n_tt;
     if (T.status) T.status[bl] = code;
 }
 
@@ -982,8 +1044,6 @@ __global__ void tr_final_kernel(ProbArgs P, MediumArgs med, TrBeamsView B, int64
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     DopriBeam<D, KIND> s;
-    s.ks = dopri_stage_smem + threadIdx.x;
-    s.kst = blockDim.x;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         s.y.x[a] = B.x[i * D + a];
@@ -1001,7 +1061,7 @@ __global__ void tr_final_kernel(ProbArgs P, MediumArgs med, TrBeamsView B, int64
         Pl.nt = 2;
         Pl.ts = tl;
         TrajArgs T{n, 0, n, nullptr, nullptr, nullptr, nullptr};  // records written below
-        RecordWriter<D> rw(Pl, T, i, 1.0, 2);
+        RecordWriter<D> rw(Pl, T, i, 1.0);
         s.init(med, Pl, o, -B.mode[i]);
         while (!s.attempt(med, Pl, o, rw)) {
         }
@@ -1105,7 +1165,7 @@ extern "C" int msgb_tr_final_states(const msgb_problem *prob, const msgb_medium 
     OdeArgs O{opts->method, opts->substeps, opts->rtol, opts->atol, opts->dt0, opts->max_steps, 0,
               opts->dense_output, nullptr};
     TrBeamsView B{beams->x, beams->p, beams->M, beams->mode, beams->t0};
-    const int blk = 64;
+    const int blk = kOdeBlock;
     const unsigned grid = (unsigned)((beams->n + blk - 1) / blk);
     cudaStream_t st = as_stream(stream);
     switch (prob->ndim) {
@@ -1149,15 +1209,15 @@ extern "C" int msgb_ode_trajectories(const msgb_problem *prob, const msgb_medium
     if (int e = check_compact(out, prob->ndim)) return e;
     TrajArgs T{out->nb, out->b_first, beams->n, out->rec64, out->rec32, out->cull, out->status};
     set_compact(T, out);
-    const int blk = 64;
+    const int blk = kOdeBlock;
     const int64_t need = (out->nb + blk - 1) / blk;
     cudaStream_t st = as_stream(stream);
     if (O.method == MSGB_ODE_RK4) {
         const unsigned grid = (unsigned)need;
         switch (prob->ndim) {
-            case 1: rk4_kernel<1><<<grid, blk, 0, st>>>(P, M, to_args(beams), T, O, MSGB_TIME_TILE); break;
-            case 2: rk4_kernel<2><<<grid, blk, 0, st>>>(P, M, to_args(beams), T, O, MSGB_TIME_TILE); break;
-            default: rk4_kernel<3><<<grid, blk, 0, st>>>(P, M, to_args(beams), T, O, MSGB_TIME_TILE); break;
+            case 1: rk4_kernel<1><<<grid, blk, 0, st>>>(P, M, to_args(beams), T, O); break;
+            case 2: rk4_kernel<2><<<grid, blk, 0, st>>>(P, M, to_args(beams), T, O); break;
+            default: rk4_kernel<3><<<grid, blk, 0, st>>>(P, M, to_args(beams), T, O); break;
         }
     } else {
         // enough resident lanes for every SM, each taking several beams
@@ -1177,11 +1237,11 @@ extern "C" int msgb_ode_trajectories(const msgb_problem *prob, const msgb_medium
         const int64_t want = (int64_t)which.minb * sms;
         const unsigned grid = (unsigned)(need < want ? need : want);
         switch (prob->ndim) {
-            case 1: launch_by_kind<1>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O, MSGB_TIME_TILE); },
+            case 1: launch_by_kind<1>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O); },
                                       which); break;
-            case 2: launch_by_kind<2>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O, MSGB_TIME_TILE); },
+            case 2: launch_by_kind<2>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O); },
                                       which); break;
-            default: launch_by_kind<3>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O, MSGB_TIME_TILE); },
+            default: launch_by_kind<3>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O); },
                                        which); break;
         }
     }

@@ -223,7 +223,7 @@ __global__ void records_kernel(ProbArgs P, MediumArgs med, BeamArgs B, SurrIO io
     const double Lc = l.c0 * Tt;
     const double H0 = l.c0 * l.np;
     const int64_t ob = io.b_first - T.b_first + bl;  // index within the trajectory chunk
-    RecordWriter<D> rw(P, T, ob, l.w, tt_len);
+    RecordWriter<D> rw(P, T, ob, l.w);
     double res = 0.0;
     bool finite = true;
     for (int64_t k = 0; k < P.nt; ++k) {

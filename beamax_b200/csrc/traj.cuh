@@ -18,6 +18,9 @@ struct MediumArgs {
     double c, lam;
     const float *coeffs32;  // (coeffs - c_ref) in FP32, or nullptr
     double c_ref;
+    // factors of the interpolant's sums (see speed_eval_k): the value's, the
+    // gradient's per axis and the Hessian's per pair of axes
+    double sv, sg[3], sh[3][3];
 };
 
 __device__ __forceinline__ int map_index(int i, int n, int boundary) {
@@ -30,10 +33,48 @@ __device__ __forceinline__ int map_index(int i, int n, int boundary) {
     }
 }
 
-// Tap k of the `taps` consecutive taps starting at lo: inside the grid (the
-// usual case) the index itself, else the boundary rule.
-__device__ __forceinline__ int tap_index(int lo, int k, int taps, int n, int boundary) {
-    return (lo >= 0 && lo + taps <= n) ? lo + k : map_index(lo + k, n, boundary);
+// Indices of the 4 (cubic) or 2 taps starting at lo by the boundary rule: only
+// for cells at the edge of the grid, kept out of the integrators' loop.
+static __device__ __noinline__ int4 edge_taps(int lo, int n, int boundary) {
+    return make_int4(map_index(lo, n, boundary), map_index(lo + 1, n, boundary), map_index(lo + 2, n, boundary),
+                     map_index(lo + 3, n, boundary));
+}
+
+// The taps x taps values of a 2D stencil whose first tap is (lo0, lo1): inside
+// the grid (the usual case) from one base address with constant row offsets.
+template <int TAPS, typename T>
+__device__ __forceinline__ void gather_plane(const T *__restrict__ g, const int *n, int lo0, int lo1, int boundary,
+                                             T (*v)[4]) {
+    if (lo0 >= 0 && lo0 <= n[0] - TAPS && lo1 >= 0 && lo1 <= n[1] - TAPS) {
+        const T *p = g + ((int64_t)lo0 * n[1] + lo1);
+#pragma unroll
+        for (int i = 0; i < TAPS; ++i) {
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) v[i][k] = __ldg(p + k);
+            p += n[1];
+        }
+        return;
+    }
+    const int4 a = edge_taps(lo0, n[0], boundary), b = edge_taps(lo1, n[1], boundary);
+    const int ia[4] = {a.x, a.y, a.z, a.w}, ib[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i)
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) v[i][k] = __ldg(g + ((int64_t)ia[i] * n[1] + ib[k]));
+}
+
+// The taps along one axis starting at lo (offsets into that axis).
+template <int TAPS>
+__device__ __forceinline__ void axis_taps(int lo, int n, int boundary, int *idx) {
+    if (lo >= 0 && lo <= n - TAPS) {
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) idx[k] = lo + k;
+        return;
+    }
+    const int4 a = edge_taps(lo, n, boundary);
+    const int ia[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) idx[k] = ia[k];
 }
 
 // c, grad c (D), hess c (D x D, row-major) at x, for a medium of kind KIND
@@ -54,7 +95,7 @@ __device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *
     constexpr int taps = cubic ? 4 : 2;
     constexpr int off0 = cubic ? -1 : 0;
     double w[D][4], d1[D][4], d2[D][4];
-    int idx[D][4];
+    int lo[D], idx[D][4];
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         const double u = (x[a] - m.origin[a]) * m.inv_spacing[a];
@@ -85,8 +126,8 @@ __device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *
             d2[a][0] = d2[a][1] = 0.0;
             w[a][2] = w[a][3] = d1[a][2] = d1[a][3] = d2[a][2] = d2[a][3] = 0.0;
         }
-#pragma unroll
-        for (int k = 0; k < taps; ++k) idx[a][k] = tap_index(i0 + off0, k, taps, m.n[a], m.boundary);
+        lo[a] = i0 + off0;
+        if (D != 2) axis_taps<taps>(lo[a], m.n[a], m.boundary, idx[a]);
     }
     // Separable reduction, last axis first: the tensor-product weights factor,
     // so the value, gradient and Hessian need 3 sums per line of the last
@@ -108,13 +149,14 @@ __device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *
         }
     } else if (D == 2) {
         const int L = D - 1;  // last axis
+        double v2[4][4];
+        gather_plane<taps>(m.coeffs, m.n, lo[0], lo[L], m.boundary, v2);
 #pragma unroll
         for (int i = 0; i < taps; ++i) {
-            const double *row = m.coeffs + (int64_t)idx[0][i] * m.n[L];
             double rw = 0.0, rd = 0.0, rdd = 0.0;
 #pragma unroll
             for (int k = 0; k < taps; ++k) {
-                const double v = __ldg(row + idx[L][k]);
+                const double v = v2[i][k];
                 rw = fma(w[L][k], v, rw);
                 rd = fma(d1[L][k], v, rd);
                 rdd = fma(d2[L][k], v, rdd);
@@ -161,22 +203,13 @@ __device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *
             hh[Z][Z] = fma(w[0][i], tzz, hh[Z][Z]);
         }
     }
-    // Cubic weights were 6 x the true ones: a sum whose terms carry the plain
-    // weight of q axes is 6^q too large (value: D axes; gradient: D - 1;
-    // diagonal Hessian: D - 1; mixed Hessian: D - 2).
-    constexpr double s6 = cubic ? 1.0 / 6.0 : 1.0;
-    constexpr double sv = D == 1 ? s6 : (D == 2 ? s6 * s6 : s6 * s6 * s6);
-    constexpr double sg = D == 1 ? 1.0 : (D == 2 ? s6 : s6 * s6);
-    constexpr double sm = D == 3 ? s6 : 1.0;
-    c = cc * sv;
+    // (the cubic weights are 6 x the true ones: see medium_args for the factors)
+    c = cc * m.sv;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-        g[a] = gg[a] * (sg * m.inv_spacing[a]);
+        g[a] = gg[a] * m.sg[a];
 #pragma unroll
-        for (int b = 0; b < D; ++b) {
-            const double hv = a <= b ? hh[a][b] : hh[b][a];
-            H[a * D + b] = hv * ((a == b ? sg : sm) * m.inv_spacing[a] * m.inv_spacing[b]);
-        }
+        for (int b = 0; b < D; ++b) H[a * D + b] = (a <= b ? hh[a][b] : hh[b][a]) * m.sh[a][b];
     }
 }
 
@@ -194,7 +227,7 @@ __device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double
     constexpr int off0 = cubic ? -1 : 0;
     constexpr int ctr = cubic ? 1 : 0;  // the tap at the cell's lower corner
     float w[D][4], d1[D][4], d2[D][4];
-    int idx[D][4];
+    int lo[D], idx[D][4];
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         const double u = (x[a] - m.origin[a]) * m.inv_spacing[a];
@@ -223,8 +256,8 @@ __device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double
             d2[a][0] = d2[a][1] = 0.0f;
             w[a][2] = w[a][3] = d1[a][2] = d1[a][3] = d2[a][2] = d2[a][3] = 0.0f;
         }
-#pragma unroll
-        for (int k = 0; k < taps; ++k) idx[a][k] = tap_index(i0 + off0, k, taps, m.n[a], m.boundary);
+        lo[a] = i0 + off0;
+        if (D != 2) axis_taps<taps>(lo[a], m.n[a], m.boundary, idx[a]);
     }
     float cc = 0.0f, gg[D], hh[D][D];
 #pragma unroll
@@ -245,14 +278,15 @@ __device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double
         }
     } else if (D == 2) {
         const int L = D - 1;
-        vc = __ldg(m.coeffs32 + (int64_t)idx[0][ctr] * m.n[L] + idx[L][ctr]);
+        float v2[4][4];
+        gather_plane<taps>(m.coeffs32, m.n, lo[0], lo[L], m.boundary, v2);
+        vc = v2[ctr][ctr];
 #pragma unroll
         for (int i = 0; i < taps; ++i) {
-            const float *row = m.coeffs32 + (int64_t)idx[0][i] * m.n[L];
             float rw = 0.0f, rd = 0.0f, rdd = 0.0f;
 #pragma unroll
             for (int k = 0; k < taps; ++k) {
-                const float v = __ldg(row + idx[L][k]) - vc;
+                const float v = v2[i][k] - vc;
                 rw = fmaf(w[L][k], v, rw);
                 rd = fmaf(d1[L][k], v, rd);
                 rdd = fmaf(d2[L][k], v, rdd);
@@ -300,20 +334,14 @@ __device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double
             hh[Z][Z] = fmaf(w[0][i], tzz, hh[Z][Z]);
         }
     }
-    constexpr double s6 = cubic ? 1.0 / 6.0 : 1.0;
-    constexpr double sv = D == 1 ? s6 : (D == 2 ? s6 * s6 : s6 * s6 * s6);
-    constexpr double sg = D == 1 ? 1.0 : (D == 2 ? s6 : s6 * s6);
-    constexpr double sm = D == 3 ? s6 : 1.0;
+    // (the cubic weights are 6 x the true ones: see medium_args for the factors)
     // the value's weights sum to 1: the centre comes back in FP64
-    c = m.c_ref + (double)vc + (double)cc * sv;
+    c = m.c_ref + (double)vc + (double)cc * m.sv;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-        g[a] = (double)gg[a] * (sg * m.inv_spacing[a]);
+        g[a] = (double)gg[a] * m.sg[a];
 #pragma unroll
-        for (int b = 0; b < D; ++b) {
-            const double hv = a <= b ? (double)hh[a][b] : (double)hh[b][a];
-            H[a * D + b] = hv * ((a == b ? sg : sm) * m.inv_spacing[a] * m.inv_spacing[b]);
-        }
+        for (int b = 0; b < D; ++b) H[a * D + b] = (a <= b ? (double)hh[a][b] : (double)hh[b][a]) * m.sh[a][b];
     }
 }
 
@@ -408,7 +436,7 @@ struct RecordWriter {
     const TrajArgs &T;
     int64_t bl;
     double w;
-    int tt_len;
+    static constexpr int tt_len = MSGB_TIME_TILE;  // a power of two: no 64-bit division per record
     float lo[D], hi[D];
     double lmin = 1e300;
     bool bad = false;
@@ -416,8 +444,8 @@ struct RecordWriter {
     // taken yet; kept across beams when a dead tile did not use it)
     int64_t blk = -1;
 
-    __device__ RecordWriter(const ProbArgs &P_, const TrajArgs &T_, int64_t bl_, double w_, int tt_len_)
-        : P(P_), T(T_), bl(bl_), w(w_), tt_len(tt_len_) {
+    __device__ RecordWriter(const ProbArgs &P_, const TrajArgs &T_, int64_t bl_, double w_)
+        : P(P_), T(T_), bl(bl_), w(w_) {
 #pragma unroll
         for (int i = 0; i < D; ++i) lo[i] = 3.4e38f, hi[i] = -3.4e38f;
     }
@@ -455,7 +483,7 @@ struct RecordWriter {
             r[q++] = y.A.re;
             r[q++] = y.A.im;
         }
-        const int kk_tile = (int)(k % tt_len);
+        const int kk_tile = (int)((uint64_t)k % tt_len);
         char *rec32_base = nullptr;
         if (T.pool) {
             if (kk_tile == 0 && blk < 0) blk = (int64_t)atomicAdd(T.pool_next, 1ULL);
@@ -498,7 +526,7 @@ struct RecordWriter {
             for (int i = 0; i < D; ++i)
 #pragma unroll
                 for (int l = 0; l < D; ++l) Sm[i][l] = y.M[i][l].im;
-            const int kk = (int)(k % tt_len);
+            const int kk = kk_tile;
             if (kk == 0) {
                 lmin = 1e300;
 #pragma unroll
@@ -536,7 +564,7 @@ struct RecordWriter {
                         }
                         live = box[2 * D] * d2 * 0.999f <= T.live_cutoff * 1.0001f;
                     }
-                    int32_t *sl = T.slot + (k / tt_len) * T.nb + bl;
+                    int32_t *sl = T.slot + (int64_t)((uint64_t)k / tt_len) * T.nb + bl;
                     if (live && blk >= 0 && blk < T.pool_blocks) {
                         *sl = (int32_t)blk;
                         float *c = T.pool_cull + blk * (2 * D + 1);
@@ -547,7 +575,7 @@ struct RecordWriter {
                         *sl = -1;  // dead tile (or pool exhausted): the block is reused
                     }
                 } else {
-                    float *c = T.cull + ((k / tt_len) * T.nb + bl) * (2 * D + 1);
+                    float *c = T.cull + ((int64_t)((uint64_t)k / tt_len) * T.nb + bl) * (2 * D + 1);
 #pragma unroll
                     for (int i = 0; i < 2 * D + 1; ++i) c[i] = box[i];
                 }
@@ -583,6 +611,18 @@ inline int medium_args(const msgb_problem *prob, const msgb_medium *med, MediumA
     M.lam = med->lam;
     M.coeffs32 = med->coeffs32;
     M.c_ref = med->c_ref;
+    // The cubic sums carry 6 x the B-spline weights (no FP64 division per
+    // weight): a sum whose terms carry the plain weight of q axes is 6^q too
+    // large (value: all axes; gradient and diagonal Hessian: ndim - 1; mixed
+    // Hessian: ndim - 2).
+    const double s6 = med->kind == MSGB_MEDIUM_BSPLINE3 ? 1.0 / 6.0 : 1.0;
+    const int D = prob->ndim;
+    M.sv = D == 1 ? s6 : (D == 2 ? s6 * s6 : s6 * s6 * s6);
+    const double sg = D == 1 ? 1.0 : (D == 2 ? s6 : s6 * s6), sm = D == 3 ? s6 : 1.0;
+    for (int a = 0; a < D; ++a) {
+        M.sg[a] = sg * M.inv_spacing[a];
+        for (int b = 0; b < D; ++b) M.sh[a][b] = (a == b ? sg : sm) * M.inv_spacing[a] * M.inv_spacing[b];
+    }
     return MSGB_OK;
 }
 
