@@ -139,13 +139,13 @@ __device__ __forceinline__ void from_full(const State<D> &f, SState<D> &s) {
 // coupled_rhs_absorption on the symmetric state (the same terms as rhs; dM
 // is formed for i <= k only).
 // (The reciprocals 1/|p| and 1/|p|^3 replace FP64 divisions.)
-template <int D, int KIND, bool F32M = false>
-__device__ void rhs_sym(const MediumArgs &med, double mode, const SState<D> &y, SState<D> &dy) {
+template <int D, int KIND, bool F32M, typename Cache>
+__device__ void rhs_sym(const MediumArgs &med, Cache &cache, double mode, const SState<D> &y, SState<D> &dy) {
     double c, gc[D], hc[D * D];
-    if (F32M && KIND != MSGB_MEDIUM_CONSTANT)
-        speed_eval_f32<D, KIND>(med, y.x, c, gc, hc);
+    if constexpr (F32M && KIND != MSGB_MEDIUM_CONSTANT)
+        speed_eval_f32<D, KIND>(med, y.x, c, gc, hc, &cache);
     else
-        speed_eval_k<D, KIND>(med, y.x, c, gc, hc);
+        speed_eval_k<D, KIND, Cache>(med, y.x, c, gc, hc, &cache);
     double n2 = 0.0;
 #pragma unroll
     for (int i = 0; i < D; ++i) n2 += y.p[i] * y.p[i];
@@ -323,13 +323,28 @@ template <int D>
 constexpr size_t dopri_smem_bytes(int blk) {
     return (size_t)blk * 7 * NVS<D>::value * sizeof(double);
 }
-// The mixed-precision integrator's: 7 FP64 ray stages and 7 FP32 Hessian and
-// amplitude stages per lane (28 KB per 64 lanes in 2D, 46.6 KB in 3D).
+// The mixed-precision integrator's: 6 FP64 ray stages and 6 FP32 Hessian and
+// amplitude stages per lane, the last stage staying in registers (24 KB per 64
+// lanes in 2D, 40 KB in 3D).
+constexpr int kMixStages = 6;
 template <int D>
 constexpr size_t dopri_mix_smem_bytes(int blk) {
-    return (size_t)blk * 7 * (2 * D * sizeof(double) + (D * (D + 1) + 2) * sizeof(float));
+    return (size_t)blk * kMixStages * (2 * D * sizeof(double) + (D * (D + 1) + 2) * sizeof(float));
 }
-constexpr int kMixBlocks = 6;  // default blocks per SM of the mixed-precision integrator (measured best at config 3)
+// Blocks per SM of the mixed-precision integrator: 4 in 3D (five spill and measured
+// 38.4 ms instead of 32.2 at 32,002 beams), 6 or 7 otherwise.  The lanes are
+// persistent and all beams take about the same number of steps, so the time goes
+// by rounds of resident lanes: 7 blocks' round takes 1.117 of 6 blocks', and a last
+// round with few lanes 0.45 (latency only).  1024^2, 120,000 beams: 6 blocks 2.1
+// rounds 193 ms, 7 blocks 1.8 rounds 168 ms; 200,000 beams: 277 and 293 ms.
+inline int mix_blocks(int ndim, int64_t nb, int sms) {
+    if (ndim == 3) return 4;
+    auto cost = [&](int blocks, double round) {
+        const int64_t lanes = (int64_t)blocks * sms * 64, full = nb / lanes, rem = nb % lanes;
+        return (double)full * round + (rem ? 0.45 + (round - 0.45) * (double)rem / (double)lanes : 0.0);
+    };
+    return cost(7, 1.117) < cost(6, 1.0) ? 7 : 6;
+}
 
 // A lane's stages in shared memory, every integrator block having 64 lanes:
 // stage j holds its N values as N / 2 pairs (FP64) or as quads and a pair (FP32),
@@ -395,7 +410,14 @@ struct DopriBeam {
     bool rejected;
     int code;  // 0 running or done, 1 non-finite, 2 step budget exhausted
     Stages64<NVS<D>::value> ks;  // this lane's stages
-    __device__ DopriBeam() { ks.at = reinterpret_cast<double2 *>(dopri_stage_smem) + threadIdx.x; }
+    using T = typename std::conditional<F32M && KIND != MSGB_MEDIUM_CONSTANT, float, double>::type;
+    MediumCache<D, KIND, T> cache;
+    __device__ DopriBeam() {
+        ks.at = reinterpret_cast<double2 *>(dopri_stage_smem) + threadIdx.x;
+        if constexpr (MediumCache<D, KIND, T>::on)
+            cache.at = reinterpret_cast<typename StencilCache<T>::V *>(dopri_stage_smem + 7 * NVS<D>::value * kOdeBlock) +
+                       threadIdx.x;
+    }
 
     __device__ void init(const MediumArgs &med, const ProbArgs &P, const OdeArgs &o, double mode_) {
         mode = mode_;
@@ -406,7 +428,7 @@ struct DopriBeam {
         rejected = false;
         code = 0;
         SState<D> f0;
-        rhs_sym<D, KIND, F32M>(med, mode, y, f0);
+        rhs_sym<D, KIND, F32M>(med, cache, mode, y, f0);
         ks.put(0, vals(f0));
     }
 
@@ -458,7 +480,7 @@ struct DopriBeam {
 #pragma unroll
             for (int c = 0; c < N; ++c) tv[c] = yv[c] + hh * acc[c];
             SState<D> kn;
-            rhs_sym<D, KIND, F32M>(med, mode, yt, kn);
+            rhs_sym<D, KIND, F32M>(med, cache, mode, yt, kn);
             ks.put(s, vals(kn));
         }
         // yt now holds the 5th-order solution (stage 7's input).
@@ -570,22 +592,6 @@ struct MState {
 };
 
 template <int D>
-__device__ __forceinline__ void mix_to_full(const MState<D> &s, State<D> &o) {
-    constexpr int S = MState<D>::S;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-        o.x[i] = s.r[i];
-        o.p[i] = s.r[D + i];
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            const int q = sym_index<D>(i, k);
-            o.M[i][k] = cd{(double)s.f[2 * q], (double)s.f[2 * q + 1]};
-        }
-    }
-    o.A = cd{(double)s.f[2 * S], (double)s.f[2 * S + 1]};
-}
-
-template <int D>
 __device__ __forceinline__ void mix_from_full(const State<D> &o, MState<D> &s) {
     constexpr int S = MState<D>::S;
 #pragma unroll
@@ -605,12 +611,12 @@ __device__ __forceinline__ void mix_from_full(const State<D> &o, MState<D> &s) {
 
 // coupled_rhs_absorption: the ray terms in FP64, the Riccati and amplitude
 // terms in FP32 (the same terms as rhs_sym).
-template <int D, int KIND>
-__device__ void rhs_mix(const MediumArgs &med, double mode, const MState<D> &y, MState<D> &dy) {
+template <int D, int KIND, typename Cache>
+__device__ void rhs_mix(const MediumArgs &med, Cache &cache, double mode, const MState<D> &y, MState<D> &dy) {
     constexpr int S = MState<D>::S;
     double c, gc[D], hc[D * D];
-    if (KIND != MSGB_MEDIUM_CONSTANT)
-        speed_eval_f32<D, KIND>(med, y.r, c, gc, hc);
+    if constexpr (KIND != MSGB_MEDIUM_CONSTANT)
+        speed_eval_f32<D, KIND>(med, y.r, c, gc, hc, &cache);
     else
         speed_eval_k<D, KIND>(med, y.r, c, gc, hc);
     const double *p = y.r + D;
@@ -731,12 +737,17 @@ struct DopriMix {
     int code;
     Stages64<ND> k64;
     Stages32<NF> k32;
+    MediumCache<D, KIND, float> cache;
     __device__ DopriMix() {
-        // 7 FP64 stages, then 7 FP32 ones: quads, then pairs
+        // kMixStages FP64 stages, then as many FP32 ones (quads, then pairs), then the
+        // medium's stencils
         k64.at = reinterpret_cast<double2 *>(dopri_stage_smem) + threadIdx.x;
-        float4 *q = reinterpret_cast<float4 *>(dopri_stage_smem + 7 * ND * kOdeBlock);
+        float4 *q = reinterpret_cast<float4 *>(dopri_stage_smem + kMixStages * ND * kOdeBlock);
         k32.at = q + threadIdx.x;
-        k32.at2 = reinterpret_cast<float2 *>(q + 7 * Stages32<NF>::Q * kOdeBlock) + threadIdx.x;
+        k32.at2 = reinterpret_cast<float2 *>(q + kMixStages * Stages32<NF>::Q * kOdeBlock) + threadIdx.x;
+        if constexpr (MediumCache<D, KIND, float>::on)
+            cache.at = reinterpret_cast<float4 *>(reinterpret_cast<float2 *>(q + kMixStages * Stages32<NF>::Q * kOdeBlock) +
+                                                  kMixStages * Stages32<NF>::R * kOdeBlock) + threadIdx.x;
     }
 
     __device__ void init(const MediumArgs &med, const ProbArgs &P, const OdeArgs &o, double mode_) {
@@ -748,7 +759,7 @@ struct DopriMix {
         rejected = false;
         code = 0;
         MState<D> f0;
-        rhs_mix<D, KIND>(med, mode, y, f0);
+        rhs_mix<D, KIND>(med, cache, mode, y, f0);
         k64.put(0, f0.r);
         k32.put(0, f0.f);
     }
@@ -795,7 +806,7 @@ struct DopriMix {
             for (int c = 0; c < ND; ++c) yt.r[c] = y.r[c] + hh * a64[c];
 #pragma unroll
             for (int c = 0; c < NF; ++c) yt.f[c] = fmaf(hf, a32[c], y.f[c]);
-            rhs_mix<D, KIND>(med, mode, yt, kn);
+            rhs_mix<D, KIND>(med, cache, mode, yt, kn);
             if (s < 6) {  // the last stage stays in registers
                 k64.put(s, kn.r);
                 k32.put(s, kn.f);
@@ -855,9 +866,7 @@ struct DopriMix {
             rejected = false;
             const double t_new = last ? target : t + hh;
             while (k < P.nt && P.ts[k] <= t_new) {
-                State<D> yf;
-                mix_to_full(yt, yf);
-                rw.put(k, yf, false);
+                rw.put_mix(k, yt.r, yt.f, false);
                 ++k;
             }
             t = t_new;
@@ -890,6 +899,14 @@ __device__ void launch_state(const BeamArgs &B, const TrajArgs &T, int64_t bl, S
     w = B.omega[j];
 }
 
+// Lane l of warp v takes beam l * (warps of the grid) + v first: with fewer beams
+// than lanes every warp has some, and its scattered accesses and its divergent
+// paths (a rejected step, a new grid cell) cost fewer lookups and trips.
+__device__ __forceinline__ int64_t first_beam() {
+    const int64_t warps = (int64_t)gridDim.x * (kOdeBlock / 32);
+    return (threadIdx.x & 31) * warps + blockIdx.x * (int64_t)(kOdeBlock / 32) + (threadIdx.x >> 5);
+}
+
 // Adaptive integration with persistent lanes: thread i integrates beams
 // i, i + stride, i + 2 stride, ... one attempted step per loop trip, so a
 // lane whose beam finishes early starts its next beam instead of idling
@@ -900,7 +917,7 @@ template <int D, int KIND, int MINB, bool F32M, bool DENSE>
 __global__ void __launch_bounds__(64, MINB)
 dopri_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t bl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - stride;
+    int64_t bl = first_beam() - stride;
     bool active = false;
     DopriBeam<D, KIND, F32M, DENSE> s;
     RecordWriter<D> rw(P, T, 0, 0.0);
@@ -949,7 +966,7 @@ __global__ void __launch_bounds__(64, MINB)
 dopri_mix_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) {
     constexpr int ND = MState<D>::ND;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t bl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - stride;
+    int64_t bl = first_beam() - stride;
     bool active = false;
     DopriMix<D, KIND> s;
     RecordWriter<D> rw(P, T, 0, 0.0);
@@ -964,7 +981,7 @@ dopri_mix_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) 
                 launch_state<D>(B, T, bl, y0, mode, w);
                 mix_from_full(y0, s.y);
                 rw.reset(bl, w);
-                rw.put(0, y0, false);
+                rw.put_mix(0, s.y.r, s.y.f, false);
                 s.init(med, P, o, mode);
                 active = true;
             }
@@ -977,9 +994,7 @@ dopri_mix_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) 
             for (int c = 0; c < ND; ++c) fin = fin && isfinite(s.y.r[c]);
             if (!fin && s.code == 0) s.code = 1;
             if (s.k < P.nt) {  // after a failure: the last state
-                State<D> yf;
-                mix_to_full(s.y, yf);
-                for (int64_t k = s.k; k < P.nt; ++k) rw.put(k, yf, true);
+                for (int64_t k = s.k; k < P.nt; ++k) rw.put_mix(k, s.y.r, s.y.f, true);
             }
             if (T.status) T.status[bl] = s.code;
             lane_steps += (unsigned long long)s.steps;
@@ -1097,14 +1112,18 @@ struct Dopri {
                                : dopri_mix_kernel<D, K, 4>;
         return minb >= 5 ? dopri_kernel<D, K, 5, false, false> : dopri_kernel<D, K, 4, false, false>;
     }
-    template <int D>
-    size_t smem() const { return mixed() ? dopri_mix_smem_bytes<D>(64) : dopri_smem_bytes<D>(64); }
+    template <int D, int K>
+    size_t smem() const {
+        return mixed() ? dopri_mix_smem_bytes<D>(64) + medium_cache_bytes<D, K, float>()
+                       : dopri_smem_bytes<D>(64) +
+                             (f32m ? medium_cache_bytes<D, K, float>() : medium_cache_bytes<D, K, double>());
+    }
 };
 struct TrFinal {
     template <int D, int K>
     auto kernel() const { return tr_final_kernel<D, K>; }
-    template <int D>
-    size_t smem() const { return dopri_smem_bytes<D>(64); }
+    template <int D, int K>
+    size_t smem() const { return dopri_smem_bytes<D>(64) + medium_cache_bytes<D, K, double>(); }
 };
 
 // Blocks of 64 lanes per SM of the adaptive integrator: MSGB_DOPRI_BLOCKS
@@ -1121,15 +1140,14 @@ int dopri_blocks_per_sm(int dflt) {
 
 template <int D, typename Launch, typename Which>
 void launch_by_kind(int kind, Launch launch, const Which &which) {
-    auto go = [&](auto kern) {
-        const size_t smem = which.template smem<D>();
+    auto go = [&](auto kern, size_t smem) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         launch(kern, smem);
     };
     switch (kind) {
-        case MSGB_MEDIUM_CONSTANT: go(which.template kernel<D, MSGB_MEDIUM_CONSTANT>()); break;
-        case MSGB_MEDIUM_LINEAR: go(which.template kernel<D, MSGB_MEDIUM_LINEAR>()); break;
-        default: go(which.template kernel<D, MSGB_MEDIUM_BSPLINE3>()); break;
+        case MSGB_MEDIUM_CONSTANT: go(which.template kernel<D, MSGB_MEDIUM_CONSTANT>(), which.template smem<D, MSGB_MEDIUM_CONSTANT>()); break;
+        case MSGB_MEDIUM_LINEAR: go(which.template kernel<D, MSGB_MEDIUM_LINEAR>(), which.template smem<D, MSGB_MEDIUM_LINEAR>()); break;
+        default: go(which.template kernel<D, MSGB_MEDIUM_BSPLINE3>(), which.template smem<D, MSGB_MEDIUM_BSPLINE3>()); break;
     }
 }
 
@@ -1226,16 +1244,24 @@ extern "C" int msgb_ode_trajectories(const msgb_problem *prob, const msgb_medium
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const bool f32m = opts->medium_fp32 != 0 && med->coeffs32 != nullptr && med->kind != MSGB_MEDIUM_CONSTANT;
         Dopri which{4, f32m, opts->dense_output != 0};
-        which.minb = dopri_blocks_per_sm(which.mixed() ? kMixBlocks : 4);
+        which.minb = dopri_blocks_per_sm(which.mixed() ? mix_blocks(prob->ndim, out->nb, sms) : 4);
         if (!which.mixed() && which.minb > 5) which.minb = 5;
         {
             // the lanes are persistent: every block must be resident at once
-            const size_t sm_bytes = prob->ndim == 1 ? which.smem<1>() : (prob->ndim == 2 ? which.smem<2>() : which.smem<3>());
+            constexpr int K = MSGB_MEDIUM_BSPLINE3;  // the largest
+            const size_t sm_bytes =
+                1024 + (prob->ndim == 1 ? which.smem<1, K>() : (prob->ndim == 2 ? which.smem<2, K>() : which.smem<3, K>()));
             const int fit = (int)((size_t)(227 * 1024) / sm_bytes);
             if (which.minb > fit) which.minb = fit < 4 ? 4 : fit;
         }
         const int64_t want = (int64_t)which.minb * sms;
-        const unsigned grid = (unsigned)(need < want ? need : want);
+        // few beams: one warp per scheduler (two blocks per SM) before any warp is
+        // full -- a step then waits on nothing but its own chain (2000 beams over
+        // 5,667 save times 56.8 -> 34.7 ms); more warps per scheduler only once the
+        // lanes are full (10,000 beams: 45.7 ms against 55.2 ms with 4 beams a warp)
+        const int64_t spread = (out->nb + 1) / 2 < 2 * sms ? (out->nb + 1) / 2 : 2 * sms;
+        const int64_t blocks = need > spread ? need : spread;
+        const unsigned grid = (unsigned)(blocks < want ? blocks : want);
         switch (prob->ndim) {
             case 1: launch_by_kind<1>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, to_args(beams), T, O); },
                                       which); break;

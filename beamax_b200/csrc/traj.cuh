@@ -4,6 +4,9 @@
 // per-time-tile culling boxes) in the layout msgb_trajectories documents.
 #pragma once
 
+#include <climits>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace msgb {
@@ -63,6 +66,69 @@ __device__ __forceinline__ void gather_plane(const T *__restrict__ g, const int 
         for (int k = 0; k < TAPS; ++k) v[i][k] = __ldg(g + ((int64_t)ia[i] * n[1] + ib[k]));
 }
 
+// A lane's stencil of a 2D cubic medium, kept in shared memory across evaluations:
+// a beam stays in its grid cell for about three steps (18 evaluations), and 16
+// scattered loads per lane and evaluation are 16 x 32 L1 lookups per warp -- they
+// took half of the beam ODE's time.  at: this lane's first vector; the rows are
+// strided by the block (16-byte accesses without bank conflicts).
+struct NoCache {
+    static constexpr bool on = false;
+};
+
+template <typename T>
+struct StencilCache {
+    static constexpr bool on = true;
+    using V = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
+    static constexpr int NV = 16 * sizeof(T) / sizeof(V);
+    static constexpr int kLanes = 64;  // the integrators' block size
+    static constexpr size_t kBytes = sizeof(V) * NV * kLanes;
+    V *at;
+    int lo0 = INT_MIN, lo1 = 0;
+    T centre;  // FP32: the value at tap (1, 1), subtracted from the stored ones
+
+    // v: the stencil at (lo0, lo1); FP32: minus its centre value c
+    __device__ __forceinline__ void get(const T *__restrict__ g, const int *n, int l0, int l1, int boundary, T (*v)[4],
+                                        T &c) {
+        if (l0 != lo0 || l1 != lo1) {
+            gather_plane<4>(g, n, l0, l1, boundary, v);
+            centre = sizeof(T) == 4 ? v[1][1] : T(0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[i][k] = sizeof(T) == 4 ? v[i][k] - centre : v[i][k];
+                if constexpr (sizeof(T) == 4) {
+                    at[i * kLanes] = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+                } else {
+                    at[2 * i * kLanes] = make_double2(v[i][0], v[i][1]);
+                    at[(2 * i + 1) * kLanes] = make_double2(v[i][2], v[i][3]);
+                }
+            }
+            lo0 = l0;
+            lo1 = l1;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (sizeof(T) == 4) {
+                const float4 q = at[i * kLanes];
+                v[i][0] = q.x, v[i][1] = q.y, v[i][2] = q.z, v[i][3] = q.w;
+            } else {
+                const double2 q = at[2 * i * kLanes], r = at[(2 * i + 1) * kLanes];
+                v[i][0] = q.x, v[i][1] = q.y, v[i][2] = r.x, v[i][3] = r.y;
+            }
+        }
+        c = centre;
+    }
+};
+
+// The integrators' cache for a medium: 2D cubic only (a 3D stencil, 64 values,
+// would cost a resident block).
+template <int D, int KIND, typename T>
+using MediumCache = typename std::conditional<D == 2 && KIND == MSGB_MEDIUM_BSPLINE3, StencilCache<T>, NoCache>::type;
+template <int D, int KIND, typename T>
+constexpr size_t medium_cache_bytes() {
+    return D == 2 && KIND == MSGB_MEDIUM_BSPLINE3 ? StencilCache<T>::kBytes : 0;
+}
+
 // The taps along one axis starting at lo (offsets into that axis).
 template <int TAPS>
 __device__ __forceinline__ void axis_taps(int lo, int n, int boundary, int *idx) {
@@ -79,8 +145,9 @@ __device__ __forceinline__ void axis_taps(int lo, int n, int boundary, int *idx)
 
 // c, grad c (D), hess c (D x D, row-major) at x, for a medium of kind KIND
 // (the tap count and the weights are then compile-time constants).
-template <int D, int KIND>
-__device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *x, double &c, double *g, double *H) {
+template <int D, int KIND, typename Cache = NoCache>
+__device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *x, double &c, double *g, double *H,
+                                             Cache *cache = nullptr) {
     if (KIND == MSGB_MEDIUM_CONSTANT) {
         c = m.c;
 #pragma unroll
@@ -150,7 +217,12 @@ __device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *
     } else if (D == 2) {
         const int L = D - 1;  // last axis
         double v2[4][4];
-        gather_plane<taps>(m.coeffs, m.n, lo[0], lo[L], m.boundary, v2);
+        if constexpr (Cache::on) {
+            double centre;
+            cache->get(m.coeffs, m.n, lo[0], lo[L], m.boundary, v2, centre);
+        } else {
+            gather_plane<taps>(m.coeffs, m.n, lo[0], lo[L], m.boundary, v2);
+        }
 #pragma unroll
         for (int i = 0; i < taps; ++i) {
             double rw = 0.0, rd = 0.0, rdd = 0.0;
@@ -219,9 +291,9 @@ __device__ __forceinline__ void speed_eval_k(const MediumArgs &m, const double *
 // weights of every derivative sum to zero, so the centring leaves the
 // gradient and Hessian unchanged and keeps their sums free of cancellation;
 // the value gets the centre back), and the results return to FP64 with c_ref.
-template <int D, int KIND>
-__device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double *x, double &c, double *g,
-                                               double *H) {
+template <int D, int KIND, typename Cache>
+__device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double *x, double &c, double *g, double *H,
+                                               Cache *cache) {
     constexpr bool cubic = KIND == MSGB_MEDIUM_BSPLINE3;
     constexpr int taps = cubic ? 4 : 2;
     constexpr int off0 = cubic ? -1 : 0;
@@ -279,14 +351,22 @@ __device__ __forceinline__ void speed_eval_f32(const MediumArgs &m, const double
     } else if (D == 2) {
         const int L = D - 1;
         float v2[4][4];
-        gather_plane<taps>(m.coeffs32, m.n, lo[0], lo[L], m.boundary, v2);
-        vc = v2[ctr][ctr];
+        if constexpr (Cache::on) {
+            cache->get(m.coeffs32, m.n, lo[0], lo[L], m.boundary, v2, vc);
+        } else {
+            gather_plane<taps>(m.coeffs32, m.n, lo[0], lo[L], m.boundary, v2);
+            vc = v2[ctr][ctr];
+#pragma unroll
+            for (int i = 0; i < taps; ++i)
+#pragma unroll
+                for (int k = 0; k < taps; ++k) v2[i][k] -= vc;
+        }
 #pragma unroll
         for (int i = 0; i < taps; ++i) {
             float rw = 0.0f, rd = 0.0f, rdd = 0.0f;
 #pragma unroll
             for (int k = 0; k < taps; ++k) {
-                const float v = v2[i][k] - vc;
+                const float v = v2[i][k];
                 rw = fmaf(w[L][k], v, rw);
                 rd = fmaf(d1[L][k], v, rd);
                 rdd = fmaf(d2[L][k], v, rdd);
@@ -396,6 +476,7 @@ struct TrajArgs {
     float *pool_cull = nullptr;
     int64_t pool_blocks = 0;
     unsigned long long *pool_next = nullptr;
+    bool align16 = false;  // the FP32 record base is 16-byte aligned (16-byte stores in 1D and 2D)
     const float *boxes = nullptr;
     int64_t n_boxes = 0;
     float live_cutoff = 0.0f;
@@ -406,6 +487,7 @@ inline void set_compact(TrajArgs &T, const msgb_trajectories *t) {
     T.slot = t->slot;
     T.pool = t->pool;
     T.pool_cull = t->pool_cull;
+    T.align16 = ((uintptr_t)(t->pool ? t->pool : t->rec32) & 15) == 0;
     T.pool_blocks = t->pool_blocks;
     T.pool_next = t->pool_next;
     T.boxes = t->live_boxes;
@@ -483,42 +565,23 @@ struct RecordWriter {
             r[q++] = y.A.re;
             r[q++] = y.A.im;
         }
-        const int kk_tile = (int)((uint64_t)k % tt_len);
-        char *rec32_base = nullptr;
-        if (T.pool) {
-            if (kk_tile == 0 && blk < 0) blk = (int64_t)atomicAdd(T.pool_next, 1ULL);
-            if (blk >= 0 && blk < T.pool_blocks)
-                rec32_base = (char *)T.pool + (blk * tt_len + kk_tile) * (int64_t)(16 * D + 8 * S + 8);
-        } else if (T.rec32) {
-            rec32_base = (char *)T.rec32 + (k * T.nb + bl) * (int64_t)(16 * D + 8 * S + 8);
-        }
-        if (rec32_base) {
-            // layout of the FP32 summation's BeamTime<D> record
-            char *base = rec32_base;
-            double *xd = (double *)base;
-            double *wpd = xd + D;
-            float *f = (float *)(wpd + D);
-#pragma unroll
-            for (int i = 0; i < D; ++i) {
-                xd[i] = xw[i];
-                wpd[i] = w * y.p[i];
-            }
+        char *base = record32(k);
+        if (base) {
+            float q[S], p[S];
 #pragma unroll
             for (int i = 0; i < D; ++i)
 #pragma unroll
                 for (int l = i; l < D; ++l) {
-                    const int q = sym_index<D>(i, l);
-                    const double fac = (i == l ? 0.5 : 0.5) * w;  // off-diagonal: (M_il + M_li)/2 doubled
+                    const int e = sym_index<D>(i, l);
+                    const double fac = 0.5 * w;  // off-diagonal: (M_il + M_li)/2 doubled
                     const double mre = i == l ? y.M[i][i].re : (y.M[i][l].re + y.M[l][i].re);
                     const double mim = i == l ? y.M[i][i].im : (y.M[i][l].im + y.M[l][i].im);
-                    f[q] = (float)(fac * mre);
-                    f[S + q] = (float)(fac * mim);
+                    q[e] = (float)(fac * mre);
+                    p[e] = (float)(fac * mim);
                 }
             // arg A and 2|A| are stored as floats: FP32 arithmetic on the
             // rounded components gives them to FP32 precision
-            const float are = (float)y.A.re, aim = (float)y.A.im;
-            f[2 * S] = atan2f(aim, (are == 0.0f && aim == 0.0f) ? 1e-12f : are);
-            f[2 * S + 1] = 2.0f * hypotf(are, aim);
+            store32(base, xw, y.p, q, p, (float)y.A.re, (float)y.A.im);
         }
         if (T.cull || T.pool) {
             double Sm[D][D];
@@ -526,19 +589,115 @@ struct RecordWriter {
             for (int i = 0; i < D; ++i)
 #pragma unroll
                 for (int l = 0; l < D; ++l) Sm[i][l] = y.M[i][l].im;
-            const int kk = kk_tile;
-            if (kk == 0) {
-                lmin = 1e300;
+            bound(k, xw, lam_min<D>(Sm));
+        }
+    }
+
+    // put() for the mixed-precision state: centre and momentum r (2 D doubles), the
+    // Hessian and the amplitude f (re, im pairs in sym_index order, then A).
+    __device__ __forceinline__ void put_mix(int64_t k, const double *r, const float *f, bool failed) {
+        bad |= failed;
+        double xw[D];
 #pragma unroll
-                for (int i = 0; i < D; ++i) lo[i] = 3.4e38f, hi[i] = -3.4e38f;
-            }
-            lmin = fmin(lmin, lam_min<D>(Sm));
+        for (int i = 0; i < D; ++i) xw[i] = P.periodic[i] ? pymod(r[i], P.L[i]) : r[i];
+        char *base = record32(k);
+        if (base) {
+            float q[S], p[S];
 #pragma unroll
-            for (int i = 0; i < D; ++i) {
-                const float xf = (float)xw[i];
-                lo[i] = fminf(lo[i], xf);
-                hi[i] = fmaxf(hi[i], xf);
+            for (int i = 0; i < D; ++i)
+#pragma unroll
+                for (int l = i; l < D; ++l) {
+                    const int e = sym_index<D>(i, l);
+                    const double fac = (i == l ? 0.5 : 1.0) * w;
+                    q[e] = (float)(fac * (double)f[2 * e]);
+                    p[e] = (float)(fac * (double)f[2 * e + 1]);
+                }
+            store32(base, xw, r + D, q, p, f[2 * S], f[2 * S + 1]);
+        }
+        if (T.cull || T.pool) {
+            double lam;
+            if (D == 2) {
+                // smaller eigenvalue as det / larger: the determinant in FP64, the
+                // rest in FP32 (relative error below 1e-6, taken off here)
+                const double a = f[1], b = f[3 % (2 * S)], c = f[5 % (2 * S)];
+                const float m = 0.5f * (f[1] + f[5 % (2 * S)]), h = 0.5f * (f[1] - f[5 % (2 * S)]);
+                const float den = m + sqrtf(fmaf(h, h, f[3 % (2 * S)] * f[3 % (2 * S)]));
+                const float det = (float)fma(a, c, -b * b);
+                const float l = den > 0.0f ? __fdividef(det, den) : 0.0f;
+                lam = (double)(l - 1e-6f * fabsf(l));
+            } else {
+                double Sm[D][D];
+#pragma unroll
+                for (int i = 0; i < D; ++i)
+#pragma unroll
+                    for (int l = 0; l < D; ++l) Sm[i][l] = (double)f[2 * sym_index<D>(i, l) + 1];
+                lam = lam_min<D>(Sm);
             }
+            bound(k, xw, lam);
+        }
+    }
+
+    // Where the FP32 record of time k goes, or nullptr.  A compact lane takes a
+    // block at the start of a time tile unless it still has one.
+    __device__ __forceinline__ char *record32(int64_t k) {
+        if (T.pool) {
+            const int kk = (int)((uint64_t)k % tt_len);
+            if (kk == 0 && blk < 0) blk = (int64_t)atomicAdd(T.pool_next, 1ULL);
+            if (blk >= 0 && blk < T.pool_blocks) return (char *)T.pool + (blk * tt_len + kk) * (int64_t)(16 * D + 8 * S + 8);
+            return nullptr;
+        }
+        return T.rec32 ? (char *)T.rec32 + (k * T.nb + bl) * (int64_t)(16 * D + 8 * S + 8) : nullptr;
+    }
+
+    // The FP32 summation's BeamTime<D> record: x, w p, q, p, arg A, 2 |A|.
+    __device__ __forceinline__ void store32(char *base, const double *xw, const double *mom, const float *q, const float *p,
+                                            float are, float aim) {
+        constexpr int NF = 2 * S + 2;
+        float f[NF];
+#pragma unroll
+        for (int e = 0; e < S; ++e) f[e] = q[e], f[S + e] = p[e];
+        f[2 * S] = atan2f(aim, (are == 0.0f && aim == 0.0f) ? 1e-12f : are);
+        f[2 * S + 1] = 2.0f * hypotf(are, aim);
+        if (D != 3 && T.align16) {  // 32 B (1D) or 64 B (2D) in 16-byte stores
+            double d[2 * D];
+#pragma unroll
+            for (int i = 0; i < D; ++i) d[i] = xw[i], d[D + i] = w * mom[i];
+            double2 *b2 = (double2 *)base;
+#pragma unroll
+            for (int i = 0; i < D; ++i) b2[i] = make_double2(d[2 * i], d[2 * i + 1]);
+            float4 *b4 = (float4 *)(b2 + D);
+#pragma unroll
+            for (int i = 0; i < NF / 4; ++i) b4[i] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+            return;
+        }
+        double *xd = (double *)base;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            xd[i] = xw[i];
+            xd[D + i] = w * mom[i];
+        }
+        float2 *b2 = (float2 *)(xd + 2 * D);
+#pragma unroll
+        for (int i = 0; i < NF / 2; ++i) b2[i] = make_float2(f[2 * i], f[2 * i + 1]);
+    }
+
+    // The culling box of the time tile: the centre xw and the smallest eigenvalue
+    // lam of Im M at time k; written (with the tile's slot) at the tile's end.
+    __device__ __forceinline__ void bound(int64_t k, const double *xw, double lam) {
+        const int kk = (int)((uint64_t)k % tt_len);
+        if (kk == 0) {
+            lmin = 1e300;
+#pragma unroll
+            for (int i = 0; i < D; ++i) lo[i] = 3.4e38f, hi[i] = -3.4e38f;
+        }
+        lmin = fmin(lmin, lam);
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            const float xf = (float)xw[i];
+            lo[i] = fminf(lo[i], xf);
+            hi[i] = fmaxf(hi[i], xf);
+        }
+        {
             if (kk == tt_len - 1 || k == P.nt - 1) {
                 float box[2 * D + 1];
 #pragma unroll
