@@ -207,7 +207,8 @@ class MSGBSolver:
         self.compact_trajectories = bool(compact_trajectories)
         self._traj_cache = None
         self._traj_owner = None
-        self._live_est = 0.5  # fraction of (time tile, beam) pairs the compact store keeps
+        # fraction of (time tile, beam) pairs the compact store keeps; None: not seen yet
+        self._live_est: Optional[float] = None
         self._compact_kept = None
         # (b_first, nb, pool blocks, blocks taken) of the last 256 compact integrations
         self.compact_log = collections.deque(maxlen=256)
@@ -469,13 +470,20 @@ class MSGBSolver:
                             dense_output=int(bool(cfg.dense_output)),
                             medium_fp32=int(self.precision == "fp32"))
 
-    def _mode_chunks(self, domain: Domain, nt: int, bt: BeamTensors, fp64: bool):
-        """Chunks over the beams of the summed branches: [0, 2n), [0, n) (mode
-        +1 only) or [n, 2n) (mode -1 only)."""
+    @staticmethod
+    def _mode_range(bt: BeamTensors):
+        """The beams of the summed branches: [0, 2n), [0, n) (mode +1 only) or
+        [n, 2n) (mode -1 only)."""
         n = bt.n
-        lo, hi = {0: (0, 2 * n), 1: (0, n), 2: (n, 2 * n)}[bt.modes]
+        return {0: (0, 2 * n), 1: (0, n), 2: (n, 2 * n)}[bt.modes]
+
+    def _mode_chunks(self, domain: Domain, nt: int, bt: BeamTensors, fp64: bool):
+        """Chunks of dense records over the beams of the summed branches."""
+        lo, hi = self._mode_range(bt)
+        if not fp64 and self._compact():
+            return [(lo, hi - lo)], 0, 0  # the compact store makes its own chunks
         budget = self._trajectory_budget(bt.x0.device)
-        if self.keep_trajectories and (fp64 or not self._compact()):
+        if self.keep_trajectories:
             budget //= 2  # the dense path may hold a kept chunk beside the chunk buffer
         chunks, per, n_tt = self._chunks(domain, nt, hi - lo, fp64, budget)
         return [(lo + b, nb) for b, nb in chunks], per, n_tt
@@ -547,11 +555,32 @@ class MSGBSolver:
         free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
         return int(max(1 << 20, min(self.trajectory_memory, free - (4 << 30))))
 
-    def _compact_chunk_beams(self, d, nt, nbeam, budget):
+    # Records up to this size are allocated without asking the device how much it
+    # has free (cudaMemGetInfo and the allocator's statistics cost 1.2 ms, a tenth
+    # of a 1000-beam step); it lies well inside the headroom.
+    _SMALL_RECORDS = 256 << 20
+
+    def _compact_budget(self, d, nt, nbeam, dev):
+        """(bytes for a chunk of compact records, fraction of live tiles to plan
+        for).  Before any integration has shown the fraction, every tile is
+        planned for when the records then take at most a quarter of the budget: a
+        pool that runs out costs integrating the chunk's halves again."""
+        n_tt, block, cull = self._compact_sizes(d, nt)
+        dense = nbeam * (n_tt * (4 + block + cull) + block + cull) + 4096
+        if dense <= min(self._SMALL_RECORDS, self.trajectory_memory):
+            budget = self._SMALL_RECORDS
+        else:
+            budget = self._trajectory_budget(dev)
+        est = self._live_est
+        if est is None:
+            est = 1.0 if dense <= budget // 4 or budget == self._SMALL_RECORDS else 0.5
+        return budget, est
+
+    def _compact_chunk_beams(self, d, nt, nbeam, budget, est):
         """Beams per chunk for the estimated fraction of live tiles (each beam
         may also leave one block that no live tile took)."""
         n_tt, block, cull = self._compact_sizes(d, nt)
-        per_beam = n_tt * 4 + self._live_est * n_tt * (block + cull) + (block + cull)
+        per_beam = n_tt * 4 + est * n_tt * (block + cull) + (block + cull)
         return int(max(1, min(nbeam, (budget - 4096) // max(per_beam, 1))))
 
     def _compact_tr(self, buf, d, nt, b_first, nb, status, boxes, n_boxes):
@@ -585,23 +614,20 @@ class MSGBSolver:
 
         d = pr.ndim
         n_tt, block, cull = self._compact_sizes(d, pr.nt)
-        boxes, n_boxes = self._live_boxes(pr, opts, domain, sensors, dev, st)
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        lanes = 4 * sms * 64  # the integrator's resident lanes
+        lanes = 7 * sms * 64  # the integrator's resident lanes, at most
         todo = []
         ranges = [(lo, hi)] if skip is None else [(lo, skip[0]), (skip[0] + skip[1], hi)]
-        budget = self._trajectory_budget(dev)
-        cb = 1
-        for a, b in ranges:
-            if b <= a:
-                continue
-            cb = self._compact_chunk_beams(d, pr.nt, b - a, budget)
-            todo += [(x, min(cb, b - x)) for x in range(a, b, cb)]
-        if not todo:
+        ranges = [(a, b) for a, b in ranges if b > a]
+        if not ranges:
             return
+        budget, est = self._compact_budget(d, pr.nt, max(b - a for a, b in ranges), dev)
+        for a, b in ranges:
+            cb = self._compact_chunk_beams(d, pr.nt, b - a, budget, est)
+            todo += [(x, min(cb, b - x)) for x in range(a, b, cb)]
         # the chunk's estimated need (plus one block per integrator lane), not the whole budget
         widest = max(nb for _, nb in todo)
-        need = int(widest * n_tt * (4 + self._live_est * (block + cull)) + min(widest, lanes) * (block + cull)
+        need = int(widest * n_tt * (4 + est * (block + cull)) + min(widest, lanes) * (block + cull)
                    + 4096)
         buf = None
         size = min(budget, need)
@@ -619,8 +645,9 @@ class MSGBSolver:
                         raise
                     widest = (widest + 1) // 2
                     todo = [(x, min(widest, b0 + n0 - x)) for b0, n0 in todo for x in range(b0, b0 + n0, widest)]
-                    size = int(widest * n_tt * (4 + self._live_est * (block + cull))
+                    size = int(widest * n_tt * (4 + est * (block + cull))
                                + min(widest, lanes) * (block + cull) + 4096)
+        boxes, n_boxes = self._live_boxes(pr, opts, domain, sensors, dev, st)
         first = True
         opts_ode = self._ode_opts(None)
         if self.ode_step_counter is not None:
@@ -638,7 +665,7 @@ class MSGBSolver:
             if used > blocks:
                 if nb == 1:
                     raise RuntimeError("compact trajectory store: one beam needs more than the budget")
-                self._live_est = min(1.0, self._live_est * 2.0)
+                est = self._live_est = min(1.0, est * 2.0)
                 todo[:0] = [(b_first, nb // 2), (b_first + nb // 2, nb - nb // 2)]
                 continue
             self._live_est = min(1.0, max(0.05, 1.15 * max(0, used - min(nb, lanes)) / max(1, n_tt * nb)))
@@ -814,8 +841,10 @@ class MSGBSolver:
         tiling = None if fp64 else self._tiling(domain, sensors, dev)
         opts = _lib.SumOpts(cutoff=self.cutoff, eval_count=cnt.data_ptr(),
                             tiling=_lib.ref(tiling[0]) if tiling else None)
-        nbytes = 0 if fp64 else _lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), max(nb for _, nb in chunks))
-        ws = None if fp64 else workspace(dev, "sum32traj", nbytes)
+        nbytes, ws = 0, None
+        if not fp64 and not self._compact():
+            nbytes = _lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), max(nb for _, nb in chunks))
+            ws = workspace(dev, "sum32traj", nbytes)
         status = torch.zeros(2 * n, dtype=torch.int32, device=dev)
         self._begin_trajectories(domain, ts)
         kept = (cached["tr"].b_first, cached["tr"].nb) if cached is not None else None
