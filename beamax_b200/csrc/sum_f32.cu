@@ -665,6 +665,8 @@ __device__ __forceinline__ bool traj_survives(const TrajSrc<D> &T, int64_t bl, i
     return c[2 * D] * d2 * 0.999f <= cutoff;
 }
 
+constexpr int SCAN = 4;  // beams tested per thread and scan
+
 // ------------------------------------------------------------------ record passes
 // A record pass holds up to G beams' records at the tile's 32 times in shared
 // memory, rec[field][beam][time], and per beam an 8-bit mask of the warps (sensor
@@ -992,6 +994,71 @@ __device__ __forceinline__ int scan_counts(const int *cnt, int row, int warp, in
     return __shfl_sync(0xffffffffu, x - v, row * NW + warp);
 }
 
+// Trajectory candidates surv[old .. nq) (kept by the tile test) against the groups
+// of the tile, from 4 of their tile's 32 times: the tile test's isotropic bound
+// keeps 2 to 3 candidates for each that reaches the tile (live: 34 % at 1024^2
+// heterogeneous, 40 % at 128^3), and fetching a dead one's whole record (2 KB in
+// 2D) cost more than half of the summation.  A beam goes if at every sample its
+// exponent exceeds thr widened by the way it moves to half-way between the samples
+// (in the sample's own metric, with a fifth to spare) and by a tenth of the
+// exponent's root for the change of Im M; Im M is smallest at an end of a sampled
+// interval.  Four lanes per candidate; the survivors move to surv[old ..) in
+// order.  Returns the new end.  All threads; ends with a barrier.
+template <int D, typename BeamOf>
+__device__ __forceinline__ int refine(const TrajSrc<D> &T, int64_t t_first, int t_cnt, const TileInfo<D> &ti,
+                                      const TileGroups<D> &tg, float thr, int32_t *surv, int old, int nq, uint8_t *keep,
+                                      int *warp_cnt, const BeamOf &beam_of) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, smp = lane & 3;
+    const int64_t tt = t_first / TT;
+    const int ts = (t_cnt - 1) * smp / 3;
+    int out = old;
+    for (int base = old; base < nq; base += SCAN * THREADS) {
+        const int end = min(nq, base + SCAN * THREADS);
+#pragma unroll 2
+        for (int c0 = base + warp * 8; c0 < end; c0 += NW * 8) {
+            const int c = min(c0 + lane / 4, end - 1);
+            const int64_t b = beam_of(c);
+            const BeamTime<D> *bt =
+                T.pool ? T.pool + ((int64_t)T.slot[tt * T.nb + b] * TT + ts) : T.rec + ((t_first + ts) * T.nb + b);
+            Rec<D> r;
+#pragma unroll
+            for (int a = 0; a < D; ++a) r.d0[a] = (float)(ti.s0[a] - bt->x[a]);
+#pragma unroll
+            for (int q = 0; q < Sym<D>::S; ++q) r.p[q] = bt->p[q];
+            float up[D], dn[D];
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                up[a] = __shfl_down_sync(0xffffffffu, r.d0[a], 1, 4) - r.d0[a];
+                dn[a] = __shfl_up_sync(0xffffffffu, r.d0[a], 1, 4) - r.d0[a];
+            }
+            const float way = sqrtf(fmaxf(0.0f, fmaxf(quad<D>(r.p, up), quad<D>(r.p, dn))));
+            const float root = (sqrtf(thr) + 0.6f * way) * (1.0f / 0.9f);
+            const unsigned hit = __ballot_sync(0xffffffffu, reached_mask<D>(r, tg, root * root) != 0);
+            if (smp == 0 && c0 + lane / 4 < end) keep[c0 + lane / 4 - base] = (hit >> lane & 15u) ? 1 : 0;
+        }
+        __syncthreads();
+        int32_t v[SCAN];
+        unsigned bk[SCAN];
+#pragma unroll
+        for (int k = 0; k < SCAN; ++k) {
+            const int i = base + k * THREADS + tid;
+            v[k] = i < end ? surv[i] : 0;
+            bk[k] = __ballot_sync(0xffffffffu, i < end && keep[i - base]);
+            if (lane == 0) warp_cnt[k * NW + warp] = __popc(bk[k]);
+        }
+        __syncthreads();
+        int tot = 0;
+#pragma unroll
+        for (int k = 0; k < SCAN; ++k) {
+            const int off = out + scan_counts<SCAN>(warp_cnt, k, warp, tot);
+            if (bk[k] >> lane & 1u) surv[off + __popc(bk[k] & ((1u << lane) - 1u))] = v[k];
+        }
+        out += tot;
+        __syncthreads();
+    }
+    return out;
+}
+
 // ------------------------------------------------------------------ forward
 __device__ __forceinline__ void kahan_add(float &acc, float &cmp, float v) {
     const float y = v - cmp;
@@ -999,8 +1066,6 @@ __device__ __forceinline__ void kahan_add(float &acc, float &cmp, float v) {
     cmp = (t - acc) - y;
     acc = t;
 }
-
-constexpr int SCAN = 4;  // beams tested per thread and scan
 
 // A tile's beams in n ranges of len, each its own work item with a partial
 // (compensated sum, compensation) per output, added in order by
@@ -1074,7 +1139,7 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
     __shared__ HomStage<D, TRAJ> hstage;
     __shared__ int32_t surv[2 * SCAN * THREADS + G];
     __shared__ int warp_cnt[SCAN * NW];
-    __shared__ uint8_t alive[G];
+    __shared__ uint8_t alive[G], keep[TRAJ ? SCAN * THREADS : 1];
     __shared__ int tile_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1163,8 +1228,14 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                 if (bp[k] >> lane & 1u) surv[off + __popc(bp[k] & lt)] = j;
                 if (!TRAJ && (bm[k] >> lane & 1u)) surv[off + __popc(bp[k]) + __popc(bm[k] & lt)] = (int32_t)(j + B.n);
             }
+            const int old = nq;
             nq += tot;
             __syncthreads();
+            if constexpr (TRAJ && !PERIODIC) {
+                if (thr > 0.0f)
+                    nq = refine<D>(T, t_first, t_cnt, ti, ginfo, thr, surv, old, nq, keep, warp_cnt,
+                                   [&](int c) { return (int64_t)surv[c]; });
+            }
             const bool last_scan = j0 + SCAN * THREADS >= nbeam;
             int g0 = 0;
             while (nq - g0 >= G || (last_scan && g0 < nq)) {
@@ -1320,7 +1391,8 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
     __shared__ TileGroups<D> ginfo;
     __shared__ HomStage<D, TRAJ> hstage;
     __shared__ int32_t surv[NACC];  // a range's survivors in one tile (local slots)
-    __shared__ int warp_cnt[NW];
+    __shared__ int warp_cnt[SCAN * NW];
+    __shared__ uint8_t keep[TRAJ ? SCAN * THREADS : 1];
     __shared__ float wpart[NW][G][2];
     __shared__ uint8_t alive2[2][G];
     __shared__ int item_s;
@@ -1393,13 +1465,20 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
 #pragma unroll
             for (int i = 0; i < D; ++i) run.ds[i] = sds[gbase][i], run.h[i] = shn[gbase][i];
             const float *dcol = dataT + (int64_t)s_first * P.nt + t_first + lane;
+            __syncthreads();
+            if (tid == 0) find_lattice<D>(ginfo);
+            __syncthreads();  // ginfo, surv
+            if constexpr (TRAJ && !PERIODIC) {
+                if (thr > 0.0f) {
+                    nq = refine<D>(T, t_first, t_cnt, ti, ginfo, thr, surv, 0, nq, keep, warp_cnt,
+                                   [&](int c) { return r0 + surv[c]; });
+                    if (nq == 0) continue;
+                }
+            }
             float dv[GS];
 #pragma unroll
             for (int k = 0; k < GS; ++k)
                 dv[k] = (tv && gbase + k < s_cnt) ? __ldg(dcol + (int64_t)(gbase + k) * P.nt) : 0.0f;
-            __syncthreads();
-            if (tid == 0) find_lattice<D>(ginfo);
-            __syncthreads();  // ginfo, surv
 
             for (int g0 = 0; g0 < nq; g0 += G) {
                 const int nb = min(G, nq - g0);
