@@ -37,6 +37,7 @@ struct msgb_mswpt {
     std::vector<int> lat_cnt, lat_first, lat_step;  // levels x nd
     std::vector<int64_t> lat_off;                   // levels
     std::vector<int64_t> goff;                      // levels
+    std::vector<int64_t> cand_off;                  // levels x 3
     int max_patch;                                  // max prod S
     // device tables
     int32_t *d_centres = nullptr;
@@ -47,6 +48,9 @@ struct msgb_mswpt {
     int32_t *d_bcum = nullptr;
     int32_t *d_bl = nullptr;
     int32_t *d_bshape = nullptr;
+    int2 *d_cand = nullptr;  // synthesis gather: see GatherLevel
+    double2 *d_tw = nullptr;  // exp(2 pi i m / tw_n), m < tw_n (the largest support)
+    int tw_n = 1;
     cufftHandle plan_d2z = 0, plan_z2z = 0;
     size_t fft_work = 0;
 };
@@ -59,32 +63,63 @@ constexpr int THREADS = 256;
 struct LevelArgs {
     int nd;
     int N[3];
-    int S[3];        // support per axis
+    int S[3];        // support per axis (powers of two)
+    int logS[3];
     int bhs[3];      // half support (box_shapes)
     int P;           // prod S
     int nbox;        // boxes at this level
     int box0;        // global id of the first box
+    int blk0;        // first CTA of the level in a launch over all levels
     int64_t c0;      // coefficient offset of the level
     int64_t seg;     // coefficients in the level
     double inv_sqrtS;
+    const double *g;  // window of the level (prod S)
 };
 
-LevelArgs level_args(const msgb_mswpt *p, int l) {
-    LevelArgs a{};
-    a.nd = p->nd;
-    a.P = 1;
-    for (int i = 0; i < 3; ++i) {
-        a.N[i] = i < p->nd ? p->N[i] : 1;
-        a.bhs[i] = i < p->nd ? p->bshape[l * p->nd + i] : 1;
-        a.S[i] = i < p->nd ? 2 * a.bhs[i] : 1;
-        a.P *= a.S[i];
+constexpr int kMaxLevels = 8;
+struct AllLevels {
+    int levels;
+    const double2 *tw;
+    int tw_n;
+    LevelArgs lv[kMaxLevels];
+};
+
+int ilog2(int n) {
+    int k = 0;
+    while ((1 << k) < n) ++k;
+    return k;
+}
+
+// Every level that has boxes, for one launch with a CTA per box; returns the CTAs.
+int all_levels(const msgb_mswpt *p, AllLevels &A) {
+    int blocks = 0;
+    A.levels = 0;
+    A.tw = p->d_tw;
+    A.tw_n = p->tw_n;
+    // the largest boxes first: the small ones fill the last wave
+    for (int l = p->levels - 1; l >= 0; --l) {
+        LevelArgs a{};
+        a.nd = p->nd;
+        a.P = 1;
+        for (int i = 0; i < 3; ++i) {
+            a.N[i] = i < p->nd ? p->N[i] : 1;
+            a.bhs[i] = i < p->nd ? p->bshape[l * p->nd + i] : 1;
+            a.S[i] = i < p->nd ? 2 * a.bhs[i] : 1;
+            a.logS[i] = ilog2(a.S[i]);
+            a.P *= a.S[i];
+        }
+        a.nbox = p->bcum[l + 1] - p->bcum[l];
+        if (a.nbox == 0) continue;
+        a.box0 = p->bcum[l];
+        a.c0 = p->ccum[l];
+        a.seg = p->ccum[l + 1] - p->ccum[l];
+        a.inv_sqrtS = 1.0 / sqrt((double)a.P);
+        a.g = p->d_gfilt + p->goff[l];
+        a.blk0 = blocks;
+        blocks += a.nbox;
+        A.lv[A.levels++] = a;
     }
-    a.nbox = p->bcum[l + 1] - p->bcum[l];
-    a.box0 = p->bcum[l];
-    a.c0 = p->ccum[l];
-    a.seg = p->ccum[l + 1] - p->ccum[l];
-    a.inv_sqrtS = 1.0 / sqrt((double)a.P);
-    return a;
+    return blocks;
 }
 
 __device__ __forceinline__ int floordiv(int a, int b) {
@@ -97,87 +132,127 @@ __device__ __forceinline__ int imod(int a, int b) {
     return r < 0 ? r + b : r;
 }
 
-// In-place unitary-free radix-2 DFT along every axis of a (S0, S1, S2) complex
-// array in shared memory; sign = +1 (inverse) or -1 (forward).  Twiddles are
-// exp(sign 2 pi i m / S) from sincospi.
-__device__ void smem_fft(double2 *x, const int *S, int nd, int sign, double2 *tw) {
-    const int S0 = S[0], S1 = S[1], S2 = S[2];
-    const int total = S0 * S1 * S2;
-    for (int ax = 0; ax < nd; ++ax) {
-        const int n = S[ax];
-        if (n == 1) continue;
-        const int stride = ax == 0 ? S1 * S2 : (ax == 1 ? S2 : 1);
-        // twiddle table
-        for (int m = threadIdx.x; m < n; m += blockDim.x) {
-            double s, c;
-            sincospi(2.0 * (double)m / (double)n, &s, &c);
-            tw[m] = make_double2(c, sign * s);
+// ---- box FFT: a (S0, S1, S2) complex array in shared memory ------------------
+// Elements are padded by one per eight, so that the strided accesses of a pass
+// spread over the banks.
+__device__ __forceinline__ int pad(int i) { return i + (i >> 3); }
+
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cmulz(double2 a, double2 b) {
+    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+// a * (sign i)
+__device__ __forceinline__ double2 mul_i(double2 a, double sign) { return make_double2(-sign * a.y, sign * a.x); }
+
+// DFT of R values in registers, outputs in natural order (v[k] = sum_j v[j] w^(jk)).
+template <int R>
+__device__ __forceinline__ void dft(double2 *v, double sign) {
+    if (R == 2) {
+        const double2 a = v[0], b = v[1 % R];
+        v[0] = cadd(a, b);
+        v[1 % R] = csub(a, b);
+    } else if (R == 4) {
+        const double2 a = cadd(v[0], v[2 % R]), b = csub(v[0], v[2 % R]);
+        const double2 c = cadd(v[1 % R], v[3 % R]), d = mul_i(csub(v[1 % R], v[3 % R]), sign);
+        v[0] = cadd(a, c);
+        v[1 % R] = cadd(b, d);
+        v[2 % R] = csub(a, c);
+        v[3 % R] = csub(b, d);
+    } else if (R == 8) {
+        double2 e[4] = {v[0], v[2 % R], v[4 % R], v[6 % R]}, o[4] = {v[1 % R], v[3 % R], v[5 % R], v[7 % R]};
+        dft<4>(e, sign);
+        dft<4>(o, sign);
+        const double h = 0.70710678118654752440;
+        o[1] = cmulz(o[1], make_double2(h, sign * h));
+        o[2] = mul_i(o[2], sign);
+        o[3] = cmulz(o[3], make_double2(-h, sign * h));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = cadd(e[k], o[k]);
+            v[(k + 4) % R] = csub(e[k], o[k]);
         }
-        int logn = 0;
-        while ((1 << logn) < n) ++logn;
-        // bit reversal along the axis
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-            const int coord = (e / stride) % n;
-            const int rev = __brev(coord) >> (32 - logn);
-            if (rev > coord) {
-                const int f = e + (rev - coord) * stride;
-                double2 t = x[e];
-                x[e] = x[f];
-                x[f] = t;
+    }
+}
+
+// One decimation-in-frequency pass of radix R over sub-length len of an axis of
+// element stride 2^lst: outputs stay in place, multiplied by w_len^(k i).
+template <int R>
+__device__ __forceinline__ void fft_pass(double2 *x, int total, int loglen, int lst, double sign, const double2 *tw,
+                                         int tw_n) {
+    constexpr int LR = R == 8 ? 3 : (R == 4 ? 2 : 1);
+    const int lsub = loglen - LR;  // log2(len / R)
+    const int step = tw_n >> loglen;
+    for (int t = threadIdx.x; t < total / R; t += blockDim.x) {
+        const int lo = t & ((1 << lst) - 1), rest = t >> lst;
+        const int i = rest & ((1 << lsub) - 1), blk = rest >> lsub;
+        const int base = (((blk << loglen) + i) << lst) + lo;
+        double2 v[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) v[j] = x[pad(base + (j << (lsub + lst)))];
+        dft<R>(v, sign);
+#pragma unroll
+        for (int k = 1; k < R; ++k) {
+            if (i) {
+                double2 w = __ldg(tw + (size_t)(k * i) * step);
+                w.y *= sign;
+                v[k] = cmulz(v[k], w);
             }
         }
-        __syncthreads();
-        for (int len = 2; len <= n; len <<= 1) {
-            const int half = len >> 1;
-            const int tstep = n / len;
-            for (int bfly = threadIdx.x; bfly < total / 2; bfly += blockDim.x) {
-                // decompose butterfly id into (line, position within line)
-                const int pos = bfly % (n / 2);
-                const int line = bfly / (n / 2);
-                const int lo_idx = line % stride, hi_idx = line / stride;
-                const int base = hi_idx * stride * n + lo_idx;
-                const int grp = pos / half, k = pos % half;
-                const int i0 = base + (grp * len + k) * stride;
-                const int i1 = i0 + half * stride;
-                const double2 w = tw[k * tstep];
-                const double2 u = x[i0], v0 = x[i1];
-                const double2 v = make_double2(v0.x * w.x - v0.y * w.y, v0.x * w.y + v0.y * w.x);
-                x[i0] = make_double2(u.x + v.x, u.y + v.y);
-                x[i1] = make_double2(u.x - v.x, u.y - v.y);
-            }
+#pragma unroll
+        for (int j = 0; j < R; ++j) x[pad(base + (j << (lsub + lst)))] = v[j];
+    }
+}
+
+// Where frequency f of an axis of length 2^logn is after fft_box (digit reversal:
+// radix 8 first, then what is left).
+__device__ __forceinline__ int fft_position(int f, int logn) {
+    int p = 0, left = logn;
+    while (left > 0) {
+        const int lr = left >= 3 ? 3 : left;
+        left -= lr;
+        p |= (f & ((1 << lr) - 1)) << left;
+        f >>= lr;
+    }
+    return p;
+}
+
+// DFT along every axis, sign +1 (inverse) or -1 (forward), no scaling; frequency
+// (f0, f1, f2) ends at position (fft_position(f0), ...).  Starts with a barrier.
+__device__ void fft_box(double2 *x, const LevelArgs &L, double sign, const double2 *tw, int tw_n) {
+    int lst = L.logS[0] + L.logS[1] + L.logS[2];
+    for (int ax = 0; ax < L.nd; ++ax) {
+        lst -= L.logS[ax];
+        for (int left = L.logS[ax]; left > 0;) {
             __syncthreads();
+            if (left >= 3) {
+                fft_pass<8>(x, L.P, left, lst, sign, tw, tw_n);
+                left -= 3;
+            } else if (left == 2) {
+                fft_pass<4>(x, L.P, left, lst, sign, tw, tw_n);
+                left = 0;
+            } else {
+                fft_pass<2>(x, L.P, left, lst, sign, tw, tw_n);
+                left = 0;
+            }
         }
     }
+    __syncthreads();
 }
 
-__device__ __forceinline__ void unravel(int e, const int *S, int *j) {
-    j[2] = e % S[2];
-    j[1] = (e / S[2]) % S[1];
-    j[0] = e / (S[1] * S[2]);
+// This CTA's level and its box within the level.
+__device__ __forceinline__ int find_level(const AllLevels &A, int &box) {
+    int l = 0;
+    while (l + 1 < A.levels && (int)blockIdx.x >= A.lv[l + 1].blk0) ++l;
+    box = blockIdx.x - A.lv[l].blk0;
+    return l;
 }
 
-// Read the unshifted spectrum value at index u (per axis), from either a full
-// complex array or a D2Z half spectrum (last axis N/2 + 1) with Hermitian
-// completion X[u] = conj(X[-u]).
-__device__ __forceinline__ double2 read_spec(const double2 *X, int half, const int *N, int nd, const int *u) {
-    if (!half) {
-        int64_t idx = 0;
-        for (int a = 0; a < nd; ++a) idx = idx * N[a] + u[a];
-        return X[idx];
-    }
-    const int last = nd - 1;
-    const int hl = N[last] / 2 + 1;
-    int v[3] = {u[0], u[1], u[2]};
-    bool cj = false;
-    if (u[last] >= hl) {
-        cj = true;
-        for (int a = 0; a < nd; ++a) v[a] = (N[a] - u[a]) % N[a];
-    }
-    int64_t idx = 0;
-    for (int a = 0; a < nd; ++a) idx = idx * (a == last ? hl : N[a]) + v[a];
-    double2 r = X[idx];
-    if (cj) r.y = -r.y;
-    return r;
+// element e of a box -> coordinates
+__device__ __forceinline__ void unravel(int e, const LevelArgs &L, int *j) {
+    j[2] = e & (L.S[2] - 1);
+    j[1] = (e >> L.logS[2]) & (L.S[1] - 1);
+    j[0] = e >> (L.logS[1] + L.logS[2]);
 }
 
 struct FwdArgs {
@@ -186,7 +261,6 @@ struct FwdArgs {
     int shifted;       // X is already in shifted order (Fourier input)
     double in_scale;   // 1/sqrt(prod N) for spatial input
     const double *ssq;
-    const double *g;   // packed g of the level (prod S)
     const int32_t *centres;
     double scale;
     int half_mask;
@@ -194,43 +268,82 @@ struct FwdArgs {
     double *keys;
 };
 
-__global__ void __launch_bounds__(THREADS) box_forward_kernel(LevelArgs L, FwdArgs A) {
+// Shared memory of a box kernel: the padded patch, then per axis and support
+// element two index tables.
+size_t box_smem(const LevelArgs &L) {
+    return sizeof(double2) * (size_t)(L.P + (L.P >> 3)) + 3 * sizeof(int) * (size_t)(L.S[0] + L.S[1] + L.S[2]);
+}
+
+// Bound: HBM and L2 (16 B read and 24 B written per coefficient); what is spent is
+// mostly shared-memory passes and FP64 work of the box FFTs.  All index
+// arithmetic with divisions is done once per axis and support element in tables.
+__global__ void __launch_bounds__(THREADS, 3) box_forward_kernel(AllLevels LV, FwdArgs A) {
     extern __shared__ double2 sm[];
+    int lbox;
+    const LevelArgs &L = LV.lv[find_level(LV, lbox)];
     double2 *patch = sm;
-    double2 *tw = sm + L.P;
-    const int box = L.box0 + blockIdx.x;
-    int cen[3] = {0, 0, 0}, r[3] = {0, 0, 0};
-    for (int a = 0; a < L.nd; ++a) {
-        cen[a] = A.centres[box * L.nd + a];
+    int *tab = reinterpret_cast<int *>(sm + L.P + (L.P >> 3));
+    const int ST = L.S[0] + L.S[1] + L.S[2];
+    int *tk = tab, *tu = tab + ST, *tq = tab + 2 * ST;  // shifted index, unshifted index, patch coordinate
+    const int box = L.box0 + lbox;
+    const int off[3] = {0, L.S[0], L.S[0] + L.S[1]};
+    for (int a = 0; a < 3; ++a) {
+        const int c = a < L.nd ? A.centres[box * L.nd + a] : 0;
         // forward rolls: ((centre + N/2) + N/2) // bhs   (transforms.py:626,665-673)
-        const int ri = floordiv(cen[a] + L.N[a] / 2 + L.N[a] / 2, L.bhs[a]);
-        r[a] = (1 - 2 * (ri & 1)) * (L.bhs[a] / 2);
-    }
-    for (int e = threadIdx.x; e < L.P; e += blockDim.x) {
-        int j[3];
-        unravel(e, L.S, j);
-        int k[3] = {0, 0, 0}, u[3] = {0, 0, 0}, q[3] = {0, 0, 0};
-        int64_t kflat = 0;
-        for (int a = 0; a < L.nd; ++a) {
-            k[a] = imod(cen[a] + L.N[a] / 2 - L.S[a] / 2 + j[a], L.N[a]);
-            u[a] = imod(k[a] + L.N[a] / 2, L.N[a]);
-            q[a] = imod(j[a] - L.S[a] / 2 + r[a], L.S[a]);
-            kflat = kflat * L.N[a] + k[a];
+        const int ri = floordiv(c + L.N[a] / 2 + L.N[a] / 2, L.bhs[a]);
+        const int r = a < L.nd ? (1 - 2 * (ri & 1)) * (L.bhs[a] / 2) : 0;
+        for (int j = threadIdx.x; j < L.S[a]; j += blockDim.x) {
+            const int k = a < L.nd ? imod(c + L.N[a] / 2 - L.S[a] / 2 + j, L.N[a]) : 0;
+            tk[off[a] + j] = k;
+            tu[off[a] + j] = imod(k + L.N[a] / 2, L.N[a]);
+            tq[off[a] + j] = imod(j - L.S[a] / 2 + r, L.S[a]);
         }
-        const double2 v = A.shifted ? A.X[kflat] : read_spec(A.X, A.half, L.N, L.nd, u);
-        // unitary spectrum / sum g^2, then * g (transforms.py:731, :663)
-        const double s = A.ssq[kflat], gv = A.g[e];
-        const double2 w = make_double2(v.x * A.in_scale / s * gv, v.y * A.in_scale / s * gv);
-        const int qf = (q[0] * L.S[1] + q[1]) * L.S[2] + q[2];
-        patch[qf] = w;
     }
     __syncthreads();
-    smem_fft(patch, L.S, L.nd, +1, tw);
-    const int64_t base = L.c0 + (int64_t)blockIdx.x * L.P;
+    const int last = L.nd - 1, hl = L.N[last] / 2 + 1;
     for (int e = threadIdx.x; e < L.P; e += blockDim.x) {
-        const int64_t loc = (int64_t)blockIdx.x * L.P + e;
+        int j[3], k[3], u[3], q[3];
+        unravel(e, L, j);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            k[a] = tk[off[a] + j[a]];
+            u[a] = tu[off[a] + j[a]];
+            q[a] = tq[off[a] + j[a]];
+        }
+        int64_t kflat = 0;
+        for (int a = 0; a < L.nd; ++a) kflat = kflat * L.N[a] + k[a];
+        double2 v;
+        if (A.shifted) {
+            v = A.X[kflat];
+        } else {
+            // a D2Z half spectrum (last axis N/2 + 1) is completed by X[u] = conj(X[-u])
+            const bool cj = A.half && u[last] >= hl;
+            int64_t idx = 0;
+            for (int a = 0; a < L.nd; ++a) {
+                const int w = cj ? (u[a] ? L.N[a] - u[a] : 0) : u[a];
+                idx = idx * (A.half && a == last ? hl : L.N[a]) + w;
+            }
+            v = __ldg(A.X + idx);
+            if (cj) v.y = -v.y;
+        }
+        // unitary spectrum / sum g^2, then * g (transforms.py:731, :663)
+        const double s = __ldg(A.ssq + kflat), gv = __ldg(L.g + e);
+        patch[pad((((q[0] << L.logS[1]) + q[1]) << L.logS[2]) + q[2])] =
+            make_double2(v.x * A.in_scale / s * gv, v.y * A.in_scale / s * gv);
+    }
+    fft_box(patch, L, 1.0, LV.tw, LV.tw_n);
+    // the tables now hold the frequencies' positions
+    for (int a = 0; a < 3; ++a)
+        for (int j = threadIdx.x; j < L.S[a]; j += blockDim.x) tq[off[a] + j] = fft_position(j, L.logS[a]);
+    __syncthreads();
+    const int64_t base = L.c0 + (int64_t)lbox * L.P;
+    for (int e = threadIdx.x; e < L.P; e += blockDim.x) {
+        int j[3];
+        unravel(e, L, j);
+        const int p = (((tq[j[0]] << L.logS[1]) + tq[off[1] + j[1]]) << L.logS[2]) + tq[off[2] + j[2]];
+        const int64_t loc = (int64_t)lbox * L.P + e;
         const double m = (!A.half_mask || loc < L.seg / 2) ? A.scale * L.inv_sqrtS : 0.0;
-        const double2 v = patch[e];
+        const double2 v = patch[pad(p)];
         const double re = v.x * m, im = v.y * m;
         A.coeffs[base + e] = make_double2(re, im);
         if (A.keys) A.keys[base + e] = __dsqrt_rn(__dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im)));
@@ -239,7 +352,6 @@ __global__ void __launch_bounds__(THREADS) box_forward_kernel(LevelArgs L, FwdAr
 
 struct SynArgs {
     const double2 *coeffs;
-    const double *g;
     const int32_t *centres;
     int adjoint;       // forward roll convention
     double2 *contrib;  // per-box contributions, coefficient layout
@@ -247,35 +359,41 @@ struct SynArgs {
 
 // Per box: unitary FFT of the coefficient block, fftshift, unroll and window
 // (transforms.py:826-837).
-__global__ void __launch_bounds__(THREADS) box_synth_kernel(LevelArgs L, SynArgs A) {
+__global__ void __launch_bounds__(THREADS, 3) box_synth_kernel(AllLevels LV, SynArgs A) {
     extern __shared__ double2 sm[];
+    int lbox;
+    const LevelArgs &L = LV.lv[find_level(LV, lbox)];
     double2 *patch = sm;
-    double2 *tw = sm + L.P;
-    const int box = L.box0 + blockIdx.x;
-    const int64_t base = L.c0 + (int64_t)blockIdx.x * L.P;
-    for (int e = threadIdx.x; e < L.P; e += blockDim.x) patch[e] = A.coeffs[base + e];
-    __syncthreads();
-    smem_fft(patch, L.S, L.nd, -1, tw);
-    int r[3] = {0, 0, 0};
-    for (int a = 0; a < L.nd; ++a) {
-        const int c = A.centres[box * L.nd + a];
+    int *tq = reinterpret_cast<int *>(sm + L.P + (L.P >> 3));
+    const int box = L.box0 + lbox;
+    const int off[3] = {0, L.S[0], L.S[0] + L.S[1]};
+    const int64_t base = L.c0 + (int64_t)lbox * L.P;
+    for (int a = 0; a < 3; ++a) {
+        const int c = a < L.nd ? A.centres[box * L.nd + a] : 0;
         const int shift = A.adjoint ? L.N[a] : L.N[a] / 2;
         const int ri = floordiv(c + shift, L.bhs[a]);
-        r[a] = (1 - 2 * (ri & 1)) * (L.bhs[a] / 2);
+        const int r = a < L.nd ? (1 - 2 * (ri & 1)) * (L.bhs[a] / 2) : 0;
+        for (int j = threadIdx.x; j < L.S[a]; j += blockDim.x)
+            tq[off[a] + j] = fft_position(imod(j + r + L.S[a] / 2, L.S[a]), L.logS[a]);
     }
+    for (int e = threadIdx.x; e < L.P; e += blockDim.x) patch[pad(e)] = __ldg(A.coeffs + base + e);
+    fft_box(patch, L, -1.0, LV.tw, LV.tw_n);
     for (int e = threadIdx.x; e < L.P; e += blockDim.x) {
         int j[3];
-        unravel(e, L.S, j);
-        int q[3] = {0, 0, 0};
-        for (int a = 0; a < L.nd; ++a) q[a] = imod(j[a] + r[a] + L.S[a] / 2, L.S[a]);
-        const double2 v = patch[(q[0] * L.S[1] + q[1]) * L.S[2] + q[2]];
-        const double s = A.g[e] * L.inv_sqrtS;
+        unravel(e, L, j);
+        const int p = (((tq[j[0]] << L.logS[1]) + tq[off[1] + j[1]]) << L.logS[2]) + tq[off[2] + j[2]];
+        const double2 v = patch[pad(p)];
+        const double s = __ldg(L.g + e) * L.inv_sqrtS;
         A.contrib[base + e] = make_double2(v.x * s, v.y * s);
     }
 }
 
+// Boxes covering a Fourier bin, per level and axis: cand + (cand_off[a] + k) * 4
+// lists the at most 4 (lattice index, support element) pairs of shifted index k,
+// closed by a pair (-1, 0); made with the plan (no divisions in the kernel).
 struct GatherLevel {
-    int cnt[3], first[3], step[3], S[3];
+    int cnt[3], S[3];
+    int64_t cand_off[3];
     int64_t lat_off;
     int box0;
     int64_t c0;
@@ -287,7 +405,7 @@ struct GatherArgs {
     int N[3];
     GatherLevel lv[8];
     const int32_t *lattice;
-    const int32_t *centres;
+    const int2 *cand;
     const double2 *contrib;
     const double *ssq;   // divide by sum g^2 (adjoint) when not NULL
     int fourier_out;     // write the shifted spectrum directly
@@ -313,53 +431,30 @@ __global__ void __launch_bounds__(THREADS) synth_gather_kernel(GatherArgs A) {
     double sr = 0.0, si = 0.0;
     for (int l = 0; l < A.levels; ++l) {
         const GatherLevel &G = A.lv[l];
-        // candidate lattice indices per axis (at most 4 each)
-        int cand[3][4], nc[3] = {1, 1, 1}, jj[3][4];
-        cand[1][0] = cand[2][0] = 0;
-        jj[1][0] = jj[2][0] = 0;
-        bool none = false;
-        for (int a = 0; a < A.nd; ++a) {
-            nc[a] = 0;
-            const int N = A.N[a], S = G.S[a], st = G.step[a];
-            // box i covers k iff (k - (first + i st + N/2) + S/2) mod N < S
-            const int z = imod(k[a] - N / 2 + S / 2 - G.first[a], N);
-            // range 1: i st <= z, z - i st < S
-            int ilo = floordiv(z - S, st) + 1, ihi = floordiv(z, st);
-            if (ilo < 0) ilo = 0;
-            if (ihi > G.cnt[a] - 1) ihi = G.cnt[a] - 1;
-            for (int i = ilo; i <= ihi && nc[a] < 4; ++i) {
-                cand[a][nc[a]] = i;
-                jj[a][nc[a]] = z - i * st;
-                nc[a]++;
-            }
-            // range 2: i st > z and z - i st + N < S
-            ilo = floordiv(z + N - S, st) + 1;
-            if (ilo <= ihi) ilo = ihi + 1;
-            ihi = G.cnt[a] - 1;
-            for (int i = ilo; i <= ihi && nc[a] < 4; ++i) {
-                if (i * st <= z) continue;
-                cand[a][nc[a]] = i;
-                jj[a][nc[a]] = z - i * st + N;
-                nc[a]++;
-            }
-            if (nc[a] == 0) none = true;
-        }
-        if (none) continue;
-        for (int i0 = 0; i0 < nc[0]; ++i0)
-            for (int i1 = 0; i1 < nc[1]; ++i1)
-                for (int i2 = 0; i2 < nc[2]; ++i2) {
-                    const int ci[3] = {cand[0][i0], cand[1][i1], cand[2][i2]};
-                    const int cj[3] = {jj[0][i0], jj[1][i1], jj[2][i2]};
-                    int64_t li = 0;
-                    for (int a = 0; a < A.nd; ++a) li = li * G.cnt[a] + ci[a];
-                    const int box = A.lattice[G.lat_off + li];
+        const int2 *c0 = A.cand + (G.cand_off[0] + k[0]) * 4;
+        const int2 *c1 = A.cand + (G.cand_off[1] + k[1]) * 4, *c2 = A.cand + (G.cand_off[2] + k[2]) * 4;
+#pragma unroll 1
+        for (int i0 = 0; i0 < 4; ++i0) {
+            const int2 q0 = __ldg(c0 + i0);
+            if (q0.x < 0) break;
+#pragma unroll 1
+            for (int i1 = 0; i1 < 4; ++i1) {
+                const int2 q1 = A.nd > 1 ? __ldg(c1 + i1) : make_int2(i1 ? -1 : 0, 0);
+                if (q1.x < 0) break;
+#pragma unroll 1
+                for (int i2 = 0; i2 < 4; ++i2) {
+                    const int2 q2 = A.nd > 2 ? __ldg(c2 + i2) : make_int2(i2 ? -1 : 0, 0);
+                    if (q2.x < 0) break;
+                    const int64_t li = ((int64_t)q0.x * G.cnt[1] + q1.x) * G.cnt[2] + q2.x;
+                    const int box = __ldg(A.lattice + G.lat_off + li);
                     if (box < 0) continue;
-                    int e = 0;
-                    for (int a = 0; a < A.nd; ++a) e = e * G.S[a] + cj[a];
-                    const double2 v = A.contrib[G.c0 + (int64_t)(box - G.box0) * G.P + e];
+                    const int e = (q0.y * G.S[1] + q1.y) * G.S[2] + q2.y;
+                    const double2 v = __ldg(A.contrib + G.c0 + (int64_t)(box - G.box0) * G.P + e);
                     sr += v.x;
                     si += v.y;
                 }
+            }
+        }
     }
     if (A.ssq) {
         const double s = A.ssq[kf];
@@ -486,6 +581,57 @@ extern "C" int msgb_mswpt_create(const msgb_mswpt_desc *d, msgb_mswpt **out) {
         msgb_mswpt_destroy(p);
         return fail(MSGB_ERR_CUDA, "msgb_mswpt_create: %s", cudaGetErrorString(e));
     }
+    for (int l = 0; l < L; ++l)
+        for (int a = 0; a < nd; ++a) p->tw_n = 2 * p->bshape[l * nd + a] > p->tw_n ? 2 * p->bshape[l * nd + a] : p->tw_n;
+    std::vector<double> tw(2 * (size_t)p->tw_n);
+    for (int m = 0; m < p->tw_n; ++m) {
+        // from the first octant: exact at the multiples of a quarter turn
+        const int q = (int)((8LL * m) / p->tw_n);  // octant
+        const double a = 2.0 * 3.14159265358979323846 * m / p->tw_n;
+        double c = cos(a), s = sin(a);
+        if ((4LL * m) % p->tw_n == 0) {
+            const int k = (int)((4LL * m) / p->tw_n);
+            c = k == 0 ? 1.0 : (k == 2 ? -1.0 : 0.0);
+            s = k == 1 ? 1.0 : (k == 3 ? -1.0 : 0.0);
+        } else {
+            const double e = 2.0 * 3.14159265358979323846 / p->tw_n;  // angle from the nearest quarter turn
+            const int k = (q + 1) / 2;                                // quarter turns
+            const double b = e * (m - (double)k * p->tw_n / 4.0);
+            const double cb = cos(b), sb = sin(b);
+            c = k % 4 == 0 ? cb : (k % 4 == 1 ? -sb : (k % 4 == 2 ? -cb : sb));
+            s = k % 4 == 0 ? sb : (k % 4 == 1 ? cb : (k % 4 == 2 ? -sb : -cb));
+        }
+        tw[2 * m] = c;
+        tw[2 * m + 1] = s;
+    }
+    // candidate lists in lattice order: first those whose support starts at or
+    // below the bin, then those that reach it around the end of the axis
+    std::vector<int2> cand;
+    p->cand_off.assign((size_t)L * 3, 0);
+    for (int l = 0; l < L; ++l)
+        for (int a = 0; a < nd; ++a) {
+            const int N = p->N[a], S = 2 * p->bshape[l * nd + a], step = p->lat_step[l * nd + a];
+            const int cnt = p->lat_cnt[l * nd + a], first = p->lat_first[l * nd + a];
+            p->cand_off[l * 3 + a] = (int64_t)cand.size() / 4;
+            for (int k = 0; k < N; ++k) {
+                // box i covers k iff (k - (first + i step + N/2) + S/2) mod N < S
+                int z = (k - N / 2 + S / 2 - first) % N;
+                if (z < 0) z += N;
+                int2 c[4] = {make_int2(-1, 0), make_int2(-1, 0), make_int2(-1, 0), make_int2(-1, 0)};
+                int n = 0;
+                for (int i = 0; i < cnt && n < 4; ++i)
+                    if (z - i * step >= 0 && z - i * step < S) c[n++] = make_int2(i, z - i * step);
+                for (int i = 0; i < cnt && n < 4; ++i)
+                    if (z - i * step < 0 && z - i * step + N < S) c[n++] = make_int2(i, z - i * step + N);
+                cand.insert(cand.end(), c, c + 4);
+            }
+        }
+    up((void **)&p->d_cand, cand.data(), sizeof(int2) * cand.size());
+    up((void **)&p->d_tw, tw.data(), sizeof(double) * tw.size());
+    if (e != cudaSuccess) {
+        msgb_mswpt_destroy(p);
+        return fail(MSGB_ERR_CUDA, "msgb_mswpt_create: %s", cudaGetErrorString(e));
+    }
     int n[3] = {p->N[0], p->N[1], p->N[2]};
     size_t w1 = 0, w2 = 0;
     cufftResult r = cufftCreate(&p->plan_d2z);
@@ -513,6 +659,8 @@ extern "C" int msgb_mswpt_destroy(msgb_mswpt *p) {
     cudaFree(p->d_bcum);
     cudaFree(p->d_bl);
     cudaFree(p->d_bshape);
+    cudaFree(p->d_tw);
+    cudaFree(p->d_cand);
     if (p->plan_d2z) cufftDestroy(p->plan_d2z);
     if (p->plan_z2z) cufftDestroy(p->plan_z2z);
     delete p;
@@ -568,16 +716,12 @@ extern "C" int msgb_mswpt_forward(const msgb_mswpt *p, const double *in, int is_
     A.half_mask = apply_half_mask;
     A.coeffs = (double2 *)coeffs;
     A.keys = keys;
-    for (int l = 0; l < p->levels; ++l) {
-        LevelArgs L = level_args(p, l);
-        if (L.nbox == 0) continue;
-        A.g = p->d_gfilt + p->goff[l];
-        int maxS = 1;
-        for (int a = 0; a < 3; ++a) maxS = L.S[a] > maxS ? L.S[a] : maxS;
-        const size_t smem = sizeof(double2) * (L.P + maxS);
-        if (int e = smem_attr((const void *)box_forward_kernel, smem)) return e;
-        box_forward_kernel<<<L.nbox, THREADS, smem, st>>>(L, A);
-    }
+    AllLevels LV;
+    const int blocks = all_levels(p, LV);
+    size_t smem = 0;
+    for (int l = 0; l < LV.levels; ++l) smem = box_smem(LV.lv[l]) > smem ? box_smem(LV.lv[l]) : smem;
+    if (int e = smem_attr((const void *)box_forward_kernel, smem)) return e;
+    box_forward_kernel<<<blocks, THREADS, smem, st>>>(LV, A);
     return check_launch("msgb_mswpt_forward");
 }
 
@@ -602,16 +746,12 @@ extern "C" int msgb_mswpt_synthesis(const msgb_mswpt *p, const double *coeffs, i
     A.centres = p->d_centres;
     A.adjoint = adjoint;
     A.contrib = contrib;
-    for (int l = 0; l < p->levels; ++l) {
-        LevelArgs L = level_args(p, l);
-        if (L.nbox == 0) continue;
-        A.g = p->d_gfilt + p->goff[l];
-        int maxS = 1;
-        for (int a = 0; a < 3; ++a) maxS = L.S[a] > maxS ? L.S[a] : maxS;
-        const size_t smem = sizeof(double2) * (L.P + maxS);
-        if (int e = smem_attr((const void *)box_synth_kernel, smem)) return e;
-        box_synth_kernel<<<L.nbox, THREADS, smem, st>>>(L, A);
-    }
+    AllLevels LV;
+    const int box_blocks = all_levels(p, LV);
+    size_t smem = 0;
+    for (int l = 0; l < LV.levels; ++l) smem = box_smem(LV.lv[l]) > smem ? box_smem(LV.lv[l]) : smem;
+    if (int e = smem_attr((const void *)box_synth_kernel, smem)) return e;
+    box_synth_kernel<<<box_blocks, THREADS, smem, st>>>(LV, A);
     GatherArgs G{};
     G.nd = p->nd;
     G.levels = p->levels;
@@ -622,8 +762,7 @@ extern "C" int msgb_mswpt_synthesis(const msgb_mswpt *p, const double *coeffs, i
         for (int a = 0; a < 3; ++a) {
             const bool in = a < p->nd;
             gl.cnt[a] = in ? p->lat_cnt[l * p->nd + a] : 1;
-            gl.first[a] = in ? p->lat_first[l * p->nd + a] : 0;
-            gl.step[a] = in ? p->lat_step[l * p->nd + a] : 1;
+            gl.cand_off[a] = in ? p->cand_off[l * 3 + a] : 0;
             gl.S[a] = in ? 2 * p->bshape[l * p->nd + a] : 1;
             gl.P *= gl.S[a];
         }
@@ -632,7 +771,7 @@ extern "C" int msgb_mswpt_synthesis(const msgb_mswpt *p, const double *coeffs, i
         gl.c0 = p->ccum[l];
     }
     G.lattice = p->d_lattice;
-    G.centres = p->d_centres;
+    G.cand = p->d_cand;
     G.contrib = contrib;
     G.ssq = adjoint ? p->d_ssq : nullptr;
     G.fourier_out = fourier_out;
