@@ -107,3 +107,32 @@ def test_other_dimensions(d, shape):
         a, b = np.meshgrid(np.arange(shape[0]), np.arange(shape[1]), indexing="ij")
         pos = np.stack([a.ravel(), b.ravel(), np.full(a.size, 0)], -1) * 1e-4
     _compare(d, N, pos, 35, _beams(d, 90, N * 1e-4, dev, d))
+
+
+@pytest.mark.parametrize("d", [2, 3])
+def test_trajectory_candidates_left_out_do_not_matter(d):
+    """Beams in a strongly refracting medium: with culling (tile test, the test on
+    four of a tile's records, group test) against every beam at every sensor."""
+    import beamax_b200 as bb
+    from beamax_b200.utils.interp import make_c_function_from_grid
+
+    dev = _dev()
+    N, dx = (128, 1e-4) if d == 2 else (48, 1e-4)
+    ax = np.stack(np.meshgrid(*[np.arange(N)] * d, indexing="ij"), 0)
+    c = 1500 * (1 + 0.08 * np.sin(2 * np.pi * ax[0] / 40) * np.cos(2 * np.pi * ax[-1] / 33))
+    med = make_c_function_from_grid(c, (dx,) * d, method="bspline3", boundary="clamp")
+    dom = bb.Domain(N=(N,) * d, dx=(dx,) * d, periodic=(False,) * d, cfl=0.3, c=med)
+    mask = np.zeros((N,) * d)
+    mask[0] = 1
+    sens = bb.Sensor(dom, binary_mask=mask)
+    ts = np.arange(300) * 0.3 * dx / 1620
+    bt = _beams(d, 200, N * dx, dev, 11 + d, width=N * dx / 25)
+    ode = bb.gb.gb_solvers.solve_ODE_base
+    mk = lambda cut: bb.MSGBSolver(8, "top_n", 8, "spatial", ode, "scan_real", precision="fp32", cutoff=cut)
+    y, y0 = (mk(cut).sum_forward(bt, dom, sens, ts).double() for cut in (16.0, 0.0))
+    # focusing raises an amplitude by at most 10 here
+    left_out = 1.2e-7 * 40 * float(bt.a0.abs().sum())
+    assert float((y - y0).abs().max()) <= left_out + 1e-5 * float(y0.abs().max())
+    data = torch.randn(y0.shape, generator=torch.Generator(device=dev).manual_seed(3), device=dev)
+    g, g0 = (mk(cut).gather_adjoint(bt, dom, sens, ts, data) for cut in (16.0, 0.0))
+    assert float((g - g0).norm()) <= 1e-5 * float(g0.norm())
