@@ -57,9 +57,13 @@ __global__ void take_last_kernel(const int32_t *sorted_idx, int64_t total, int64
 // above it are compacted in index order and only they are sorted: the same list as
 // sorting everything.  1024^2 (4.2 million keys, n = 262,144): 400 us for the full
 // sort, 150 us this way.
-// The full sort stays for small sets (it is one or a few short kernels) and where
-// more than half is wanted.
-constexpr int64_t kSelectFrom = 8192;
+// A sort of more than a few thousand pairs takes 8 passes of 8 us whatever its size,
+// and the select 7 of 5 us: it pays from about two million keys on, or where the
+// selected fit the sort's single-kernel form (262,144 keys, n = 12,815: 210 us with
+// the transform by selecting, 202 by sorting everything before).
+inline bool select_first(int64_t total, int64_t n) {
+    return n <= total / 2 && (total >= (int64_t(1) << 21) || (n <= 2048 && total > 8192));
+}
 constexpr int kSelBits = 13, kSelBins = 1 << kSelBits, kSelThreads = 512;
 
 struct SelState {
@@ -557,7 +561,7 @@ extern "C" int msgb_topn(const double *keys, const double *coeffs, int64_t total
     int32_t *vin = (int32_t *)(ws + l.vin), *vout = (int32_t *)(ws + l.vout);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     size_t cb = l.cub_bytes;
-    if (n <= total / 2 && total > kSelectFrom) {
+    if (select_first(total, n)) {
         SelState *s = (SelState *)(ws + l.state);
         int64_t *count = (int64_t *)(s + 1);
         unsigned *hist = (unsigned *)(ws + l.hist);

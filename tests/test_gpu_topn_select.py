@@ -29,7 +29,7 @@ def _keys(kind, total, rng):
 
 
 @pytest.mark.parametrize("kind", ["random", "ties", "equal", "halfzero", "special"])
-@pytest.mark.parametrize("total", [100, 8192, 8193, 20000, 300001])
+@pytest.mark.parametrize("total", [100, 8192, 8193, 20000, 300001, (1 << 21) - 1, (1 << 21) + 3])
 def test_selected_indices_and_order(kind, total):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
@@ -43,7 +43,7 @@ def test_selected_indices_and_order(kind, total):
     kd = torch.from_numpy(keys).to(dev)
     c = torch.from_numpy(rng.standard_normal((total, 2))).to(dev)
     L = _lib.lib()
-    for n in sorted({1, 2, 37, total // 3, total // 2, total // 2 + 1, total}):
+    for n in sorted({1, 2, 37, min(total, 2048), min(total, 2049), total // 3, total // 2, total // 2 + 1, total}):
         nbytes = L.msgb_topn_workspace_size(total, n)
         ws = torch.full((nbytes,), 0x5A, dtype=torch.uint8, device=dev)
         idx = torch.empty(n, dtype=torch.int64, device=dev)
