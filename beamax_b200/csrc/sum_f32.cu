@@ -847,7 +847,7 @@ __device__ __forceinline__ void record_pass(const ProbArgs &P, const BeamArgs &B
         __syncwarp();
     }
     const double t = !TRAJ && tv ? P.ts[t_first + lane] : 0.0;
-#pragma unroll 2
+#pragma unroll (TRAJ ? 2 : 1)
     for (int k = 0; k < PW; ++k) {
         if (k >= mine) break;
         const int i = warp + k * NW;
@@ -1250,10 +1250,13 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                         const int i0 = take_bit(bits), i1 = take_bit(bits), i2 = take_bit(bits), i3 = take_bit(bits);
                         cf2 za, fa, qa, zb, fb, qb;
                         int direct = seed_pair<D>(rec, i0, i1, lane, run, skip, za, fa, qa);
-                        if (i2 >= 0) {
-                            direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+                        zb = fb = qb = cf2{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                        if (i2 >= 0) direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+                        {
                             // z_{k+1} = z_k f_k, f_{k+1} = f_k q; sensors 2h, 2h + 1
-                            // share a paired compensated addition
+                            // share a paired compensated addition (one or two beams
+                            // left: the other pair is zero -- a second loop for them
+                            // costs more in instruction fetches than it saves)
 #pragma unroll
                             for (int h = 0; h < GS / 2; ++h) {
                                 if (h > 0) {
@@ -1269,18 +1272,6 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                                 fb = cmul2(fb, qb);
                                 const float2 v1 = __fadd2_rn(za.re, zb.re);
                                 kahan_add2(acc2[h], cmp2[h], make_float2(v0.x + v0.y, v1.x + v1.y));
-                            }
-                        } else {
-#pragma unroll
-                            for (int h = 0; h < GS / 2; ++h) {
-                                if (h > 0) {
-                                    za = cmul2(za, fa);
-                                    fa = cmul2(fa, qa);
-                                }
-                                const float v0 = za.re.x + za.re.y;
-                                za = cmul2(za, fa);
-                                fa = cmul2(fa, qa);
-                                kahan_add2(acc2[h], cmp2[h], make_float2(v0, za.re.x + za.re.y));
                             }
                         }
                         if (!__any_sync(0xffffffffu, direct != 0)) continue;
@@ -1500,8 +1491,9 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                         i3 = take_bit(bits);
                         cf2 za, fa, qa, zb, fb, qb;
                         int direct = seed_pair<D>(rec, i0, i1, lane, run, skip, za, fa, qa);
-                        if (i2 >= 0) {
-                            direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+                        zb = fb = qb = cf2{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                        if (i2 >= 0) direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+                        {
 #pragma unroll
                             for (int k = 0; k < GS; ++k) {
                                 if (k > 0) {
@@ -1515,17 +1507,6 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                                 ai = __ffma2_rn(neg2(dk), za.im, ai);
                                 br = __ffma2_rn(dk, zb.re, br);
                                 bi = __ffma2_rn(neg2(dk), zb.im, bi);
-                            }
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < GS; ++k) {
-                                if (k > 0) {
-                                    za = cmul2(za, fa);
-                                    fa = cmul2(fa, qa);
-                                }
-                                const float2 dk = make_float2(dv[k], dv[k]);
-                                ar = __ffma2_rn(dk, za.re, ar);
-                                ai = __ffma2_rn(neg2(dk), za.im, ai);
                             }
                         }
                         if (__any_sync(0xffffffffu, direct != 0)) {
