@@ -724,6 +724,32 @@ __constant__ float DP_E32[7] = {(float)(35.0 / 384 - 5179.0 / 57600),
                                 (float)(11.0 / 84 - 187.0 / 2100),
                                 (float)(-1.0 / 40)};
 
+// acc += sum over j < s of DP_A[s][j] k_j, straight-line per stage: the stages'
+// loads are in flight together and the coefficients are constant operands (a loop
+// over j waited out each load: 39 % of the mixed integrator's time).
+template <int S, typename K64, int ND>
+__device__ __forceinline__ void combine64(const K64 &k, double (&acc)[ND]) {
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        if (S == 6 && j == 1) continue;  // weight 0
+        double r[ND];
+        k.get(j, r);
+#pragma unroll
+        for (int c = 0; c < ND; ++c) acc[c] += DP_A[S][j] * r[c];
+    }
+}
+template <int S, typename K32, int NF>
+__device__ __forceinline__ void combine32(const K32 &k, float (&acc)[NF]) {
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        if (S == 6 && j == 1) continue;
+        float f[NF];
+        k.get(j, f);
+#pragma unroll
+        for (int c = 0; c < NF; ++c) acc[c] = fmaf(DP_A32[S][j], f[c], acc[c]);
+    }
+}
+
 // DopriBeam's step (save times landed on, no continuous extension) on the
 // mixed state.  Stages in shared memory: the FP64 ray stages, then the FP32
 // Hessian and amplitude stages, each entry strided by the block size.
@@ -789,18 +815,13 @@ struct DopriMix {
             for (int c = 0; c < ND; ++c) a64[c] = 0.0;
 #pragma unroll
             for (int c = 0; c < NF; ++c) a32[c] = 0.0f;
-#pragma unroll 1
-            for (int j = 0; j < s; ++j) {
-                const double a = DP_A[s][j];
-                const float af = DP_A32[s][j];
-                double r[ND];
-                float f[NF];
-                k64.get(j, r);
-                k32.get(j, f);
-#pragma unroll
-                for (int c = 0; c < ND; ++c) a64[c] += a * r[c];
-#pragma unroll
-                for (int c = 0; c < NF; ++c) a32[c] = fmaf(af, f[c], a32[c]);
+            switch (s) {
+                case 1: combine64<1>(k64, a64), combine32<1>(k32, a32); break;
+                case 2: combine64<2>(k64, a64), combine32<2>(k32, a32); break;
+                case 3: combine64<3>(k64, a64), combine32<3>(k32, a32); break;
+                case 4: combine64<4>(k64, a64), combine32<4>(k32, a32); break;
+                case 5: combine64<5>(k64, a64), combine32<5>(k32, a32); break;
+                default: combine64<6>(k64, a64), combine32<6>(k32, a32); break;
             }
 #pragma unroll
             for (int c = 0; c < ND; ++c) yt.r[c] = y.r[c] + hh * a64[c];
@@ -840,7 +861,8 @@ struct DopriMix {
 #pragma unroll
             for (int c = 0; c < ND; ++c) {
                 const float e = (float)(hh * e64[c]);
-                const float sc = fmaf(rt, (float)fmax(fabs(y.r[c]), fabs(yt.r[c])), at);
+                // (rounding is monotone: the same as rounding the larger)
+                const float sc = fmaf(rt, fmaxf(fabsf((float)y.r[c]), fabsf((float)yt.r[c])), at);
                 s32 = fmaf(e, __fdividef(e, sc * sc), s32);
             }
 #pragma unroll
@@ -860,7 +882,8 @@ struct DopriMix {
             rejected = true;
             return false;
         }
-        double fac = err == 0.0f ? 10.0 : fmin(10.0, fmax(0.2, (double)(0.9f * exp2f(-0.2f * log2f(err)))));
+        const float gr = 0.9f * exp2f(-0.2f * log2f(err));
+        double fac = err == 0.0f || gr > 10.0f ? 10.0 : (gr < 0.2f ? 0.2 : (double)gr);
         if (err <= 1.0f) {
             if (rejected) fac = fmin(fac, 1.0);
             rejected = false;
@@ -1056,7 +1079,8 @@ struct TrBeamsView {
 template <int D, int KIND>
 __global__ void tr_final_kernel(ProbArgs P, MediumArgs med, TrBeamsView B, int64_t n, OdeArgs o, double *rec64,
                                 int32_t *status) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    // dealt as the persistent lanes' beams: with few beams every warp has some
+    const int64_t i = first_beam();
     if (i >= n) return;
     DopriBeam<D, KIND> s;
 #pragma unroll
@@ -1184,7 +1208,11 @@ extern "C" int msgb_tr_final_states(const msgb_problem *prob, const msgb_medium 
               opts->dense_output, nullptr};
     TrBeamsView B{beams->x, beams->p, beams->M, beams->mode, beams->t0};
     const int blk = kOdeBlock;
-    const unsigned grid = (unsigned)((beams->n + blk - 1) / blk);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t full = (beams->n + blk - 1) / blk, spread = (beams->n + 1) / 2 < 2 * sms ? (beams->n + 1) / 2 : 2 * sms;
+    const unsigned grid = (unsigned)(full > spread ? full : spread);
     cudaStream_t st = as_stream(stream);
     switch (prob->ndim) {
         case 1: launch_by_kind<1>(M.kind, [&](auto kern, size_t sm) { kern<<<grid, blk, sm, st>>>(P, M, B, beams->n, O, rec64, status); },
