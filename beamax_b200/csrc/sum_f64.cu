@@ -88,9 +88,15 @@ __device__ __forceinline__ int reduced_sincos(double x, double &c, double &s, bo
 }
 
 // exp(x) = p * s1 * s2 with s1, s2 powers of two (two factors: the product may be
-// subnormal or zero); flip: its low bit is xored into the sign of s1.  far is set for
-// |x| >= 1400, inf and NaN.
+// subnormal or zero); flip: its low bit is xored into the sign of s1.  x below -1400
+// is taken as -1400: the product is zero either way, and in a large domain narrow
+// beams are that far from most sensors.  far is set for x >= 1400, inf and NaN.
 __device__ __forceinline__ void split_exp(double x, int flip, double &p, double &s1, double &s2, bool &far) {
+    const int hi = __double2hiint(x);
+    const bool off = (unsigned)(hi & 0x7fffffff) >= 0x4095e000u;  // |x| >= 1400
+    const bool zero = off && (unsigned)hi < 0xfff00000u && hi < 0;
+    far |= off && !zero;
+    if (zero) x = -1400.0;
     double nd = fma(x, kRed[3], kRed[6]);
     int n = __double2loint(nd);
     nd -= kRed[6];
@@ -101,7 +107,6 @@ __device__ __forceinline__ void split_exp(double x, int flip, double &p, double 
     for (int k = 1; k < 10; ++k) p = fma(p, r, kExp[k]);
     p = fma(p, r, kRed[7]);
     p = fma(p, r, kRed[7]);
-    far |= (unsigned)(__double2hiint(x) & 0x7fffffff) >= 0x4095e000u;
     const int n1 = n >> 1, n2 = n - n1;
     s1 = __hiloint2double(((n1 + 1023) << 20) ^ (flip << 31), 0);
     s2 = __hiloint2double((n2 + 1023) << 20, 0);
