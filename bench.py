@@ -293,10 +293,20 @@ def ode_flops_split(d: int):
 
 
 # ---------------------------------------------------------------- ours
-def launches_per_step(levels: int) -> int:
-    """Kernels of libmsgb launched per step (cuFFT's own kernels excluded)."""
-    fwd = levels + 1 + 2 + 1 + (1 + 2 + 1 + 1) + 1  # boxes, key bits, radix sort, take, init, prep(4), sum
-    adj = 1 + 5 + 1 + 1 + 1 + levels + 1 + 1        # init, prep+permute, gather, scatter, zero, boxes, synth, real
+def launches_per_step(hetero: bool, total_coeffs: int, n: int, nt: int, ns: int) -> int:
+    """Hand-written kernels of libmsgb launched per step (cuFFT's and CUB's own
+    kernels excluded)."""
+    select = total_coeffs >= 1 << 21 and n <= total_coeffs // 2
+    passes = 5 + -(-max(1, (total_coeffs - 1).bit_length()) // 13)
+    topn = 1 + passes + 2 if select else 2  # start, digit passes, gather of the keys, take; or key bits, take
+    prep = 4                                # tiling copy, check, clamp, tile description
+    if hetero:
+        sums, gather = 1 + 1, 1             # beam ODE, sum; gather
+    else:
+        split = ((ns + 127) // 128) * ((nt + 31) // 32) < 8 * 2 * 148
+        sums, gather = 2 + 1 + int(split), 2 + 1  # culling and closed-form tables, sum, its combination; gather
+    fwd = 1 + topn + 1 + prep + sums        # box transforms, selection, beam init
+    adj = 1 + prep + 1 + gather + 1 + 1 + 3  # beam init, data permutation, partials, scatter, synthesis
     return fwd + adj
 
 
@@ -400,11 +410,11 @@ def run_ours(args, rank, world, device):
     result = {"rank": rank, "t_step": total / args.steps, "t_fwd_kernel": t_fwd_kernel, "t_adj_kernel": t_adj_kernel,
               "t_ode": t_ode, "ode_steps": ode_steps, "ndim": len(dom.N), "hetero": W["hetero"],
               "nt": nt, "ns": ns, "n_beams": 2 * n,
-              # heterogeneous: one ODE and one summation call per trajectory chunk, each a prep + main kernel
-              "extra_launches": 3 * sum(1 for nm, *_ in spans if "traj" in nm or "ode" in nm),
+              # heterogeneous: chunks of trajectories beyond the one per call that launches_per_step counts
+              "extra_launches": 3 * max(0, sum(1 for nm, *_ in spans if "traj" in nm or "ode" in nm) - 3 * args.steps),
               "fwd_evals": fwd_evals, "adj_evals": adj_evals, "dense_step": dense_step, "clocks": clocks,
               "e2e_t": e2e_t, "h2d": p0.nbytes + nt * ns * 4, "d2h": nt * ns * 4 + p0.nbytes,
-              "levels": wpt.dyadic_decomp.num_levels, "workload": W["name"]}
+              "total_coeffs": wpt.total_coeffs, "workload": W["name"]}
 
     # FP64 plain path (dense, reference semantics): once, also the accuracy reference
     s32.release_trajectories()
@@ -828,7 +838,7 @@ def main():
                    "l2": "flushed (256 MiB write) between timed steps", "cutoff_efolds": args.cutoff},
         "e2e": {"value": world * r["dense_step"] / r["e2e_t"], "unit": UNIT, "h2d_bytes_per_step": r["h2d"],
                 "d2h_bytes_per_step": r["d2h"], "ms_per_step": r["e2e_t"] * 1e3},
-        "gpu_launches": args.steps * launches_per_step(r["levels"]) + r["extra_launches"],
+        "gpu_launches": args.steps * launches_per_step(r["hetero"], r["total_coeffs"], r["n_beams"] // 2, r["nt"], r["ns"]) + r["extra_launches"],
         "roofline": roof,
         "roofline_other": roof_other,
         "kernels": {"fwd32_s": r["t_fwd_kernel"], "adj32_s": r["t_adj_kernel"], "fwd_evals": r["fwd_evals"],

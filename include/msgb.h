@@ -87,7 +87,9 @@ typedef struct msgb_sensor_tiling {
 /* Options of the FP32 summation. */
 typedef struct msgb_sum_opts {
     double cutoff;           /* skip a (beam, tile) pair when the Gaussian exponent
-                                is provably above this many e-folds (<= 0: dense) */
+                                is provably above this many e-folds, and a (beam, 32
+                                times, 16 sensors) block of the tile beyond 4 more
+                                (<= 0: dense) */
     unsigned long long *eval_count; /* optional device counter: evaluated
                                 (beam, t, sensor) triples are added to it */
     const msgb_sensor_tiling *tiling; /* optional (NULL) */
