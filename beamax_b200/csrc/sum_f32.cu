@@ -802,7 +802,9 @@ __device__ __noinline__ void general_beam_time(const ProbArgs &P, const BeamArgs
 }
 
 // Write the records of the pass's beams beam_of(0 .. nb) and their masks alive[].
-// What a record needs beyond the test (the anchor phase, the amplitude) is formed
+// Bound: latency (dependent FP64 and MUFU chains of one record per warp); a third of
+// the homogeneous forward (15.7 of 48.6 ms at 512^2), half of the trajectory sums
+// before refine.  What a record needs beyond the test (the anchor phase, the amplitude) is formed
 // only when the beam reaches some group at some time.
 template <int D, bool TRAJ, typename BeamOf>
 __device__ __forceinline__ void record_pass(const ProbArgs &P, const BeamArgs &B, const TrajSrc<D> &T,
@@ -1078,7 +1080,10 @@ struct Split {
 
 // Work items a launch should have: 8 per resident CTA (2 per SM), so that the
 // last, unevenly filled wave is a small part of it.  Fewer tiles than that are
-// split over the beams, in ranges of at least kSplitMin (8 passes of both modes).
+// split over the beams, in ranges of at least kSplitMin (8 passes of both modes):
+// 4,096 coefficients at 128^2 ran 19 blocks for 3.9 ms, now 0.24 ms; a 512-point
+// sensor at 512^2 304 blocks in two waves for 31.0 ms, 18.9 ms without the split
+// after the other steps, 10.5 with it.
 constexpr int64_t kItemsWanted = 8 * 2 * 148;
 constexpr int64_t kSplitMin = 128;
 
@@ -1127,7 +1132,11 @@ __global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *p
 // added before one compensated addition).
 //
 // Bound: FP32 pipe (recurrence 8 FMA-pipe operations per triple, seed ~75 per 16
-// triples) with the seeds' MUFU work beside it.
+// triples) with the seeds' MUFU work beside it; measured 51 % (2D) and 58 % (3D) of
+// that pipe's cycles, the rest in pass barriers and latency.  512^2 homogeneous
+// (65,536 coefficients, 2,414 times, 2,044 sensors): 78.3 ms when every group
+// evaluated every survivor of the tile, 45.5 now; 1024^2 heterogeneous, 200,000
+// beams: 538 -> 173 ms; 128^3: 300 -> 116 ms.
 template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
 fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
@@ -1359,7 +1368,9 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
 // per-beam FP64 accumulators in shared memory (one owner thread per value and
 // pass).  The item then writes every accumulator (zeros included) to
 // part[tt][slot], and reduce_parts_kernel sums part over the time tiles in
-// order.  Each partial has one writer and every sum has a fixed order, so the
+// order.  Bound: as the forward, with more time at the pass barriers (FMA pipe
+// 43-45 %).  512^2: 86.4 -> 54.1 ms; 1024^2 heterogeneous 576 -> 195 ms; 128^3 504 ->
+// 151 ms.  Each partial has one writer and every sum has a fixed order, so the
 // result is bit-identical between runs; the work counter only hands out items.
 template <int D, bool TRAJ>
 struct AdjRange {

@@ -14,8 +14,10 @@
 // over all times and sensors in a fixed order (no atomics).
 //
 // Bound: FP64 pipe (16 lanes per scheduler), 45 operations per evaluation in 2D
-// forward and 55 in the transpose.  With the library's cos, sincos and exp an
-// evaluation issued 148 instructions, 62 of them FP64.
+// forward and 55 in the transpose; 83 % and 67 % of its cycles busy.  With the
+// library's cos, sincos and exp an evaluation issued 148 instructions, 62 of them
+// FP64.  256^2, 3,000 coefficients, 1,207 times, 1,020 sensors: forward 52.5 -> 24.0
+// ms, transpose 51.6 -> 34.0 ms.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -272,7 +274,8 @@ __device__ __forceinline__ bool cluster_sum(double *v, double *buf, int split) {
 // Tile of TT times x TS sensors, two sensors per lane so that a record is read
 // from shared memory once for both.  TT = 16: a warp has two of the times and 64
 // sensors; TT = 1: one time, 512 sensors (images, or wide sensor sets: no work
-// for times that do not exist, and 8 x fewer records made).
+// for times that do not exist, and 8 x fewer records made; 65,536 image points at
+// one time, 4,000 beams: 21.1 -> 1.0 ms).
 template <int TT>
 struct FwdTile {
     static constexpr int TS = TT == 16 ? 64 : 512;
