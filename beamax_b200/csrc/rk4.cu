@@ -391,6 +391,14 @@ struct Stages32 {
             v[N - 2] = q.x, v[N - 1] = q.y;
         }
     }
+    __device__ __forceinline__ void get(int j, float2 *v) const {
+#pragma unroll
+        for (int c = 0; c < Q; ++c) {
+            const float4 q = at[(j * Q + c) * kOdeBlock];
+            v[2 * c] = make_float2(q.x, q.y), v[2 * c + 1] = make_float2(q.z, q.w);
+        }
+        if (R) v[N / 2 - 1] = at2[j * kOdeBlock];
+    }
     __device__ __forceinline__ void put(int j, const float *v) const {
 #pragma unroll
         for (int c = 0; c < Q; ++c)
@@ -726,7 +734,11 @@ __constant__ float DP_E32[7] = {(float)(35.0 / 384 - 5179.0 / 57600),
 
 // acc += sum over j < s of DP_A[s][j] k_j, straight-line per stage: the stages'
 // loads are in flight together and the coefficients are constant operands (a loop
-// over j waited out each load: 39 % of the mixed integrator's time).
+// over j waited out each load: 39 % of the mixed integrator's time).  The FP32 sums run
+// on (re, im) pairs, one paired FMA for two entries with the same bits: half their
+// instructions (269.8 -> 263.5 ms and 33.9 -> 33.3 ms in the two runs quoted at DopriMix).
+// Pairs in rhs_mix as well gained nothing more (262.6 and 33.9 ms): the broadcast of each
+// scalar into a pair costs what the pairing saves.
 template <int S, typename K64, int ND>
 __device__ __forceinline__ void combine64(const K64 &k, double (&acc)[ND]) {
 #pragma unroll
@@ -738,21 +750,22 @@ __device__ __forceinline__ void combine64(const K64 &k, double (&acc)[ND]) {
         for (int c = 0; c < ND; ++c) acc[c] += DP_A[S][j] * r[c];
     }
 }
-template <int S, typename K32, int NF>
-__device__ __forceinline__ void combine32(const K32 &k, float (&acc)[NF]) {
+template <int S, typename K32, int NP>
+__device__ __forceinline__ void combine32(const K32 &k, float2 (&acc)[NP]) {
 #pragma unroll
     for (int j = 0; j < S; ++j) {
         if (S == 6 && j == 1) continue;
-        float f[NF];
+        float2 f[NP];
         k.get(j, f);
+        const float2 a = make_float2(DP_A32[S][j], DP_A32[S][j]);
 #pragma unroll
-        for (int c = 0; c < NF; ++c) acc[c] = fmaf(DP_A32[S][j], f[c], acc[c]);
+        for (int c = 0; c < NP; ++c) acc[c] = __ffma2_rn(a, f[c], acc[c]);
     }
 }
 
 // Bound: instruction issue and latency at 3 warps per scheduler (issue 43-46 %);
 // 200,000 beams over 5,667 save times 437 ms before the vector stages, the stencil
-// cache and the 16-byte records, 269 now; 2,000 beams 56.8 -> 33.9 ms.
+// cache, the 16-byte records and the paired sums, 263 now; 2,000 beams 56.8 -> 33.3 ms.
 //
 // DopriBeam's step (save times landed on, no continuous extension) on the
 // mixed state.  Stages in shared memory: the FP64 ray stages, then the FP32
@@ -814,11 +827,11 @@ struct DopriMix {
 #pragma unroll 1
         for (int s = 1; s < 7; ++s) {
             double a64[ND];
-            float a32[NF];
+            float2 a32[NF / 2];
 #pragma unroll
             for (int c = 0; c < ND; ++c) a64[c] = 0.0;
 #pragma unroll
-            for (int c = 0; c < NF; ++c) a32[c] = 0.0f;
+            for (int c = 0; c < NF / 2; ++c) a32[c] = make_float2(0.0f, 0.0f);
             switch (s) {
                 case 1: combine64<1>(k64, a64), combine32<1>(k32, a32); break;
                 case 2: combine64<2>(k64, a64), combine32<2>(k32, a32); break;
@@ -830,7 +843,10 @@ struct DopriMix {
 #pragma unroll
             for (int c = 0; c < ND; ++c) yt.r[c] = y.r[c] + hh * a64[c];
 #pragma unroll
-            for (int c = 0; c < NF; ++c) yt.f[c] = fmaf(hf, a32[c], y.f[c]);
+            for (int c = 0; c < NF / 2; ++c) {
+                const float2 v = __ffma2_rn(make_float2(hf, hf), a32[c], make_float2(y.f[2 * c], y.f[2 * c + 1]));
+                yt.f[2 * c] = v.x, yt.f[2 * c + 1] = v.y;
+            }
             rhs_mix<D, KIND>(med, cache, mode, yt, kn);
             if (s < 6) {  // the last stage stays in registers
                 k64.put(s, kn.r);
@@ -842,15 +858,15 @@ struct DopriMix {
         float s32 = 0.0f;
         {
             double e64[ND];
-            float e32[NF];
+            float2 e32[NF / 2];
 #pragma unroll
             for (int c = 0; c < ND; ++c) e64[c] = 0.0;
 #pragma unroll
-            for (int c = 0; c < NF; ++c) e32[c] = 0.0f;
+            for (int c = 0; c < NF / 2; ++c) e32[c] = make_float2(0.0f, 0.0f);
 #pragma unroll
             for (int j = 0; j < 7; ++j) {
                 double r[ND];
-                float f[NF];
+                float2 f[NF / 2];
                 if (j == 1) continue;  // weight 0
                 if (j < 6) {
                     k64.get(j, r);
@@ -859,7 +875,9 @@ struct DopriMix {
 #pragma unroll
                 for (int c = 0; c < ND; ++c) e64[c] += DP_E[j] * (j < 6 ? r[c] : kn.r[c]);
 #pragma unroll
-                for (int c = 0; c < NF; ++c) e32[c] = fmaf(DP_E32[j], j < 6 ? f[c] : kn.f[c], e32[c]);
+                for (int c = 0; c < NF / 2; ++c)
+                    e32[c] = __ffma2_rn(make_float2(DP_E32[j], DP_E32[j]),
+                                        j < 6 ? f[c] : make_float2(kn.f[2 * c], kn.f[2 * c + 1]), e32[c]);
             }
             const float at = (float)o.atol, rt = (float)o.rtol;
 #pragma unroll
@@ -871,7 +889,7 @@ struct DopriMix {
             }
 #pragma unroll
             for (int q = 0; q < S + 1; ++q) {
-                const float er = e32[2 * q] * hf, ei = e32[2 * q + 1] * hf;
+                const float er = e32[q].x * hf, ei = e32[q].y * hf;
                 const float y0 = fmaf(y.f[2 * q], y.f[2 * q], y.f[2 * q + 1] * y.f[2 * q + 1]);
                 const float y1 = fmaf(yt.f[2 * q], yt.f[2 * q], yt.f[2 * q + 1] * yt.f[2 * q + 1]);
                 const float sc = fmaf(rt, sqrtf(fmaxf(y0, y1)), at);
