@@ -640,6 +640,7 @@ struct TrajSrc {
     const BeamTime<D> *pool;  // compact: (blocks, TT)
     const float *pool_cull;   // compact: (blocks, 2D + 1)
     float *state;             // (2, nt, ns) Kahan sum / compensation, sorted sensor order
+    const uint32_t *limits;   // (n_tt, nb): see traj_limits_kernel; nullptr: refine is not run
     int first, last;
 };
 
@@ -1021,23 +1022,158 @@ __device__ __forceinline__ int scan_counts(const int *cnt, int row, int warp, in
     return __shfl_sync(0xffffffffu, x - v, row * NW + warp);
 }
 
+// What four of a tile's records say about all of them.  Segment s of a (time tile,
+// beam) is its times 8 s .. 8 s + 7, its sample the time segment_sample(s).  With P the
+// sample's w/2 Im M, rho the smallest eigenvalue of P^-1 P_t over the segment's times t
+// and way the largest distance, in the norm of P, of a centre from the sample's,
+//   sqrt(chi_t(y)) >= sqrt(rho) (sqrt(chi(y)) - way)  for every t and sensor y,
+// chi being the sample's exponent: a sensor where sqrt(chi) exceeds
+// root = sqrt(thr / rho) + way is beyond thr at all of the segment's times.  Byte s of
+// limits[tt][b] is that root, rounded up, in steps of sqrt(thr) / kLimitSteps above
+// sqrt(thr); 255: none is known (P or some P_t not positive definite or not finite, or
+// the beam changes too much), and the beam stays.
+constexpr int kLimitSteps = 32;
+constexpr int kNoLimit = 255;
+__device__ __forceinline__ int segment_sample(int s, int t_cnt) { return min(8 * s + 4, t_cnt - 1); }
+
+// A lower bound on the smallest eigenvalue of P^-1 Q (at most 0 or NaN when none is
+// known), for symmetric P (positive definite where the result is positive) and Q.
+template <int D>
+__device__ __forceinline__ float pencil_min(const double *P, const double *Q) {
+    if (D == 1) return P[0] > 0.0 ? 0.99999f * (float)(Q[0] / P[0]) : 0.0f;
+    if (D == 2) {
+        // the smaller root of x^2 - T x + det Q / det P, T = tr(adj(P) Q) / det P: FP64
+        // where thin beams' determinants cancel, then FP32 with the discriminant
+        // raised by more than its rounding (all in FP64 took 11 ms for 200,000 beams
+        // over 5,667 save times, a third of it in sqrt and divisions)
+        const double a = P[0], b = P[1 % Sym<D>::S], d = P[2 % Sym<D>::S];
+        const double q = Q[0], r = Q[1 % Sym<D>::S], u = Q[2 % Sym<D>::S];
+        const double det = fma(a, d, -b * b);
+        if (!(a > 0.0 && det > 0.0)) return 0.0f;
+        const double inv = 1.0 / det;
+        const float T = (float)((fma(d, q, a * u) - 2.0 * b * r) * inv), N = (float)(fma(q, u, -r * r) * inv);
+        const float disc = fmaxf(0.0f, fmaf(T, T, -4.0f * N)) + 1e-6f * T * T;
+        return T > 0.0f ? 0.99999f * __fdividef(2.0f * N, T + sqrtf(disc)) : 0.0f;
+    }
+    // 1 - |L^-1 (Q - P) L^-T|_F with P = L L^T; the norm's square is tr (P^-1 (Q - P))^2
+    auto at = [](const double *M, int i, int k) { return M[i <= k ? sym_index<D>(i, k) : sym_index<D>(k, i)]; };
+    double adj[D][D], det = 0.0;
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            const int i1 = (i + 1) % D, i2 = (i + 2) % D, k1 = (k + 1) % D, k2 = (k + 2) % D;
+            adj[i][k] = at(P, k1, i1) * at(P, k2, i2) - at(P, k1, i2) * at(P, k2, i1);
+        }
+#pragma unroll
+    for (int k = 0; k < D; ++k) det = fma(at(P, 0, k), adj[k][0], det);
+    // leading minors: P00, adj[2][2] = P00 P11 - P01^2, det
+    if (!(P[0] > 0.0 && adj[D - 1][D - 1] > 0.0 && det > 0.0)) return 0.0;
+    double G[D][D], f = 0.0;
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            G[i][k] = 0.0;
+#pragma unroll
+            for (int l = 0; l < D; ++l) G[i][k] = fma(adj[i][l], at(Q, l, k) - at(P, l, k), G[i][k]);
+        }
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int k = 0; k < D; ++k) f = fma(G[i][k], G[k][i], f);
+    return 0.99999f * (1.0f - 1.00001f * (float)(sqrt(fmax(0.0, f)) / det));
+}
+
+// A warp takes `per` (at most 32) consecutive (time tile, beam) pairs, then those of
+// them that are stored one at a time, lane = time: every record is read once.  32 pairs
+// share the index division and the look at the slots; few pairs are spread over the
+// GPU instead (2,000 beams over 700 times: 42 us with 32 a warp).
+// Bound: HBM, and the instructions of the pencils: 200,000 beams over 5,667 times (a
+// third of the tiles stored, 26 GB) 6.4 ms; a pair per warp with FP64 roots 11.0.
+// (This and the four samples replace a test of four records alone, which assumed how
+// a beam changes between them.  Testing all 32 of each candidate's records in refine
+// instead made the summation 247 and 226 ms where it is 185 and 166, no better than
+// without refine, 259 and 233.)
+template <int D>
+__global__ void __launch_bounds__(THREADS) traj_limits_kernel(TrajSrc<D> T, int64_t nt, float thr, int per,
+                                                              uint32_t *limits) {
+    constexpr int S = Sym<D>::S;
+    const int lane = threadIdx.x & 31;
+    const int64_t n = (nt + TT - 1) / TT * T.nb, stride = (int64_t)gridDim.x * NW * per;
+    for (int64_t i0 = (blockIdx.x * (int64_t)NW + (threadIdx.x >> 5)) * per; i0 < n; i0 += stride) {
+        const int64_t mine = min(i0 + lane, n - 1), tt_lane = mine / T.nb;
+        const int32_t blk_lane = T.pool ? T.slot[mine] : 0;
+        const unsigned live = __ballot_sync(0xffffffffu, lane < per && i0 + lane < n && blk_lane >= 0);
+        unsigned word_lane = 0;
+        for (unsigned left = live; left;) {
+            const int l = take_bit(left);
+            const int64_t tt = __shfl_sync(0xffffffffu, tt_lane, l), b = i0 + l - tt * T.nb;
+            const int32_t blk = __shfl_sync(0xffffffffu, blk_lane, l);
+            const int t_cnt = (int)min((int64_t)TT, nt - tt * TT), t = min(lane, t_cnt - 1);
+            const BeamTime<D> *bt = T.pool ? T.pool + ((int64_t)blk * TT + t) : T.rec + ((tt * TT + t) * T.nb + b);
+            const int at = segment_sample(lane >> 3, t_cnt);
+            float q[S], p[S], dx[D], mag = 0.0f;  // this record's form, the sample's (off-diagonals doubled)
+            double Q[S], P[S];
+#pragma unroll
+            for (int e = 0; e < S; ++e) q[e] = bt->p[e];
+#pragma unroll
+            for (int e = 0; e < S; ++e) p[e] = __shfl_sync(0xffffffffu, q[e], at);
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+#pragma unroll
+                for (int k = a; k < D; ++k) {
+                    const int e = sym_index<D>(a, k);
+                    Q[e] = (a == k ? 1.0 : 0.5) * (double)q[e];
+                    P[e] = (a == k ? 1.0 : 0.5) * (double)p[e];
+                }
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                const double x = bt->x[a];
+                dx[a] = (float)(x - __shfl_sync(0xffffffffu, x, at));
+            }
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+#pragma unroll
+                for (int k = a; k < D; ++k) mag = fmaf(fabsf(p[sym_index<D>(a, k)]), fabsf(dx[a] * dx[k]), mag);
+            // (the quadratic form's rounding is below 1e-6 of its terms' magnitudes)
+            float rho = pencil_min<D>(P, Q);
+            const float way = quad<D>(p, dx) + 1e-6f * mag;
+            float w = sqrtf(fmaxf(way, 0.0f)) * 1.00001f;
+            // a value that is not a number is not a limit
+            bool known = rho > 0.0f && way < 1e30f;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                rho = fminf(rho, __shfl_xor_sync(0xffffffffu, rho, o));
+                w = fmaxf(w, __shfl_xor_sync(0xffffffffu, w, o));
+                known = __shfl_xor_sync(0xffffffffu, (int)known, o) != 0 && known;
+            }
+            const float c = ceilf((rsqrtf(rho) * 1.00001f + w * rsqrtf(thr) * 1.00001f - 1.0f) * (float)kLimitSteps);
+            const unsigned code = known && c < (float)kNoLimit ? (unsigned)fmaxf(c, 0.0f) : (unsigned)kNoLimit;
+            unsigned word = code << (8 * (lane >> 3));
+            word |= __shfl_xor_sync(0xffffffffu, word, 8);
+            word |= __shfl_xor_sync(0xffffffffu, word, 16);
+            if (lane == l) word_lane = word;
+        }
+        if (live >> lane & 1u) limits[mine] = word_lane;
+    }
+}
+
 // Trajectory candidates surv[old .. nq) (kept by the tile test) against the groups
-// of the tile, from 4 of their tile's 32 times: the tile test's isotropic bound
-// keeps 2 to 3 candidates for each that reaches the tile (live: 34 % at 1024^2
-// heterogeneous, 40 % at 128^3), and fetching a dead one's whole record (2 KB in
-// 2D) cost more than half of the summation.  A beam goes if at every sample its
-// exponent exceeds thr widened by the way it moves to half-way between the samples
-// (in the sample's own metric, with a fifth to spare) and by a tenth of the
-// exponent's root for the change of Im M; Im M is smallest at an end of a sampled
-// interval.  Four lanes per candidate; the survivors move to surv[old ..) in
-// order.  Returns the new end.  All threads; ends with a barrier.
+// of the tile, from 4 of their tile's 32 times and their limits: the tile test's
+// isotropic bound keeps 2 to 3 candidates for each that reaches the tile (live: 34 % at
+// 1024^2 heterogeneous, 40 % at 128^3), and fetching a dead one's whole record (2 KB in
+// 2D) cost more than half of the summation.  A candidate goes if no group is within
+// its limit of any of the four samples: the record pass would leave it out at every
+// group.  Four lanes per candidate; the survivors move to surv[old ..) in order.
+// Returns the new end.  All threads; ends with a barrier.
 template <int D, typename BeamOf>
 __device__ __forceinline__ int refine(const TrajSrc<D> &T, int64_t t_first, int t_cnt, const TileInfo<D> &ti,
                                       const TileGroups<D> &tg, float thr, int32_t *surv, int old, int nq, uint8_t *keep,
                                       int *warp_cnt, const BeamOf &beam_of) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, smp = lane & 3;
     const int64_t tt = t_first / TT;
-    const int ts = (t_cnt - 1) * smp / 3;
+    const int ts = segment_sample(smp, t_cnt);
     int out = old;
     for (int base = old; base < nq; base += SCAN * THREADS) {
         const int end = min(nq, base + SCAN * THREADS);
@@ -1047,20 +1183,15 @@ __device__ __forceinline__ int refine(const TrajSrc<D> &T, int64_t t_first, int 
             const int64_t b = beam_of(c);
             const BeamTime<D> *bt =
                 T.pool ? T.pool + ((int64_t)T.slot[tt * T.nb + b] * TT + ts) : T.rec + ((t_first + ts) * T.nb + b);
+            const int code = T.limits[tt * T.nb + b] >> (8 * smp) & 255u;
             Rec<D> r;
 #pragma unroll
             for (int a = 0; a < D; ++a) r.d0[a] = (float)(ti.s0[a] - bt->x[a]);
 #pragma unroll
             for (int q = 0; q < Sym<D>::S; ++q) r.p[q] = bt->p[q];
-            float up[D], dn[D];
-#pragma unroll
-            for (int a = 0; a < D; ++a) {
-                up[a] = __shfl_down_sync(0xffffffffu, r.d0[a], 1, 4) - r.d0[a];
-                dn[a] = __shfl_up_sync(0xffffffffu, r.d0[a], 1, 4) - r.d0[a];
-            }
-            const float way = sqrtf(fmaxf(0.0f, fmaxf(quad<D>(r.p, up), quad<D>(r.p, dn))));
-            const float root = (sqrtf(thr) + 0.6f * way) * (1.0f / 0.9f);
-            const unsigned hit = __ballot_sync(0xffffffffu, reached_mask<D>(r, tg, root * root) != 0);
+            const float up = fmaf((float)code, 1.0f / kLimitSteps, 1.0f);
+            const unsigned hit =
+                __ballot_sync(0xffffffffu, code == kNoLimit || reached_mask<D>(r, tg, thr * up * up) != 0);
             if (smp == 0 && c0 + lane / 4 < end) keep[c0 + lane / 4 - base] = (hit >> lane & 15u) ? 1 : 0;
         }
         __syncthreads();
@@ -1266,7 +1397,7 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
             nq += tot;
             __syncthreads();
             if constexpr (TRAJ && !PERIODIC) {
-                if (thr > 0.0f)
+                if (T.limits)
                     nq = refine<D>(T, t_first, t_cnt, ti, ginfo, thr, surv, old, nq, keep, warp_cnt,
                                    [&](int c) { return (int64_t)surv[c]; });
             }
@@ -1496,7 +1627,7 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
             if (tid == 0) find_lattice<D>(ginfo);
             __syncthreads();  // ginfo, surv
             if constexpr (TRAJ && !PERIODIC) {
-                if (thr > 0.0f) {
+                if (T.limits) {
                     nq = refine<D>(T, t_first, t_cnt, ti, ginfo, thr, surv, 0, nq, keep, warp_cnt,
                                    [&](int c) { return r0 + surv[c]; });
                     if (nq == 0) continue;
@@ -1743,6 +1874,12 @@ Split make_split(const msgb_problem *p, int64_t n_tiles, int64_t nbeam, char *at
     return Split{(int)n, len, n > 1 ? (float2 *)at : nullptr};
 }
 
+// Limits of a trajectory chunk of nb beams (refine).  They follow everything else in a
+// workspace sized by msgb_sum_f32_traj_workspace_size; a smaller one goes without.
+size_t traj_limit_bytes(const msgb_problem *p, int64_t nb) {
+    return align256((size_t)((p->nt + TT - 1) / TT) * (size_t)(nb > 0 ? nb : 0) * sizeof(uint32_t));
+}
+
 // Adjoint partials of a trajectory chunk of nb beams: (n_tt, nb) complex FP64.
 size_t traj_part_bytes(const msgb_problem *p, int64_t nb) {
     return align256((size_t)((p->nt + TT - 1) / TT) * (size_t)(nb > 0 ? nb : 0) * 16);
@@ -1819,6 +1956,25 @@ int sm_count() {
     return n;
 }
 
+// The limits of T's records at `at`, where cutoff, domain and the `spare` bytes there
+// allow; returns the bytes taken.
+template <int D>
+size_t prepare_limits(const msgb_problem *p, const msgb_sum_opts *o, TrajSrc<D> &T, char *at, size_t spare,
+                      cudaStream_t st) {
+    const size_t bytes = traj_limit_bytes(p, T.nb);
+    const float cutoff = o ? (float)o->cutoff : 0.0f;
+    for (int i = 0; i < D; ++i)
+        if (p->periodic[i]) return 0;
+    if (!(cutoff > 0.0f) || T.nb == 0 || spare < bytes) return 0;
+    const int64_t items = (p->nt + TT - 1) / TT * T.nb, want = 8LL * sm_count(), share = items / (want * NW);
+    const int per = (int)(share < 1 ? 1 : (share > 32 ? 32 : share));
+    const int64_t need = (items + (int64_t)per * NW - 1) / ((int64_t)per * NW);
+    traj_limits_kernel<D><<<(unsigned)(want < need ? want : need), THREADS, 0, st>>>(
+        T, p->nt, cutoff + kGroupMarginEfolds, per, (uint32_t *)at);
+    T.limits = (const uint32_t *)at;
+    return bytes;
+}
+
 template <int D, bool TRAJ>
 int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, char *ws, const Layout &l,
             size_t ws_used, size_t ws_bytes, float *out, cudaStream_t st, TrajSrc<D> T) {
@@ -1839,6 +1995,9 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     if (!TRAJ) {
         hom = prepare_hom<D>(p, b, ws + at, spare, st);
         if (hom) at += hom_bytes(D, b->n), spare -= hom_bytes(D, b->n);
+    } else {
+        const size_t taken = prepare_limits<D>(p, o, T, ws + at, spare, st);
+        at += taken, spare -= taken;
     }
     const Split sp = make_split(p, n_st * n_tt, TRAJ ? T.nb : b->n, ws + at, spare);
     if (n_st * n_tt * sp.n > 0x7fffffffLL) return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: too many tiles");
@@ -1872,7 +2031,7 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
 
 template <int D, bool TRAJ>
 int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, char *ws, const Layout &l,
-            size_t ws_bytes, const float *data, double *part, double *g, cudaStream_t st, TrajSrc<D> T) {
+            size_t ws_used, size_t ws_bytes, const float *data, double *part, double *g, cudaStream_t st, TrajSrc<D> T) {
     msgb_beam_set none{};
     if (int e = prep<D>(p, TRAJ ? &none : b, o, l, ws, st)) return e;
     dim3 tg((unsigned)((p->ns + 31) / 32), (unsigned)((p->nt + 31) / 32));
@@ -1897,7 +2056,8 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     const int64_t want = 2LL * sm_count();
     const unsigned grid = (unsigned)(want < n_items ? want : n_items);
     constexpr size_t smem = (size_t)AdjRange<D, TRAJ>::NACC * 2 * sizeof(double) + rec_bytes<D>();
-    const HomBeam<D> *hom = TRAJ ? nullptr : prepare_hom<D>(p, b, ws + l.total, ws_bytes - l.total, st);
+    const HomBeam<D> *hom = TRAJ ? nullptr : prepare_hom<D>(p, b, ws + ws_used, ws_bytes - ws_used, st);
+    if (TRAJ) prepare_limits<D>(p, o, T, ws + ws_used, ws_bytes - ws_used, st);
     auto args = [&](auto kern) {
         // static + dynamic shared memory exceed the default 48 KB: opt in
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1998,11 +2158,11 @@ extern "C" int msgb_adj_gather_f32(const msgb_problem *prob, const msgb_beam_set
     cudaStream_t st = as_stream(stream);
     char *ws = (char *)workspace;
     switch (prob->ndim) {
-        case 1: return run_adj<1, false>(prob, beams, opts, ws, l, workspace_bytes, data, (double *)(ws + l.part), g, st,
+        case 1: return run_adj<1, false>(prob, beams, opts, ws, l, l.total, workspace_bytes, data, (double *)(ws + l.part), g, st,
                                          traj_src<1>(nullptr, nullptr, 1, 1));
-        case 2: return run_adj<2, false>(prob, beams, opts, ws, l, workspace_bytes, data, (double *)(ws + l.part), g, st,
+        case 2: return run_adj<2, false>(prob, beams, opts, ws, l, l.total, workspace_bytes, data, (double *)(ws + l.part), g, st,
                                          traj_src<2>(nullptr, nullptr, 1, 1));
-        default: return run_adj<3, false>(prob, beams, opts, ws, l, workspace_bytes, data, (double *)(ws + l.part), g, st,
+        default: return run_adj<3, false>(prob, beams, opts, ws, l, l.total, workspace_bytes, data, (double *)(ws + l.part), g, st,
                                           traj_src<3>(nullptr, nullptr, 1, 1));
     }
 }
@@ -2015,9 +2175,10 @@ static size_t traj_state_bytes(const msgb_problem *p) { return align256((size_t)
 extern "C" size_t msgb_sum_f32_traj_workspace_size(const msgb_problem *prob, int64_t nb_max) {
     if (validate_problem(prob) || nb_max < 0) return 0;
     const Layout l = layout(prob, 0, true, (prob->ns + GS - 1) / GS);
-    // after the Kahan state: the adjoint's partials, or those of the split forward
+    // after the Kahan state: the adjoint's partials, or those of the split forward, and
+    // the limits
     const size_t part = traj_part_bytes(prob, nb_max), split = split_bytes(prob, int64_t(1) << 62);
-    return l.total + traj_state_bytes(prob) + (part > split ? part : split);
+    return l.total + traj_state_bytes(prob) + (part > split ? part : split) + traj_limit_bytes(prob, nb_max);
 }
 
 // with_part: the adjoint's partials (n_tt, nb) follow the Kahan state.
@@ -2076,10 +2237,11 @@ extern "C" int msgb_adj_gather_f32_traj(const msgb_problem *prob, const msgb_bea
     cudaStream_t st = as_stream(stream);
     char *ws = (char *)workspace;
     double *part = (double *)(ws + traj_state_offset(l) + traj_state_bytes(prob));
+    const size_t used = traj_state_offset(l) + traj_state_bytes(prob) + traj_part_bytes(prob, traj->nb);
     switch (prob->ndim) {
-        case 1: return run_adj<1, true>(prob, beams, opts, ws, l, workspace_bytes, data, part, g, st, traj_src<1>(traj, nullptr, 1, 1));
-        case 2: return run_adj<2, true>(prob, beams, opts, ws, l, workspace_bytes, data, part, g, st, traj_src<2>(traj, nullptr, 1, 1));
-        default: return run_adj<3, true>(prob, beams, opts, ws, l, workspace_bytes, data, part, g, st, traj_src<3>(traj, nullptr, 1, 1));
+        case 1: return run_adj<1, true>(prob, beams, opts, ws, l, used, workspace_bytes, data, part, g, st, traj_src<1>(traj, nullptr, 1, 1));
+        case 2: return run_adj<2, true>(prob, beams, opts, ws, l, used, workspace_bytes, data, part, g, st, traj_src<2>(traj, nullptr, 1, 1));
+        default: return run_adj<3, true>(prob, beams, opts, ws, l, used, workspace_bytes, data, part, g, st, traj_src<3>(traj, nullptr, 1, 1));
     }
 }
 

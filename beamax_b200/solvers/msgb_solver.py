@@ -210,6 +210,7 @@ class MSGBSolver:
         # fraction of (time tile, beam) pairs the compact store keeps; None: not seen yet
         self._live_est: Optional[float] = None
         self._compact_kept = None
+        self._compact_widest = 0  # beams of the widest chunk of the integration under way
         # (b_first, nb, pool blocks, blocks taken) of the last 256 compact integrations
         self.compact_log = collections.deque(maxlen=256)
         # When set to a list, every FP32 summation entry point call appends
@@ -647,6 +648,7 @@ class MSGBSolver:
                     todo = [(x, min(widest, b0 + n0 - x)) for b0, n0 in todo for x in range(b0, b0 + n0, widest)]
                     size = int(widest * n_tt * (4 + est * (block + cull))
                                + min(widest, lanes) * (block + cull) + 4096)
+        self._compact_widest = widest
         boxes, n_boxes = self._live_boxes(pr, opts, domain, sensors, dev, st)
         first = True
         opts_ode = self._ode_opts(None)
@@ -673,6 +675,28 @@ class MSGBSolver:
                 self._compact_kept = buf
             yield tr, first, not todo
             first = False
+
+    @staticmethod
+    def _limit_bytes(nt: int, nb: int) -> int:
+        """The part of a trajectory sum's workspace that it can do without (slower):
+        the limits of nb beams' time tiles, 4 bytes each."""
+        return ((nt + 31) // 32 * nb * 4 + 255) // 256 * 256
+
+    @staticmethod
+    def _traj_workspace(dev, least: int, limits: int):
+        """(workspace, bytes) of least + limits bytes, or least where memory is short."""
+        import torch
+
+        try:
+            return workspace(dev, "sum32traj", least + limits), least + limits
+        except torch.OutOfMemoryError:
+            return workspace(dev, "sum32traj", least), least
+
+    def _chunk_workspace(self, pr, nb: int, dev):
+        """The workspace of a trajectory sum over chunks of at most nb beams."""
+        limits = self._limit_bytes(pr.nt, nb)
+        full = int(_lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), nb))
+        return self._traj_workspace(dev, full - limits, limits)
 
     def _begin_trajectories(self, domain, ts):
         self._accepted = None
@@ -743,11 +767,14 @@ class MSGBSolver:
             keep_last = self.keep_trajectories and self._traj_owner is not None
             self._compact_kept = None
             # the forward keeps its Kahan state in this workspace from the first
-            # chunk to the last: one size (no per-chunk partials), never regrown
+            # chunk to the last: one size (no per-chunk partials, the limits of the
+            # widest chunk), never regrown after the first
             nbytes = _lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), 0)
             ws = workspace(dev, "sum32traj", nbytes)
             for tr, first, last in self._compact_integrate(pr, med, bs, lo, hi, domain, sensors, opts, dev, st,
                                                           status, keep=keep_last):
+                if first:
+                    ws, nbytes = self._traj_workspace(dev, nbytes, self._limit_bytes(pr.nt, self._compact_widest))
                 with self._kernel_span("msgb_sum_fwd_f32_traj", cnt):
                     _lib.check(_lib.lib().msgb_sum_fwd_f32_traj(_lib.ref(pr), _lib.ref(bs), _lib.ref(tr),
                                                                 _lib.ref(opts), int(first), int(last), ws.data_ptr(),
@@ -757,8 +784,7 @@ class MSGBSolver:
             self._remember_trajectories(self._compact_kept, tr, domain, ts, pr.nt)
             self._compact_kept = None
             return out
-        nbytes = _lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), max(nb for _, nb in chunks))
-        ws = workspace(dev, "sum32traj", nbytes)
+        ws, nbytes = self._chunk_workspace(pr, max(nb for _, nb in chunks), dev)
         for i, (b_first, nb) in enumerate(chunks):
             tr, buf = self._trajectories(pr, med, bs, b_first, nb, False, per, n_tt, dev, st, status,
                                          keep_buf if i == last else None)
@@ -843,8 +869,7 @@ class MSGBSolver:
                             tiling=_lib.ref(tiling[0]) if tiling else None)
         nbytes, ws = 0, None
         if not fp64 and not self._compact():
-            nbytes = _lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), max(nb for _, nb in chunks))
-            ws = workspace(dev, "sum32traj", nbytes)
+            ws, nbytes = self._chunk_workspace(pr, max(nb for _, nb in chunks), dev)
         status = torch.zeros(2 * n, dtype=torch.int32, device=dev)
         self._begin_trajectories(domain, ts)
         kept = (cached["tr"].b_first, cached["tr"].nb) if cached is not None else None
@@ -857,8 +882,7 @@ class MSGBSolver:
                 kept = None
             gen = self._compact_integrate(pr, med, bs, lo, hi, domain, sensors, opts, dev, st, status, skip=kept)
             for tr in _chain(trs, (t for t, _, _ in gen)):
-                nbytes = _lib.lib().msgb_sum_f32_traj_workspace_size(_lib.ref(pr), tr.nb)
-                ws = workspace(dev, "sum32traj", nbytes)
+                ws, nbytes = self._chunk_workspace(pr, tr.nb, dev)
                 gp = torch.view_as_real(g_all[tr.b_first:tr.b_first + tr.nb]).data_ptr()
                 with self._kernel_span("msgb_adj_gather_f32_traj", cnt):
                     _lib.check(_lib.lib().msgb_adj_gather_f32_traj(_lib.ref(pr), _lib.ref(bs), _lib.ref(tr),

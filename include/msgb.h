@@ -88,8 +88,9 @@ typedef struct msgb_sensor_tiling {
 typedef struct msgb_sum_opts {
     double cutoff;           /* skip a (beam, tile) pair when the Gaussian exponent
                                 is provably above this many e-folds, and a (beam, 32
-                                times, 16 sensors) block of the tile beyond 4 more
-                                (<= 0: dense) */
+                                times, 16 sensors) block of the tile where it is
+                                provably above 4 more (<= 0: dense).  A beam whose
+                                exponent is not a number is never skipped for it */
     unsigned long long *eval_count; /* optional device counter: evaluated
                                 (beam, t, sensor) triples are added to it */
     const msgb_sensor_tiling *tiling; /* optional (NULL) */
@@ -276,7 +277,10 @@ int msgb_rk4_trajectories(const msgb_problem *prob, const msgb_medium *med, cons
  * amplitude of beam b is a0[b mod n] times the trajectory's A.
  * FP64: dense, accumulates (+=) into out (nt, ns) FP64, which the caller
  * zeroes before the first chunk.
- * FP32: culled by the trajectory's boxes; Kahan state (2 nt ns floats) lives in
+ * FP32: culled by the trajectory's boxes and, before the records are made, by
+ * limits that each call forms from the records in its workspace (4 bytes per
+ * time tile and beam; a workspace without room for them gives the same sums
+ * slower); Kahan state (2 nt ns floats) lives in
  * the workspace from the call with first_chunk != 0 to the call with
  * last_chunk != 0, which writes out (nt, ns) FP32.  All chunks of one
  * summation must use the same workspace and problem. */

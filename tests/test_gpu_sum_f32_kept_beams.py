@@ -5,7 +5,9 @@ provably beyond the cutoff.
 Not finite: a NaN in a beam's centre, momentum or Hessian reaches every output of
 the forward and the beam's own entry of the transpose, as in the FP64 sums.
 Growing: an indefinite Im M, whose exponent along a row of sensors is concave, in
-the closed form and in trajectory records with an open culling box.
+the closed form and in trajectory records with an open culling box.  Varying:
+records that come near a sensor at a few times of a tile only, or whose centre and
+Hessian jump from time to time.
 
 Tolerances: 3e-5 rel-L2 of the FP64 value, as for every FP32 sum (at most 15^2 / 2
 roundings of 2^-24 in a run's ratio, plus the seed's); the trajectory cases also
@@ -118,32 +120,46 @@ def test_a_growing_beam_is_in_every_group_of_sensors(kind):
 
 
 # ---- trajectory records --------------------------------------------------------
-REC = np.dtype([("x", "f8", 2), ("wp", "f8", 2), ("q", "f4", 3), ("p", "f4", 3), ("ang", "f4"), ("amp", "f4")])
+PAIRS = {2: [(0, 0), (0, 1), (1, 1)], 3: [(0, 0), (0, 1), (0, 2), (1, 1), (1, 2), (2, 2)]}
+
+
+def _rec(d):
+    S = len(PAIRS[d])
+    return np.dtype([("x", "f8", d), ("wp", "f8", d), ("q", "f4", S), ("p", "f4", S), ("ang", "f4"), ("amp", "f4")])
+
+
+def _matrix(p, d):
+    """Packed coefficients (off-diagonals doubled) -> symmetric matrices."""
+    M = np.zeros(p.shape[:-1] + (d, d))
+    for e, (i, k) in enumerate(PAIRS[d]):
+        M[..., i, k] = M[..., k, i] = p[..., e] * (1.0 if i == k else 0.5)
+    return M
 
 
 class _Records:
-    """Records of nb beams at nt times (REC), their boxes, and the sums over them."""
+    """Records of nb beams at nt times, their boxes, and the sums over them."""
 
     def __init__(self, rec, open_box, pos, cutoff=16.0):
         from beamax_b200 import _lib
 
         self.dev = _dev()
-        self.rec, self.pos = rec, pos
+        self.rec, self.d = rec, rec["x"].shape[-1]
+        d = self.d
+        self.pos = pos = np.concatenate([pos, np.full((len(pos), d - 2), 40 * DX)], 1)
         nt, nb = rec.shape
         n_tt = (nt + 31) // 32
-        box = np.zeros((n_tt, nb, 5), np.float32)
+        box = np.zeros((n_tt, nb, 2 * d + 1), np.float32)
         for t in range(n_tt):
             r = rec[32 * t:32 * t + 32]
-            P = np.stack([r["p"][..., 0], r["p"][..., 1] / 2, r["p"][..., 1] / 2, r["p"][..., 2]], -1)
-            lam = np.linalg.eigvalsh(P.reshape(P.shape[:-1] + (2, 2)).astype(np.float64)).min(-1).min(0)
-            box[t, :, 0:2], box[t, :, 2:4] = r["x"].min(0), r["x"].max(0)
-            box[t, :, 4] = np.maximum(lam * (1 - 1e-6), 0)
-        box[:, open_box, 0:2], box[:, open_box, 2:4], box[:, open_box, 4] = -3.4e38, 3.4e38, 0
+            lam = np.linalg.eigvalsh(_matrix(r["p"], d)).min(-1).min(0)
+            box[t, :, :d], box[t, :, d:2 * d] = r["x"].min(0), r["x"].max(0)
+            box[t, :, 2 * d] = np.maximum(lam * (1 - 1e-6), 0)
+        box[:, open_box, :d], box[:, open_box, d:2 * d], box[:, open_box, 2 * d] = -3.4e38, 3.4e38, 0
         up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(self.dev)
         self.d_rec = up(rec.view(np.uint8))
         self.d_box = up(box)
         # the compact form: one block of 32 records per (tile, beam)
-        pool = np.zeros((n_tt, nb, 32), REC)
+        pool = np.zeros((n_tt, nb, 32), rec.dtype)
         for t in range(n_tt):
             r = rec[32 * t:32 * t + 32]
             pool[t, :, :len(r)] = r.T
@@ -151,12 +167,12 @@ class _Records:
         self.ts, self.d_pos = up(np.arange(nt) * 1e-8), up(pos)
         n = (nb + 1) // 2
         self.one = up(np.tile([1.0, 0.0], n))
-        z = up(np.ones((n, 4)))
-        self.keep = (z,)
-        self.bs = _lib.BeamSet(n=n, x0=z.data_ptr(), p0=z.data_ptr(), alpha=z.data_ptr(), a0=self.one.data_ptr(),
-                               omega=z.data_ptr(), modes=0)
-        self.pr = _lib.Problem(ndim=2, c=1500.0, nt=nt, ts=self.ts.data_ptr(), ns=len(pos), sensors=self.d_pos.data_ptr())
-        self.pr.L[0] = self.pr.L[1] = N * DX
+        self.z = up(np.ones((n, 2 * d)))
+        z = self.z.data_ptr()
+        self.bs = _lib.BeamSet(n=n, x0=z, p0=z, alpha=z, a0=self.one.data_ptr(), omega=z, modes=0)
+        self.pr = _lib.Problem(ndim=d, c=1500.0, nt=nt, ts=self.ts.data_ptr(), ns=len(pos), sensors=self.d_pos.data_ptr())
+        for a in range(3):
+            self.pr.L[a] = N * DX
         self.opts = _lib.SumOpts(cutoff=cutoff)
         self.nt, self.nb = nt, nb
 
@@ -186,23 +202,29 @@ class _Records:
     def exact(self, data):
         """The same sums in 64 bits."""
         r = self.rec
-        D = self.pos[None, None] - r["x"][:, :, None]  # (nt, nb, ns, 2)
-        dd = np.stack([D[..., 0] ** 2, D[..., 0] * D[..., 1], D[..., 1] ** 2], -1)
+        D = self.pos[None, None] - r["x"][:, :, None]  # (nt, nb, ns, d)
+        dd = np.stack([D[..., i] * D[..., k] for i, k in PAIRS[self.d]], -1)
         th = (r["wp"][:, :, None] * D).sum(-1) + (r["q"][:, :, None].astype(float) * dd).sum(-1) + r["ang"][:, :, None]
         z = r["amp"][:, :, None] * np.exp(1j * th - (r["p"][:, :, None].astype(float) * dd).sum(-1))
         d = data.cpu().numpy().astype(float)
         return z.real.sum(1), (np.conj(z) * d[:, None]).sum((0, 2))
 
 
-def _records(nt, nb, seed=5):
+def _records(nt, nb, d=2, seed=5):
     rng = np.random.default_rng(seed)
-    rec = np.zeros((nt, nb), REC)
-    rec["x"] = np.array([30.0, 47.0]) * DX + DX * rng.random((1, nb, 2))
-    rec["wp"] = rng.standard_normal((1, nb, 2)) * 300
-    rec["q"] = rng.standard_normal((1, nb, 3)) * 1e4
-    rec["p"][..., 0] = rec["p"][..., 2] = 2.0 / (10 * DX) ** 2
+    rec = np.zeros((nt, nb), _rec(d))
+    rec["x"] = np.array([30.0, 47.0, 40.0][:d]) * DX + DX * rng.random((1, nb, d))
+    rec["wp"] = rng.standard_normal((1, nb, d)) * 300
+    rec["q"] = rng.standard_normal((1, nb, len(PAIRS[d]))) * 1e4
+    _round(rec, slice(None), 2.0)
     rec["ang"], rec["amp"] = rng.random((1, nb)), 2.0
     return rec
+
+
+def _round(rec, at, efolds):
+    """Isotropic Hessians: `efolds` at ten grid steps."""
+    for e, (i, k) in enumerate(PAIRS[rec["x"].shape[-1]]):
+        rec["p"][at, :, e] = efolds / (10 * DX) ** 2 if i == k else 0.0
 
 
 def _compare(R, compact):
@@ -212,6 +234,37 @@ def _compare(R, compact):
     out = 1.2e-7 * 2 * R.nb
     assert np.linalg.norm(y - y0) <= TOL * np.linalg.norm(y0) + out * y0.size ** 0.5
     assert np.linalg.norm(g - g0) <= TOL * np.linalg.norm(g0) + 2.4e-7 * float(data.norm()) * (R.nb * y0.size) ** 0.5
+
+
+@pytest.mark.parametrize("compact", [False, True])
+@pytest.mark.parametrize("kind,d", [("line", 2), ("run", 2), ("runs", 2), ("short", 2), ("scattered", 2), ("line", 3)])
+def test_records_that_come_near_at_a_few_times_only(kind, d, compact):
+    """Narrow beams (exponent 200 at the sensors) that are wide (2) at three of a
+    tile's times."""
+    rec = _records(40, 70, d)
+    _round(rec, slice(None), 200.0)
+    for k in (5, 13, 27, 33):
+        _round(rec, k, 2.0)
+    _compare(_Records(rec, np.zeros(70, bool), _positions(kind)), compact)
+
+
+@pytest.mark.parametrize("kind,d", [("line", 2), ("scattered", 2), ("line", 3)])
+@pytest.mark.parametrize("nt", [1, 7, 32, 37])
+@pytest.mark.parametrize("change", [0.02, 0.3, 3.0])
+def test_records_that_change_from_time_to_time(change, nt, kind, d):
+    """Centres that walk and Hessians that turn and stretch, by little and by much,
+    at distances from within the beams to far beyond the cutoff."""
+    rng = np.random.default_rng(int(100 * change) + nt)
+    nb = 300
+    rec = _records(nt, nb, d)
+    rec["x"] = DX * (np.array([0.0, 0.0, 40.0][:d]) + rng.random((1, nb, d)) * [80.0, 200.0, 1e-9][:d])
+    rec["x"] = rec["x"] + DX * 8 * change * rng.standard_normal((nt, nb, d)).cumsum(0)
+    q, _ = np.linalg.qr(rng.standard_normal((1, nb, d, d)) + change * 0.3 * rng.standard_normal((nt, nb, d, d)).cumsum(0))
+    lam = np.exp(rng.normal(0, 1.0, (1, nb, d)) + change * rng.standard_normal((nt, nb, d))) * 4.0 / (10 * DX) ** 2
+    M = np.einsum("tbik,tbk,tbjk->tbij", q, lam, q)
+    for e, (i, k) in enumerate(PAIRS[d]):
+        rec["p"][..., e] = M[..., i, k] * (1 if i == k else 2)
+    _compare(_Records(rec, np.zeros(nb, bool), _positions(kind)), True)
 
 
 @pytest.mark.parametrize("compact", [False, True])
