@@ -1284,8 +1284,8 @@ __global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *p
 // Per item: beams are scanned 1024 at a time against the tile (survives /
 // traj_survives), survivors queue up, and every G of them make a record pass;
 // then each warp evaluates the pass's beams that reach its group, four at a
-// time (two independent paired recurrences; the four values of a sensor are
-// added before one compensated addition).
+// time (two independent paired recurrences; two values of a sensor are added
+// before each compensated addition).
 //
 // Bound: FP32 pipe (recurrence 8 FMA-pipe operations per triple, seed ~75 per 16
 // triples) with the seeds' MUFU work beside it; measured 51 % (2D) and 58 % (3D) of
@@ -1419,9 +1419,9 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                         if (i2 >= 0) direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
                         {
                             // z_{k+1} = z_k f_k, f_{k+1} = f_k q; sensors 2h, 2h + 1
-                            // share a paired compensated addition (one or two beams
-                            // left: the other pair is zero -- a second loop for them
-                            // costs more in instruction fetches than it saves)
+                            // share a paired compensated addition per two beams (one or
+                            // two beams left: the other pair is zero -- a second loop for
+                            // them costs more in instruction fetches than it saves)
 #pragma unroll
                             for (int h = 0; h < GS / 2; ++h) {
                                 if (h > 0) {
@@ -1430,13 +1430,13 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                                     fa = cmul2(fa, qa);
                                     fb = cmul2(fb, qb);
                                 }
-                                const float2 v0 = __fadd2_rn(za.re, zb.re);
+                                const float2 a0 = za.re, b0 = zb.re;
                                 za = cmul2(za, fa);
                                 zb = cmul2(zb, fb);
                                 fa = cmul2(fa, qa);
                                 fb = cmul2(fb, qb);
-                                const float2 v1 = __fadd2_rn(za.re, zb.re);
-                                kahan_add2(acc2[h], cmp2[h], make_float2(v0.x + v0.y, v1.x + v1.y));
+                                kahan_add2(acc2[h], cmp2[h], make_float2(a0.x + a0.y, za.re.x + za.re.y));
+                                if (i2 >= 0) kahan_add2(acc2[h], cmp2[h], make_float2(b0.x + b0.y, zb.re.x + zb.re.y));
                             }
                         }
                         if (!__any_sync(0xffffffffu, direct != 0)) continue;
