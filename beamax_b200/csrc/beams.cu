@@ -55,14 +55,21 @@ __global__ void take_last_kernel(const int32_t *sorted_idx, int64_t total, int64
 // A radix select finds the n-th largest (key, index) -- 13 bits a pass, from the
 // top, each pass one kernel whose last block picks the digit -- then the n pairs at or
 // above it are compacted in index order and only they are sorted: the same list as
-// sorting everything.  1024^2 (4.2 million keys, n = 262,144): 400 us for the full
-// sort, 150 us this way.
+// sorting everything.  4.2 million keys, n = 262,500: 461 us for the full sort, 257
+// this way.
 // A sort of more than a few thousand pairs takes 8 passes of 8 us whatever its size,
-// and the select 7 of 5 us: it pays from about two million keys on, or where the
-// selected fit the sort's single-kernel form (262,144 keys, n = 12,815: 210 us with
-// the transform by selecting, 202 by sorting everything before).
+// and the select 7 of 5 us, all of them where the n-th key is one of many equal ones
+// (zeros); otherwise it is done after three or four.  The line lies where the select
+// loses for no keys.  Selected against sorted, distinct keys and then n-th key zero:
+//   n > 2048   1,048,576 keys, n = 65,536: 211 / 181, 271 / 182 us
+//              2,097,152, 131,072: 229 / 269, 288 / 254
+//              3,000,000, 46,875: 226 / 338, 303 / 310; 1,500,000: 331 / 350, 425 / 351
+//              4,200,000, 700,000: 292 / 466, 377 / 445; 2,100,000: 399 / 469, 515 / 475
+// Up to 2048 selected fit the sort's single-kernel form; there the line is drawn for
+// distinct keys (an n-th key of zero takes an image with fewer than n coefficients):
+//   n <= 2048  65,536, 1000: 85 / 116, 156 / 103; 1,048,576, 2048: 90 / 204, 168 / 163.
 inline bool select_first(int64_t total, int64_t n) {
-    return n <= total / 2 && (total >= (int64_t(1) << 21) || (n <= 2048 && total > 8192));
+    return total - 2 * n >= 2800000 || (n <= 2048 && total > 8192);
 }
 constexpr int kSelBits = 13, kSelBins = 1 << kSelBits, kSelThreads = 512;
 
