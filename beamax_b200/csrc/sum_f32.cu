@@ -802,9 +802,9 @@ __device__ __forceinline__ unsigned reached_mask(const Rec<D> &r, const TileGrou
         }
         return m;
     }
+    const bool positive = positive_form<D>(r.p);
     // (not unrolled: eight copies of the ball test cost the kernels' instruction
     // fetches more than the loop: 0.72 against 0.63 ms for a periodic transpose)
-    const bool positive = positive_form<D>(r.p);
 #pragma unroll 1
     for (int g = 0; g < NW; ++g) {
         const GroupInfo<D> &q = tg.g[g];
@@ -1227,12 +1227,19 @@ __device__ __forceinline__ void kahan_add(float &acc, float &cmp, float v) {
 
 // A tile's beams in n ranges of len, each its own work item with a partial
 // (compensated sum, compensation) per output, added in order by
-// combine_parts_kernel.  n = 1: the item writes the output itself.
+// combine_parts_kernel.  n = 1: the item writes the output itself.  part = nullptr (a
+// workspace without room for the partials) and n > 1: an item takes all of its tile's
+// ranges, one after the other, and adds them in the same order in shared memory, so
+// that the result is the same bits whatever the workspace.
 struct Split {
     int n;
     int64_t len;
     float2 *part;  // (n, ns, nt)
+    __host__ __device__ bool serial() const { return n > 1 && !part; }
+    __host__ __device__ int items_per_tile() const { return part ? n : 1; }
 };
+// Shared memory of the ranges' totals in that case: (sensor, time) of the tile.
+constexpr size_t kTotalBytes = sizeof(float2) * TS * TT;
 
 // Work items a launch should have: 8 per resident CTA (2 per SM), so that the
 // last, unevenly filled wave is a small part of it.  Fewer tiles than that are
@@ -1245,6 +1252,11 @@ constexpr int64_t kSplitMin = 128;
 
 // out (or the chunk state) = sum over the ranges, in order, and over earlier
 // chunks; one 32 x 32 block of (sorted sensor, time) per CTA.
+__device__ __forceinline__ void add_part(float &a, float &c, float2 v) {
+    kahan_add(a, c, v.x);
+    kahan_add(a, c, -v.y);
+}
+
 __global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *perm, int64_t nt, int64_t ns, float *state,
                                      int first, int last, float *out) {
     __shared__ float2 tile[32][33];
@@ -1253,11 +1265,7 @@ __global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *p
         const int64_t s = s0 + k, t = t0 + threadIdx.x;
         float a = 0.0f, c = 0.0f;
         if (s < ns && t < nt) {
-            for (int q = 0; q < n; ++q) {
-                const float2 v = part[((int64_t)q * ns + s) * nt + t];
-                kahan_add(a, c, v.x);
-                kahan_add(a, c, -v.y);
-            }
+            for (int q = 0; q < n; ++q) add_part(a, c, part[((int64_t)q * ns + s) * nt + t]);
         }
         tile[k][threadIdx.x] = make_float2(a, c);
     }
@@ -1266,10 +1274,7 @@ __global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *p
         const int64_t s = s0 + threadIdx.x, t = t0 + k;
         if (s >= ns || t >= nt) continue;
         float2 v = tile[threadIdx.x][k];
-        if (!first) {
-            kahan_add(v.x, v.y, state[t * ns + s]);
-            kahan_add(v.x, v.y, -state[(nt + t) * ns + s]);
-        }
+        if (!first) add_part(v.x, v.y, make_float2(state[t * ns + s], state[(nt + t) * ns + s]));
         if (last) {
             out[t * ns + perm[s]] = v.x - v.y;
         } else {
@@ -1298,7 +1303,7 @@ __global__ void __launch_bounds__(THREADS, 2)
 fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
              const float *ds_g, const float *hn_g, const uint8_t *gfast_g, const int32_t *perm, float cutoff,
              float *out, unsigned long long *eval_count, int *work, int n_st, int n_items, Split sp, TrajSrc<D> T) {
-    extern __shared__ float rec[];  // rec_bytes<D>()
+    extern __shared__ __align__(16) float rec[];  // rec_bytes<D>(), then (sp.serial()) the ranges' totals
     __shared__ float sds[TS][D], shn[TS][D];
     __shared__ TileGroups<D> ginfo;
     __shared__ HomStage<D, TRAJ> hstage;
@@ -1316,7 +1321,7 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
         __syncthreads();
         const int item = tile_s;
         if (item >= n_items) break;
-        const int tile = item / sp.n, part = item % sp.n;
+        const int per_tile = sp.items_per_tile(), tile = item / per_tile;
         const int64_t st = tile % n_st, tt = tile / n_st;
         const int64_t s_first = offs[st], t_first = tt * TT;
         const int s_cnt = offs[st + 1] - offs[st];
@@ -1341,168 +1346,186 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
 #pragma unroll
         for (int i = 0; i < D; ++i) run.ds[i] = sds[gbase][i], run.h[i] = shn[gbase][i];
         const int g_cnt = max(0, min(GS, s_cnt - gbase));
-        // Kahan sums of sensors 2h and 2h + 1 in .x and .y
-        float2 acc2[GS / 2], cmp2[GS / 2];
+        // one range, or with sp.serial() all of the tile's in order
+        for (int part = item % per_tile, end = sp.serial() ? sp.n : part + 1; part < end; ++part) {
+            // Kahan sums of sensors 2h and 2h + 1 in .x and .y
+            float2 acc2[GS / 2], cmp2[GS / 2];
 #pragma unroll
-        for (int h = 0; h < GS / 2; ++h) acc2[h] = make_float2(0.0f, 0.0f), cmp2[h] = make_float2(0.0f, 0.0f);
-        if (TRAJ && sp.n == 1 && !T.first && lane < t_cnt && active) {
-            const int64_t t = t_first + lane;
+            for (int h = 0; h < GS / 2; ++h) acc2[h] = make_float2(0.0f, 0.0f), cmp2[h] = make_float2(0.0f, 0.0f);
+            if (TRAJ && sp.n == 1 && !T.first && lane < t_cnt && active) {
+                const int64_t t = t_first + lane;
 #pragma unroll
-            for (int k = 0; k < GS; ++k) {
-                const int s = gbase + k;
-                if (s < s_cnt) {
-                    const float a = T.state[t * P.ns + s_first + s];
-                    const float c = T.state[(P.nt + t) * P.ns + s_first + s];
-                    if (k & 1)
-                        acc2[k / 2].y = a, cmp2[k / 2].y = c;
-                    else
-                        acc2[k / 2].x = a, cmp2[k / 2].x = c;
-                }
-            }
-        }
-        const int64_t jb = part * sp.len;
-        const int64_t nbeam = min(jb + sp.len, TRAJ ? T.nb : B.n);
-        int nq = 0;  // queued survivors (the same in every thread)
-
-        for (int64_t j0 = jb; j0 < nbeam; j0 += SCAN * THREADS) {
-            unsigned bp[SCAN], bm[SCAN];
-#pragma unroll
-            for (int k = 0; k < SCAN; ++k) {
-                const int64_t j = j0 + k * THREADS + tid;
-                bool keep_p = false, keep_m = false;
-                if (j < nbeam) {
-                    if (TRAJ) {
-                        keep_p = traj_survives<D>(T, j, tt, ti, cutoff);
-                    } else {
-                        const Cull<D> cb = cull[j];
-                        keep_p = mode_on(B.modes, 0) && survives<D>(cb, (float)P.c, ta, tb, ti, P, cutoff);
-                        keep_m = mode_on(B.modes, 1) && survives<D>(cb, -(float)P.c, ta, tb, ti, P, cutoff);
+                for (int k = 0; k < GS; ++k) {
+                    const int s = gbase + k;
+                    if (s < s_cnt) {
+                        const float a = T.state[t * P.ns + s_first + s];
+                        const float c = T.state[(P.nt + t) * P.ns + s_first + s];
+                        if (k & 1)
+                            acc2[k / 2].y = a, cmp2[k / 2].y = c;
+                        else
+                            acc2[k / 2].x = a, cmp2[k / 2].x = c;
                     }
                 }
-                bp[k] = __ballot_sync(0xffffffffu, keep_p);
-                bm[k] = TRAJ ? 0u : __ballot_sync(0xffffffffu, keep_m);
-                if (lane == 0) warp_cnt[k * NW + warp] = __popc(bp[k]) + __popc(bm[k]);
             }
-            __syncthreads();
-            int tot = 0;
-            const unsigned lt = (1u << lane) - 1u;
+            const int64_t jb = part * sp.len;
+            const int64_t nbeam = min(jb + sp.len, TRAJ ? T.nb : B.n);
+            int nq = 0;  // queued survivors (the same in every thread)
+
+            for (int64_t j0 = jb; j0 < nbeam; j0 += SCAN * THREADS) {
+                unsigned bp[SCAN], bm[SCAN];
 #pragma unroll
-            for (int k = 0; k < SCAN; ++k) {
-                const int off = nq + scan_counts<SCAN>(warp_cnt, k, warp, tot);
-                const int32_t j = (int32_t)(j0 + k * THREADS + tid);
-                if (bp[k] >> lane & 1u) surv[off + __popc(bp[k] & lt)] = j;
-                if (!TRAJ && (bm[k] >> lane & 1u)) surv[off + __popc(bp[k]) + __popc(bm[k] & lt)] = (int32_t)(j + B.n);
-            }
-            const int old = nq;
-            nq += tot;
-            __syncthreads();
-            if constexpr (TRAJ && !PERIODIC) {
-                if (T.limits)
-                    nq = refine<D>(T, t_first, t_cnt, ti, ginfo, thr, surv, old, nq, keep, warp_cnt,
-                                   [&](int c) { return (int64_t)surv[c]; });
-            }
-            const bool last_scan = j0 + SCAN * THREADS >= nbeam;
-            int g0 = 0;
-            while (nq - g0 >= G || (last_scan && g0 < nq)) {
-                const int nb = min(G, nq - g0);
-                record_pass<D, TRAJ>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb,
-                                     [&](int i) { return (int64_t)surv[g0 + i]; });
+                for (int k = 0; k < SCAN; ++k) {
+                    const int64_t j = j0 + k * THREADS + tid;
+                    bool keep_p = false, keep_m = false;
+                    if (j < nbeam) {
+                        if (TRAJ) {
+                            keep_p = traj_survives<D>(T, j, tt, ti, cutoff);
+                        } else {
+                            const Cull<D> cb = cull[j];
+                            keep_p = mode_on(B.modes, 0) && survives<D>(cb, (float)P.c, ta, tb, ti, P, cutoff);
+                            keep_m = mode_on(B.modes, 1) && survives<D>(cb, -(float)P.c, ta, tb, ti, P, cutoff);
+                        }
+                    }
+                    bp[k] = __ballot_sync(0xffffffffu, keep_p);
+                    bm[k] = TRAJ ? 0u : __ballot_sync(0xffffffffu, keep_m);
+                    if (lane == 0) warp_cnt[k * NW + warp] = __popc(bp[k]) + __popc(bm[k]);
+                }
                 __syncthreads();
-                unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
-                evals += (unsigned long long)__popc(bits) * (unsigned)(t_cnt * g_cnt);
-                while (bits) {
-                    if (fast) {
-                        const int i0 = take_bit(bits), i1 = take_bit(bits), i2 = take_bit(bits), i3 = take_bit(bits);
-                        cf2 za, fa, qa, zb, fb, qb;
-                        int direct = seed_pair<D>(rec, i0, i1, lane, run, skip, za, fa, qa);
-                        zb = fb = qb = cf2{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-                        if (i2 >= 0) direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
-                        {
-                            // z_{k+1} = z_k f_k, f_{k+1} = f_k q; sensors 2h, 2h + 1
-                            // share a paired compensated addition per two beams (one or
-                            // two beams left: the other pair is zero -- a second loop for
-                            // them costs more in instruction fetches than it saves)
+                int tot = 0;
+                const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-                            for (int h = 0; h < GS / 2; ++h) {
-                                if (h > 0) {
+                for (int k = 0; k < SCAN; ++k) {
+                    const int off = nq + scan_counts<SCAN>(warp_cnt, k, warp, tot);
+                    const int32_t j = (int32_t)(j0 + k * THREADS + tid);
+                    if (bp[k] >> lane & 1u) surv[off + __popc(bp[k] & lt)] = j;
+                    if (!TRAJ && (bm[k] >> lane & 1u)) surv[off + __popc(bp[k]) + __popc(bm[k] & lt)] = (int32_t)(j + B.n);
+                }
+                const int old = nq;
+                nq += tot;
+                __syncthreads();
+                if constexpr (TRAJ && !PERIODIC) {
+                    if (T.limits)
+                        nq = refine<D>(T, t_first, t_cnt, ti, ginfo, thr, surv, old, nq, keep, warp_cnt,
+                                       [&](int c) { return (int64_t)surv[c]; });
+                }
+                const bool last_scan = j0 + SCAN * THREADS >= nbeam;
+                int g0 = 0;
+                while (nq - g0 >= G || (last_scan && g0 < nq)) {
+                    const int nb = min(G, nq - g0);
+                    record_pass<D, TRAJ>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb,
+                                         [&](int i) { return (int64_t)surv[g0 + i]; });
+                    __syncthreads();
+                    unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
+                    evals += (unsigned long long)__popc(bits) * (unsigned)(t_cnt * g_cnt);
+                    while (bits) {
+                        if (fast) {
+                            const int i0 = take_bit(bits), i1 = take_bit(bits), i2 = take_bit(bits), i3 = take_bit(bits);
+                            cf2 za, fa, qa, zb, fb, qb;
+                            int direct = seed_pair<D>(rec, i0, i1, lane, run, skip, za, fa, qa);
+                            zb = fb = qb = cf2{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                            if (i2 >= 0) direct |= seed_pair<D>(rec, i2, i3, lane, run, skip, zb, fb, qb) << 2;
+                            {
+                                // z_{k+1} = z_k f_k, f_{k+1} = f_k q; sensors 2h, 2h + 1
+                                // share a paired compensated addition per two beams (one or
+                                // two beams left: the other pair is zero -- a second loop for
+                                // them costs more in instruction fetches than it saves)
+#pragma unroll
+                                for (int h = 0; h < GS / 2; ++h) {
+                                    if (h > 0) {
+                                        za = cmul2(za, fa);
+                                        zb = cmul2(zb, fb);
+                                        fa = cmul2(fa, qa);
+                                        fb = cmul2(fb, qb);
+                                    }
+                                    const float2 a0 = za.re, b0 = zb.re;
                                     za = cmul2(za, fa);
                                     zb = cmul2(zb, fb);
                                     fa = cmul2(fa, qa);
                                     fb = cmul2(fb, qb);
+                                    kahan_add2(acc2[h], cmp2[h], make_float2(a0.x + a0.y, za.re.x + za.re.y));
+                                    if (i2 >= 0) kahan_add2(acc2[h], cmp2[h], make_float2(b0.x + b0.y, zb.re.x + zb.re.y));
                                 }
-                                const float2 a0 = za.re, b0 = zb.re;
-                                za = cmul2(za, fa);
-                                zb = cmul2(zb, fb);
-                                fa = cmul2(fa, qa);
-                                fb = cmul2(fb, qb);
-                                kahan_add2(acc2[h], cmp2[h], make_float2(a0.x + a0.y, za.re.x + za.re.y));
-                                if (i2 >= 0) kahan_add2(acc2[h], cmp2[h], make_float2(b0.x + b0.y, zb.re.x + zb.re.y));
                             }
-                        }
-                        if (!__any_sync(0xffffffffu, direct != 0)) continue;
-                        // rare: recurrences out of FP32's range
+                            if (!__any_sync(0xffffffffu, direct != 0)) continue;
+                            // rare: recurrences out of FP32's range
 #pragma unroll 1
-                        for (int e = 0; e < 4; ++e) {
-                            if (!__any_sync(0xffffffffu, direct >> e & 1)) continue;
-                            Rec<D> r;
-                            load_rec<D>(rec, e == 0 ? i0 : (e == 1 ? i1 : (e == 2 ? i2 : i3)), lane, r);
+                            for (int e = 0; e < 4; ++e) {
+                                if (!__any_sync(0xffffffffu, direct >> e & 1)) continue;
+                                Rec<D> r;
+                                load_rec<D>(rec, e == 0 ? i0 : (e == 1 ? i1 : (e == 2 ? i2 : i3)), lane, r);
+                                float v[GS];
+#pragma unroll 1
+                                for (int k = 0; k < GS; ++k)
+                                    v[k] = (direct >> e & 1) ? direct_eval<D, false>(r, sds[gbase + k], P).re : 0.0f;
+#pragma unroll
+                                for (int h = 0; h < GS / 2; ++h)
+                                    kahan_add2(acc2[h], cmp2[h], make_float2(v[2 * h], v[2 * h + 1]));
+                            }
+                        } else {
+                            // broken runs (sensors off the grid, periodic domains): every
+                            // sensor directly, values staged in a small array (one copy
+                            // of the evaluation in the instruction cache)
+                            const int i0 = take_bit(bits), i1 = take_bit(bits);
+                            Rec<D> ra, rb;
+                            load_rec<D>(rec, i0, lane, ra);
+                            load_rec<D>(rec, i1 >= 0 ? i1 : i0, lane, rb);
+                            if (i1 < 0) rb.amp = 0.0f;
                             float v[GS];
 #pragma unroll 1
                             for (int k = 0; k < GS; ++k)
-                                v[k] = (direct >> e & 1) ? direct_eval<D, false>(r, sds[gbase + k], P).re : 0.0f;
+                                v[k] = direct_eval<D, PERIODIC>(ra, sds[gbase + k], P).re +
+                                       direct_eval<D, PERIODIC>(rb, sds[gbase + k], P).re;
 #pragma unroll
                             for (int h = 0; h < GS / 2; ++h)
                                 kahan_add2(acc2[h], cmp2[h], make_float2(v[2 * h], v[2 * h + 1]));
                         }
-                    } else {
-                        // broken runs (sensors off the grid, periodic domains): every
-                        // sensor directly, values staged in a small array (one copy
-                        // of the evaluation in the instruction cache)
-                        const int i0 = take_bit(bits), i1 = take_bit(bits);
-                        Rec<D> ra, rb;
-                        load_rec<D>(rec, i0, lane, ra);
-                        load_rec<D>(rec, i1 >= 0 ? i1 : i0, lane, rb);
-                        if (i1 < 0) rb.amp = 0.0f;
-                        float v[GS];
-#pragma unroll 1
-                        for (int k = 0; k < GS; ++k)
-                            v[k] = direct_eval<D, PERIODIC>(ra, sds[gbase + k], P).re +
-                                   direct_eval<D, PERIODIC>(rb, sds[gbase + k], P).re;
+                    }
+                    g0 += nb;
+                    __syncthreads();
+                }
+                if (g0 > 0 && g0 < nq) {  // fewer than G survivors wait for the next scan
+                    const int32_t left = tid < nq - g0 ? surv[g0 + tid] : 0;
+                    __syncthreads();
+                    if (tid < nq - g0) surv[tid] = left;
+                }
+                nq -= g0;
+            }
+            if (lane < t_cnt && active) {
+                const int64_t t = t_first + lane;
 #pragma unroll
-                        for (int h = 0; h < GS / 2; ++h)
-                            kahan_add2(acc2[h], cmp2[h], make_float2(v[2 * h], v[2 * h + 1]));
+                for (int k = 0; k < GS; ++k) {
+                    const int s = gbase + k;
+                    if (s < s_cnt) {
+                        const float a = (k & 1) ? acc2[k / 2].y : acc2[k / 2].x;
+                        const float c = (k & 1) ? cmp2[k / 2].y : cmp2[k / 2].x;
+                        if (sp.part) {
+                            sp.part[((int64_t)part * P.ns + s_first + s) * P.nt + t] = make_float2(a, c);
+                        } else if (sp.n > 1) {
+                            // this thread's own entries
+                            float2 &tot = reinterpret_cast<float2 *>(rec + rec_bytes<D>() / sizeof(float))[s * TT + lane];
+                            float sa = part ? tot.x : 0.0f, sc = part ? tot.y : 0.0f;
+                            add_part(sa, sc, make_float2(a, c));
+                            tot = make_float2(sa, sc);
+                            if (part < sp.n - 1) continue;
+                            const int64_t at = t * P.ns + s_first + s;
+                            if (TRAJ && !T.first) add_part(sa, sc, make_float2(T.state[at], T.state[P.nt * P.ns + at]));
+                            if (TRAJ && !T.last) {
+                                T.state[at] = sa;
+                                T.state[P.nt * P.ns + at] = sc;
+                            } else {
+                                out[t * P.ns + perm[s_first + s]] = sa - sc;
+                            }
+                        } else if (TRAJ && !T.last) {
+                            T.state[t * P.ns + s_first + s] = a;
+                            T.state[(P.nt + t) * P.ns + s_first + s] = c;
+                        } else {
+                            out[t * P.ns + perm[s_first + s]] = a - c;
+                        }
                     }
                 }
-                g0 += nb;
-                __syncthreads();
             }
-            if (g0 > 0 && g0 < nq) {  // fewer than G survivors wait for the next scan
-                const int32_t left = tid < nq - g0 ? surv[g0 + tid] : 0;
-                __syncthreads();
-                if (tid < nq - g0) surv[tid] = left;
-            }
-            nq -= g0;
+            __syncthreads();
         }
-        if (lane < t_cnt && active) {
-            const int64_t t = t_first + lane;
-#pragma unroll
-            for (int k = 0; k < GS; ++k) {
-                const int s = gbase + k;
-                if (s < s_cnt) {
-                    const float a = (k & 1) ? acc2[k / 2].y : acc2[k / 2].x;
-                    const float c = (k & 1) ? cmp2[k / 2].y : cmp2[k / 2].x;
-                    if (sp.n > 1) {
-                        sp.part[((int64_t)part * P.ns + s_first + s) * P.nt + t] = make_float2(a, c);
-                    } else if (TRAJ && !T.last) {
-                        T.state[t * P.ns + s_first + s] = a;
-                        T.state[(P.nt + t) * P.ns + s_first + s] = c;
-                    } else {
-                        out[t * P.ns + perm[s_first + s]] = a - c;
-                    }
-                }
-            }
-        }
-        __syncthreads();
     }
     if (eval_count && lane == 0 && evals) atomicAdd(eval_count, evals);
 }
@@ -1863,15 +1886,14 @@ size_t split_bytes(const msgb_problem *p, int64_t nbeam) {
     return n > 1 ? align256((size_t)n * (size_t)p->ns * (size_t)p->nt * sizeof(float2)) : 0;
 }
 
-// The ranges that fit in `spare` bytes at `at` (one range needs none).
+// The ranges of a problem, with their partials at `at` where `spare` bytes hold them.
 Split make_split(const msgb_problem *p, int64_t n_tiles, int64_t nbeam, char *at, size_t spare) {
     const size_t per = (size_t)p->ns * (size_t)p->nt * sizeof(float2);
     int64_t n = split_count(n_tiles, nbeam);
-    if (per * (size_t)n > spare) n = (int64_t)(spare / per);
     if (n < 2) return Split{1, nbeam > 0 ? nbeam : 1, nullptr};
     const int64_t len = ((nbeam + n - 1) / n + G - 1) / G * G;
     n = (nbeam + len - 1) / len;
-    return Split{(int)n, len, n > 1 ? (float2 *)at : nullptr};
+    return Split{(int)n, len, n > 1 && per * (size_t)n <= spare ? (float2 *)at : nullptr};
 }
 
 // Limits of a trajectory chunk of nb beams (refine).  They follow everything else in a
@@ -2000,11 +2022,12 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
         at += taken, spare -= taken;
     }
     const Split sp = make_split(p, n_st * n_tt, TRAJ ? T.nb : b->n, ws + at, spare);
-    if (n_st * n_tt * sp.n > 0x7fffffffLL) return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: too many tiles");
-    const int n_items = (int)(n_st * n_tt * sp.n);
+    if (n_st * n_tt * sp.items_per_tile() > 0x7fffffffLL)
+        return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: too many tiles");
+    const int n_items = (int)(n_st * n_tt * sp.items_per_tile());
     const int64_t want = 2LL * sm_count();
     const unsigned grid = (unsigned)(want < n_items ? want : n_items);
-    constexpr size_t smem = rec_bytes<D>();
+    const size_t smem = rec_bytes<D>() + (sp.serial() ? kTotalBytes : 0);
     auto args = [&](auto kern) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<grid, THREADS, smem, st>>>(P, to_args(b), (const Cull<D> *)(ws + l.cull), hom,
@@ -2019,7 +2042,7 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     else
         args(fwd32_kernel<D, false, TRAJ>);
     if (int e = check_launch("msgb_sum_fwd_f32")) return e;
-    if (sp.n > 1) {
+    if (sp.part) {
         const dim3 cg((unsigned)((p->ns + 31) / 32), (unsigned)n_tt);
         if (cg.y > 65535u) return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: nt too large");
         combine_parts_kernel<<<cg, dim3(32, 8), 0, st>>>(sp.part, sp.n, (const int32_t *)(ws + l.vals_out), p->nt, p->ns,

@@ -116,7 +116,9 @@ int msgb_adj_gather_f64(const msgb_problem *prob, const msgb_beam_set *beams,
 /* FP32 forward with Kahan-compensated accumulation across beams, per-(beam,
  * time) FP64 range-reduced anchor phases and Gaussian cutoff culling.
  * out: (nt, ns) FP32.  The workspace (for n selected coefficients) covers
- * both this call and msgb_adj_gather_f32. */
+ * both this call and msgb_adj_gather_f32.  A smaller one that still holds what
+ * the call cannot do without (the error message gives the size) makes it slower;
+ * the result is the same bits. */
 size_t msgb_sum_f32_workspace_size(const msgb_problem *prob, int64_t n);
 int msgb_sum_fwd_f32(const msgb_problem *prob, const msgb_beam_set *beams,
                      const msgb_sum_opts *opts, void *workspace, size_t workspace_bytes,
@@ -279,8 +281,8 @@ int msgb_rk4_trajectories(const msgb_problem *prob, const msgb_medium *med, cons
  * zeroes before the first chunk.
  * FP32: culled by the trajectory's boxes and, before the records are made, by
  * limits that each call forms from the records in its workspace (4 bytes per
- * time tile and beam; a workspace without room for them gives the same sums
- * slower); Kahan state (2 nt ns floats) lives in
+ * time tile and beam; without room for them the call is slower and its sums
+ * agree to FP32 rounding); Kahan state (2 nt ns floats) lives in
  * the workspace from the call with first_chunk != 0 to the call with
  * last_chunk != 0, which writes out (nt, ns) FP32.  All chunks of one
  * summation must use the same workspace and problem. */
