@@ -775,8 +775,11 @@ __device__ __forceinline__ void find_lattice(TileGroups<D> &tg) {
 }
 
 // Mask of the groups of the tile that this lane's record reaches within thr, for any
-// Im M: growing beams and records that are not finite among them.
-template <int D>
+// Im M: growing beams and records that are not finite among them.  UNROLL: of the loop
+// over groups that are no lattice.  Eight copies of the ball test are faster where it
+// runs (ring sensor at 256^2, forward: 3.43 ms, two copies 3.50) but slow the
+// transpose's instruction fetches where it does not (512^2: 56.1 against 53.4 ms).
+template <int D, int UNROLL>
 __device__ __forceinline__ unsigned reached_mask(const Rec<D> &r, const TileGroups<D> &tg, float thr) {
     unsigned m = 0;
     if (tg.lattice) {
@@ -803,9 +806,7 @@ __device__ __forceinline__ unsigned reached_mask(const Rec<D> &r, const TileGrou
         return m;
     }
     const bool positive = positive_form<D>(r.p);
-    // (not unrolled: eight copies of the ball test cost the kernels' instruction
-    // fetches more than the loop: 0.72 against 0.63 ms for a periodic transpose)
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int g = 0; g < NW; ++g) {
         const GroupInfo<D> &q = tg.g[g];
         if (q.kind && (q.kind == 3 || group_reached<D>(r, positive, q, thr))) m |= 1u << g;
@@ -832,7 +833,7 @@ __device__ __noinline__ void general_beam_time(const ProbArgs &P, const BeamArgs
 // the homogeneous forward (15.7 of 48.6 ms at 512^2), half of the trajectory sums
 // before refine.  What a record needs beyond the test (the anchor phase, the amplitude) is formed
 // only when the beam reaches some group at some time.
-template <int D, bool TRAJ, typename BeamOf>
+template <int D, bool PERIODIC, bool TRAJ, int UNROLL, typename BeamOf>
 __device__ __forceinline__ void record_pass(const ProbArgs &P, const BeamArgs &B, const TrajSrc<D> &T,
                                             const HomBeam<D> *hom, HomStage<D, TRAJ> &stage, int64_t t_first, int t_cnt,
                                             const TileInfo<D> &ti, const TileGroups<D> &tg, float thr, float *rec,
@@ -951,7 +952,8 @@ __device__ __forceinline__ void record_pass(const ProbArgs &P, const BeamArgs &B
             r.d0[a] = (float)dd[a];
             r.wp[a] = (float)wpd[a];
         }
-        const unsigned reach = !tv ? 0u : (thr > 0.0f ? reached_mask<D>(r, tg, thr) : tg.present);
+        // (periodic domains: no group is left out)
+        const unsigned reach = !tv ? 0u : (!PERIODIC && thr > 0.0f ? reached_mask<D, UNROLL>(r, tg, thr) : tg.present);
         const unsigned m = __reduce_or_sync(0xffffffffu, reach);
         if (m) {
             double lin = 0.0;
@@ -1191,7 +1193,7 @@ __device__ __forceinline__ int refine(const TrajSrc<D> &T, int64_t t_first, int 
             for (int q = 0; q < Sym<D>::S; ++q) r.p[q] = bt->p[q];
             const float up = fmaf((float)code, 1.0f / kLimitSteps, 1.0f);
             const unsigned hit =
-                __ballot_sync(0xffffffffu, code == kNoLimit || reached_mask<D>(r, tg, thr * up * up) != 0);
+                __ballot_sync(0xffffffffu, code == kNoLimit || reached_mask<D, 2>(r, tg, thr * up * up) != 0);
             if (smp == 0 && c0 + lane / 4 < end) keep[c0 + lane / 4 - base] = (hit >> lane & 15u) ? 1 : 0;
         }
         __syncthreads();
@@ -1412,7 +1414,7 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                 int g0 = 0;
                 while (nq - g0 >= G || (last_scan && g0 < nq)) {
                     const int nb = min(G, nq - g0);
-                    record_pass<D, TRAJ>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb,
+                    record_pass<D, PERIODIC, TRAJ, 8>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb,
                                          [&](int i) { return (int64_t)surv[g0 + i]; });
                     __syncthreads();
                     unsigned bits = __ballot_sync(0xffffffffu, active && lane < nb && (alive[lane] >> warp & 1));
@@ -1665,7 +1667,7 @@ adj32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
                 const int nb = min(G, nq - g0);
                 uint8_t *alive = alive2[flip];
                 flip ^= 1;
-                record_pass<D, TRAJ>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb, [&](int i) {
+                record_pass<D, PERIODIC, TRAJ, 2>(P, B, T, hom, hstage, t_first, t_cnt, ti, ginfo, thr, rec, alive, nb, [&](int i) {
                     const int q = surv[g0 + i];
                     return TRAJ || q < RJ ? r0 + q : B.n + r0 + q - RJ;
                 });
