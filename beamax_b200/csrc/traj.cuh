@@ -627,12 +627,13 @@ struct RecordWriter {
             double lam;
             if (D == 2) {
                 // smaller eigenvalue as det / larger: the determinant in FP64, the
-                // rest in FP32 (relative error below 1e-6, taken off here)
+                // rest in FP32 (relative error below 1e-6, taken off here; zero, which
+                // leaves no beam out, where a square would leave FP32's range)
                 const double a = f[1], b = f[3 % (2 * S)], c = f[5 % (2 * S)];
                 const float m = 0.5f * (f[1] + f[5 % (2 * S)]), h = 0.5f * (f[1] - f[5 % (2 * S)]);
                 const float den = m + sqrtf(fmaf(h, h, f[3 % (2 * S)] * f[3 % (2 * S)]));
                 const float det = (float)fma(a, c, -b * b);
-                const float l = den > 0.0f ? __fdividef(det, den) : 0.0f;
+                const float l = m > 1e-15f && m < 1e18f ? __fdividef(det, den) : 0.0f;
                 lam = (double)(l - 1e-6f * fabsf(l));
             } else {
                 double Sm[D][D];
