@@ -316,7 +316,7 @@ __constant__ double DP_D[7] = {-12715105075.0 / 11282082432.0, 0.0, 87487479700.
 //   1: steps follow the error control alone (only the last is shortened to
 //      end at ts[nt-1]) and save times inside a step are read from the
 //      continuous extension, as diffrax's SaveAt(ts) reads its interpolant.
-extern __shared__ double dopri_stage_smem[];
+extern __shared__ __align__(16) double dopri_stage_smem[];
 // Dynamic shared memory of the integrator kernels: 7 stages per lane (43 KB
 // for a block of 64 lanes in 2D, 72 KB in 3D).
 template <int D>
