@@ -609,8 +609,7 @@ extern "C" int msgb_mswpt_create(const msgb_mswpt_desc *d, msgb_mswpt **out) {
     for (int m = 0; m < p->tw_n; ++m) {
         // from the first octant: exact at the multiples of a quarter turn
         const int q = (int)((8LL * m) / p->tw_n);  // octant
-        const double a = 2.0 * 3.14159265358979323846 * m / p->tw_n;
-        double c = cos(a), s = sin(a);
+        double c, s;
         if ((4LL * m) % p->tw_n == 0) {
             const int k = (int)((4LL * m) / p->tw_n);
             c = k == 0 ? 1.0 : (k == 2 ? -1.0 : 0.0);

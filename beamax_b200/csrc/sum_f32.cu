@@ -511,12 +511,11 @@ __global__ void sensor_key_kernel(const double *sens, int64_t ns, ProbArgs P, ui
     val[s] = (int32_t)s;
 }
 
-// Per tile: anchor, bounding box, FP32 offsets, steps, run starts and the
-// per-group fast flag (one straight run of GS sensors, no periodic wrap).
+// Per tile: anchor, bounding box, FP32 offsets, steps and the per-group fast flag (one
+// straight run of GS sensors, no periodic wrap).
 template <int D>
 __global__ void tile_kernel(const double *sens, const int32_t *perm, const int32_t *offs, ProbArgs P,
-                            TileInfo<D> *tiles, float *ds, float *hn, uint8_t *seed, uint8_t *gfast,
-                            double *sorted) {
+                            TileInfo<D> *tiles, float *ds, float *hn, uint8_t *gfast) {
     const int64_t tile = blockIdx.x;
     const int64_t first = offs[tile];
     const int cnt = offs[tile + 1] - offs[tile];
@@ -563,7 +562,6 @@ __global__ void tile_kernel(const double *sens, const int32_t *perm, const int32
                         s = e2 > 1e-12 * n2;
                     }
                 }
-                seed[first + k] = s ? 1 : 0;
             }
             if (s) have_h = false;
             if (k % GS == 0) fastmask = 1;
@@ -577,7 +575,6 @@ __global__ void tile_kernel(const double *sens, const int32_t *perm, const int32
             const double c = 0.5 * (lo[i] + hi[i]);
             ds[(first + k) * D + i] = (float)(pos[k][i] - c);
             hn[(first + k) * D + i] = (k + 1 < cnt) ? (float)(pos[k + 1][i] - pos[k][i]) : 0.0f;
-            sorted[(first + k) * D + i] = pos[k][i];
         }
     }
 }
@@ -1810,8 +1807,7 @@ __global__ void reduce_parts_kernel(const double *part, int64_t n_tt, int64_t ns
 
 // ------------------------------------------------------------------ workspace
 struct Layout {
-    size_t keys_in, keys_out, vals_in, vals_out, cub, tiles, offs, gfast, ds, hn, seed, sorted, cull, data, work, part,
-        total;
+    size_t keys_in, keys_out, vals_in, vals_out, cub, tiles, offs, gfast, ds, hn, cull, data, work, part, total;
     size_t cub_bytes;
     int64_t n_st;
     int64_t cull_cap;  // beams the culling table has room for
@@ -1844,8 +1840,6 @@ Layout layout(const msgb_problem *p, int64_t n_beams, bool with_data, int64_t n_
     l.gfast = o; o = align256(o + n_st * NW);
     l.ds = o; o = align256(o + ns * D * 4);
     l.hn = o; o = align256(o + ns * D * 4);
-    l.seed = o; o = align256(o + ns + 1);
-    l.sorted = o; o = align256(o + ns * D * 8);
     l.cull_cap = n_beams > 0 ? n_beams : 1;
     l.cull = o; o = align256(o + l.cull_cap * sizeof(Cull<3>));
     l.data = o; o = align256(o + (with_data ? p->nt * ns * 4 : 0));
@@ -1966,8 +1960,7 @@ int prep(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *o, 
         fixed_offsets_kernel<<<(unsigned)((l.n_st + 1 + blk - 1) / blk), blk, 0, st>>>(offs, l.n_st, ns);
     }
     tile_kernel<D><<<(unsigned)l.n_st, 128, 0, st>>>(p->sensors, vout, offs, to_args(p), (TileInfo<D> *)(ws + l.tiles),
-                                                    (float *)(ws + l.ds), (float *)(ws + l.hn), (uint8_t *)(ws + l.seed),
-                                                    (uint8_t *)(ws + l.gfast), (double *)(ws + l.sorted));
+                                                    (float *)(ws + l.ds), (float *)(ws + l.hn), (uint8_t *)(ws + l.gfast));
     if (b->n > 0)
         cull_prep_kernel<D><<<(unsigned)((b->n + blk - 1) / blk), blk, 0, st>>>(to_args(b), (Cull<D> *)(ws + l.cull));
     return check_launch("msgb sum f32 prep");
@@ -2008,8 +2001,7 @@ int run_fwd(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     if (int e = prep<D>(p, TRAJ ? &none : b, o, l, ws, st)) return e;
     const int64_t n_st = l.n_st, n_tt = (p->nt + TT - 1) / TT;
     if (n_st * n_tt > 0x7fffffffLL) return fail(MSGB_ERR_UNSUPPORTED, "msgb_sum_fwd_f32: too many tiles");
-    ProbArgs P = to_args(p);
-    P.sensors = (const double *)(ws + l.sorted);
+    const ProbArgs P = to_args(p);
     int *work = (int *)(ws + l.work);
     cudaMemsetAsync(work, 0, sizeof(int), st);
     bool periodic = false;
@@ -2063,8 +2055,7 @@ int run_adj(const msgb_problem *p, const msgb_beam_set *b, const msgb_sum_opts *
     if (tg.y > 65535u) return fail(MSGB_ERR_UNSUPPORTED, "msgb_adj_gather_f32: nt too large");
     transpose_permute_kernel<<<tg, dim3(32, 8), 0, st>>>(data, (const int32_t *)(ws + l.vals_out), p->nt, p->ns,
                                                          (float *)(ws + l.data));
-    ProbArgs P = to_args(p);
-    P.sensors = (const double *)(ws + l.sorted);
+    const ProbArgs P = to_args(p);
     bool periodic = false;
     for (int i = 0; i < D; ++i) periodic |= (p->periodic[i] != 0);
     const int64_t nw = TRAJ ? T.nb : b->n;  // beam indices j of the items

@@ -213,7 +213,7 @@ struct AcceptArgs {
 
 template <int D>
 __global__ void records_kernel(ProbArgs P, MediumArgs med, BeamArgs B, SurrIO io, const float *Yp, const float *mean,
-                               const float *stdv, AcceptArgs acc, TrajArgs T, int tt_len) {
+                               const float *stdv, AcceptArgs acc, TrajArgs T) {
     constexpr int S = SurrDims<D>::S;
     const int64_t bl = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (bl >= io.nb) return;
@@ -354,9 +354,9 @@ extern "C" int msgb_surrogate_records(const msgb_problem *prob, const msgb_mediu
     cudaStream_t st = as_stream(stream);
     ProbArgs P = to_args(prob);
     switch (prob->ndim) {
-        case 1: records_kernel<1><<<grid, blk, 0, st>>>(P, M, to_args(beams), S, Y, mean, stdv, A, T, MSGB_TIME_TILE); break;
-        case 2: records_kernel<2><<<grid, blk, 0, st>>>(P, M, to_args(beams), S, Y, mean, stdv, A, T, MSGB_TIME_TILE); break;
-        default: records_kernel<3><<<grid, blk, 0, st>>>(P, M, to_args(beams), S, Y, mean, stdv, A, T, MSGB_TIME_TILE); break;
+        case 1: records_kernel<1><<<grid, blk, 0, st>>>(P, M, to_args(beams), S, Y, mean, stdv, A, T); break;
+        case 2: records_kernel<2><<<grid, blk, 0, st>>>(P, M, to_args(beams), S, Y, mean, stdv, A, T); break;
+        default: records_kernel<3><<<grid, blk, 0, st>>>(P, M, to_args(beams), S, Y, mean, stdv, A, T); break;
     }
     return check_launch("msgb_surrogate_records");
 }

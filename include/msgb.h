@@ -135,7 +135,7 @@ int msgb_sum_fwd_f32(const msgb_problem *prob, const msgb_beam_set *beams,
  * numerics as msgb_sum_fwd_f32 on the current device.
  *   - Limit: problems whose forward scratch exceeds the array are rejected
  *     with MSGB_ERR_UNSUPPORTED and a message giving the bytes needed (about
- *     44 B per coefficient plus 50-70 B per sensor: 65536 coefficients and
+ *     44 B per coefficient plus 30-50 B per sensor: 65536 coefficients and
  *     2044 sensors take about 3 MB, and 16 MiB holds about 370000
  *     coefficients at that sensor count).
  *   - The first call on each device, with that device current, looks up the

@@ -120,7 +120,7 @@ def test_a_growing_beam_is_in_every_group_of_sensors(kind):
 
 
 # ---- trajectory records --------------------------------------------------------
-PAIRS = {2: [(0, 0), (0, 1), (1, 1)], 3: [(0, 0), (0, 1), (0, 2), (1, 1), (1, 2), (2, 2)]}
+PAIRS = {1: [(0, 0)], 2: [(0, 0), (0, 1), (1, 1)], 3: [(0, 0), (0, 1), (0, 2), (1, 1), (1, 2), (2, 2)]}
 
 
 def _rec(d):
@@ -145,7 +145,9 @@ class _Records:
         self.dev = _dev()
         self.rec, self.d = rec, rec["x"].shape[-1]
         d = self.d
-        self.pos = pos = np.concatenate([pos, np.full((len(pos), d - 2), 40 * DX)], 1)
+        # 1D: along the row; 3D: the row lies in a plane
+        pos = pos[:, 1:] if d == 1 else np.concatenate([pos, np.full((len(pos), d - 2), 40 * DX)], 1)
+        self.pos = pos = np.ascontiguousarray(pos)
         nt, nb = rec.shape
         n_tt = (nt + 31) // 32
         box = np.zeros((n_tt, nb, 2 * d + 1), np.float32)
@@ -237,7 +239,7 @@ def _compare(R, compact):
 
 
 @pytest.mark.parametrize("compact", [False, True])
-@pytest.mark.parametrize("kind,d", [("line", 2), ("run", 2), ("runs", 2), ("short", 2), ("scattered", 2), ("line", 3)])
+@pytest.mark.parametrize("kind,d", [("line", 2), ("run", 2), ("runs", 2), ("short", 2), ("scattered", 2), ("line", 1), ("line", 3)])
 def test_records_that_come_near_at_a_few_times_only(kind, d, compact):
     """Narrow beams (exponent 200 at the sensors) that are wide (2) at three of a
     tile's times."""
@@ -248,7 +250,7 @@ def test_records_that_come_near_at_a_few_times_only(kind, d, compact):
     _compare(_Records(rec, np.zeros(70, bool), _positions(kind)), compact)
 
 
-@pytest.mark.parametrize("kind,d", [("line", 2), ("scattered", 2), ("line", 3)])
+@pytest.mark.parametrize("kind,d", [("line", 1), ("line", 2), ("scattered", 2), ("line", 3)])
 @pytest.mark.parametrize("nt", [1, 7, 32, 37])
 @pytest.mark.parametrize("change", [0.02, 0.3, 3.0])
 def test_records_that_change_from_time_to_time(change, nt, kind, d):
