@@ -1,7 +1,8 @@
-// MSWPT tiling on the GPU: one global FFT (cuFFT, a library call) followed by
-// per-level batched box kernels that fuse the dual-filter division, the window
-// multiply, the parity roll, the unitary box IFFT (shared-memory radix-2), the
-// IVP half-wave factor, the conjugate half-mask and the top_n key.
+// MSWPT tiling on the GPU: one global FFT (cuFFT, a library call) followed by one
+// launch with a CTA per box, over all levels, that fuses the dual-filter division,
+// the window multiply, the parity roll, the unitary box IFFT (register passes of
+// radix 8, 4 and 2 in shared memory), the IVP half-wave factor, the conjugate
+// half-mask and the top_n key.
 //
 // Restates beamax transforms.py:591-733 (MSWPT.forward/_compute_coeffs) and
 // :735-850 (MSWPT.inverse); the Hermitian adjoint of the forward is the

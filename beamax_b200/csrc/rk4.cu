@@ -336,7 +336,10 @@ constexpr size_t dopri_mix_smem_bytes(int blk) {
 // persistent and all beams take about the same number of steps, so the time goes
 // by rounds of resident lanes: 7 blocks' round takes 1.117 of 6 blocks', and a last
 // round with few lanes 0.45 (latency only).  1024^2, 120,000 beams: 6 blocks 2.1
-// rounds 193 ms, 7 blocks 1.8 rounds 168 ms; 200,000 beams: 277 and 293 ms.
+// rounds 193 ms, 7 blocks 1.8 rounds 168 ms; 200,000 beams: 277 and 293 ms.  Linear
+// and 1D media go by the same rounds (128^2 linear, 60,000 beams: 20.5 and 16.9 ms,
+// 200,000: 44.7 and 48.6; 1D cubic, 120,000: 5.4 and 4.9); where a few lanes start a
+// round, as 114,000 beams, six would be up to a tenth faster than the rule's seven.
 inline int mix_blocks(int ndim, int64_t nb, int sms) {
     if (ndim == 3) return 4;
     auto cost = [&](int blocks, double round) {
@@ -952,12 +955,13 @@ __device__ __forceinline__ int64_t first_beam() {
     return (threadIdx.x & 31) * warps + blockIdx.x * (int64_t)(kOdeBlock / 32) + (threadIdx.x >> 5);
 }
 
-// Adaptive integration with persistent lanes: thread i integrates beams
-// i, i + stride, i + 2 stride, ... one attempted step per loop trip, so a
-// lane whose beam finishes early starts its next beam instead of idling
-// until the slowest beam of its warp is done.
-// MINB: resident 64-lane blocks per SM the register allocation is bounded for
-// (the stages take 43 KB of shared memory per block in 2D, so at most 5 fit).
+// Adaptive integration with persistent lanes: a lane integrates beam b =
+// first_beam(), then b + stride, b + 2 stride, ... (stride: the grid's lanes), one
+// attempted step per loop trip, so a lane whose beam finishes early starts its next
+// beam instead of idling until the slowest beam of its warp is done.
+// MINB: resident 64-lane blocks per SM the register allocation is bounded for (in 2D
+// the stages and, for a cubic medium, the stencils take 43 + 8 KB of shared memory
+// per block: 4 fit, 5 without stencils).
 template <int D, int KIND, int MINB, bool F32M, bool DENSE>
 __global__ void __launch_bounds__(64, MINB)
 dopri_kernel(ProbArgs P, MediumArgs med, BeamArgs B, TrajArgs T, OdeArgs o) {
@@ -1173,8 +1177,9 @@ struct TrFinal {
 };
 
 // Blocks of 64 lanes per SM of the adaptive integrator: MSGB_DOPRI_BLOCKS
-// (4 to 7; 5, 6 and 7 bound the registers to 204, 170 and 146; the FP64
-// integrator takes at most 5), else `dflt`.
+// (4 to 7; 5, 6 and 7 bound the registers to 204, 170 and 146), else `dflt`.  The
+// FP64 integrator takes at most 5, and 4 where its shared memory leaves no room for
+// more (2D and 3D cubic media).
 int dopri_blocks_per_sm(int dflt) {
     static const int env = [] {
         const char *e = getenv("MSGB_DOPRI_BLOCKS");
@@ -1297,7 +1302,8 @@ extern "C" int msgb_ode_trajectories(const msgb_problem *prob, const msgb_medium
         which.minb = dopri_blocks_per_sm(which.mixed() ? mix_blocks(prob->ndim, out->nb, sms) : 4);
         if (!which.mixed() && which.minb > 5) which.minb = 5;
         {
-            // the lanes are persistent: every block must be resident at once
+            // the lanes are persistent, so every block should be resident at once (in 3D
+            // the FP64 integrator's 72 KB let three be: a quarter of its lanes start late)
             constexpr int K = MSGB_MEDIUM_BSPLINE3;  // the largest
             const size_t sm_bytes =
                 1024 + (prob->ndim == 1 ? which.smem<1, K>() : (prob->ndim == 2 ? which.smem<2, K>() : which.smem<3, K>()));

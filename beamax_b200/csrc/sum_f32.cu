@@ -1240,8 +1240,9 @@ struct Split {
 // Shared memory of the ranges' totals in that case: (sensor, time) of the tile.
 constexpr size_t kTotalBytes = sizeof(float2) * TS * TT;
 
-// Work items a launch should have: 8 per resident CTA (2 per SM), so that the
-// last, unevenly filled wave is a small part of it.  Fewer tiles than that are
+// Work items a launch should have: 8 per resident CTA (2 per SM of the 148), so that
+// the last, unevenly filled wave is a small part of it (a constant, not the device's
+// own count: the order of the sums follows from it).  Fewer tiles than that are
 // split over the beams, in ranges of at least kSplitMin (8 passes of both modes):
 // 4,096 coefficients at 128^2 ran 19 blocks for 3.9 ms, now 0.24 ms; a 512-point
 // sensor at 512^2 304 blocks in two waves for 31.0 ms, 18.9 ms without the split

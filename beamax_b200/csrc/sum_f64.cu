@@ -490,7 +490,8 @@ adj64_kernel(ProbArgs P, BeamArgs B, TrajView<D> T, const double *__restrict__ d
 }
 
 // ---------------------------------------------------------------- launches
-// CTAs a launch should have: 4 per resident CTA (2 per SM); a cluster of at most 8
+// CTAs a launch should have: 4 per resident CTA (2 per SM of the 148; a constant, as the
+// order of the sums follows from it); a cluster of at most 8
 // shares what would be one CTA's work until there are as many.
 constexpr int64_t kCtasWanted = 4 * 2 * 148;
 

@@ -296,15 +296,15 @@ def ode_flops_split(d: int):
 def launches_per_step(hetero: bool, total_coeffs: int, n: int, nt: int, ns: int) -> int:
     """Hand-written kernels of libmsgb launched per step (cuFFT's and CUB's own
     kernels excluded)."""
-    select = total_coeffs >= 1 << 21 and n <= total_coeffs // 2
+    select = total_coeffs - 2 * n >= 2800000 or (n <= 2048 and total_coeffs > 8192)
     passes = 5 + -(-max(1, (total_coeffs - 1).bit_length()) // 13)
     topn = 1 + passes + 2 if select else 2  # start, digit passes, gather of the keys, take; or key bits, take
     prep = 4                                # tiling copy, check, clamp, tile description
+    split = int(((ns + 127) // 128) * ((nt + 31) // 32) < 8 * 2 * 148)
     if hetero:
-        sums, gather = 1 + 1, 1             # beam ODE, sum; gather
+        sums, gather = 1 + 1 + 1 + split, 1 + 1  # beam ODE, limits, sum, its combination; limits, gather
     else:
-        split = ((ns + 127) // 128) * ((nt + 31) // 32) < 8 * 2 * 148
-        sums, gather = 2 + 1 + int(split), 2 + 1  # culling and closed-form tables, sum, its combination; gather
+        sums, gather = 2 + 1 + split, 2 + 1  # culling and closed-form tables, sum, its combination; gather
     fwd = 1 + topn + 1 + prep + sums        # box transforms, selection, beam init
     adj = 1 + prep + 1 + gather + 1 + 1 + 3  # beam init, data permutation, partials, scatter, synthesis
     return fwd + adj
@@ -411,7 +411,7 @@ def run_ours(args, rank, world, device):
               "t_ode": t_ode, "ode_steps": ode_steps, "ndim": len(dom.N), "hetero": W["hetero"],
               "nt": nt, "ns": ns, "n_beams": 2 * n,
               # heterogeneous: chunks of trajectories beyond the one per call that launches_per_step counts
-              "extra_launches": 3 * max(0, sum(1 for nm, *_ in spans if "traj" in nm or "ode" in nm) - 3 * args.steps),
+              "extra_launches": 5 * max(0, sum(1 for nm, *_ in spans if "traj" in nm or "ode" in nm) - 3 * args.steps),
               "fwd_evals": fwd_evals, "adj_evals": adj_evals, "dense_step": dense_step, "clocks": clocks,
               "e2e_t": e2e_t, "h2d": p0.nbytes + nt * ns * 4, "d2h": nt * ns * 4 + p0.nbytes,
               "total_coeffs": wpt.total_coeffs, "workload": W["name"]}
