@@ -275,9 +275,10 @@ size_t box_smem(const LevelArgs &L) {
     return sizeof(double2) * (size_t)(L.P + (L.P >> 3)) + 3 * sizeof(int) * (size_t)(L.S[0] + L.S[1] + L.S[2]);
 }
 
-// Bound: HBM and L2 (16 B read and 24 B written per coefficient); what is spent is
-// mostly shared-memory passes and FP64 work of the box FFTs.  All index
-// arithmetic with divisions is done once per axis and support element in tables.
+// Bound: latency (loads, the barriers between the FFT's passes) and index instructions:
+// issue active 50 %, FP64 pipe 12 %, 5.6 warps per scheduler; the bytes (16 read and 24
+// written per coefficient) take a fifth of its time.  All index arithmetic with
+// divisions is done once per axis and support element in tables.
 // 4.2 million coefficients of 1024^2: 477 us with radix-2 passes, a launch per level
 // and divisions per element, 114 now (25 at the HBM rate).
 __global__ void __launch_bounds__(THREADS, 3) box_forward_kernel(AllLevels LV, FwdArgs A) {

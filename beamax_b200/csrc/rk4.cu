@@ -766,7 +766,8 @@ __device__ __forceinline__ void combine32(const K32 &k, float2 (&acc)[NP]) {
     }
 }
 
-// Bound: instruction issue and latency at 3 warps per scheduler (issue 43-46 %);
+// Bound: instruction issue and latency at 3 warps per scheduler (issue active 58 % with
+// every lane in use, no pipe above a third; 41 % at 1.7 warps);
 // 200,000 beams over 5,667 save times 437 ms before the vector stages, the stencil
 // cache, the 16-byte records and the paired sums, 263 now; 2,000 beams 56.8 -> 33.3 ms.
 //

@@ -1293,11 +1293,12 @@ __global__ void combine_parts_kernel(const float2 *part, int n, const int32_t *p
 // before each compensated addition).
 //
 // Bound: FP32 pipe (recurrence 8 FMA-pipe operations per triple, seed ~75 per 16
-// triples) with the seeds' MUFU work beside it; measured 51 % (2D) and 58 % (3D) of
-// that pipe's cycles, the rest in pass barriers and latency.  512^2 homogeneous
-// (65,536 coefficients, 2,414 times, 2,044 sensors): 78.3 ms when every group
-// evaluated every survivor of the tile, 45.5 now; 1024^2 heterogeneous, 200,000
-// beams: 538 -> 173 ms; 128^3: 300 -> 116 ms.
+// triples) with the seeds' MUFU work beside it; measured 55 % (512^2), 51 % (1024^2
+// heterogeneous) and 59 % (128^3) of that pipe's cycles, the rest in pass barriers and latency.  512^2
+// homogeneous (65,536 coefficients, 2,414 times, 2,044 sensors): 78.3 ms when every
+// group evaluated every survivor of the tile, 46.7 now (45.5 with four beams' values
+// added before each compensated addition instead of two); 1024^2 heterogeneous,
+// 200,000 beams: 538 -> 168 ms; 128^3: 300 -> 116 ms.
 template <int D, bool PERIODIC, bool TRAJ>
 __global__ void __launch_bounds__(THREADS, 2)
 fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom, const TileInfo<D> *tiles, const int32_t *offs,
@@ -1548,8 +1549,8 @@ fwd32_kernel(ProbArgs P, BeamArgs B, const Cull<D> *cull, const HomBeam<D> *hom,
 // pass).  The item then writes every accumulator (zeros included) to
 // part[tt][slot], and reduce_parts_kernel sums part over the time tiles in
 // order.  Bound: as the forward, with more time at the pass barriers (FMA pipe
-// 43-45 %).  512^2: 86.4 -> 54.1 ms; 1024^2 heterogeneous 576 -> 195 ms; 128^3 504 ->
-// 151 ms.  Each partial has one writer and every sum has a fixed order, so the
+// 44-49 %).  512^2: 86.4 -> 54.2 ms; 1024^2 heterogeneous 576 -> 185 ms; 128^3 504 ->
+// 147 ms.  Each partial has one writer and every sum has a fixed order, so the
 // result is bit-identical between runs; the work counter only hands out items.
 template <int D, bool TRAJ>
 struct AdjRange {
