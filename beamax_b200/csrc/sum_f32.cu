@@ -789,7 +789,8 @@ __device__ __forceinline__ unsigned reached_mask(const Rec<D> &r, const TileGrou
         const float Bg = bilin2<D>(r.p, e, Dl), Ag = quad<D>(r.p, e), C = bilin2<D>(r.p, h, e);
         // a run's smallest exponent: at the vertex, or (Ak not positive) at the end that
         // the chord of slope B + 15 Ak falls to
-        const float im = Ak > 0.0f ? __fdividef(-0.5f, Ak) : -1e18f;
+        // (finite also for a subnormal Ak: the factor 0 below would make infinity a NaN)
+        const float im = Ak > 0.0f ? fmaxf(__fdividef(-0.5f, Ak), -1e18f) : -1e18f;
         const float kn = (float)(GS - 1) * fminf(Ak, 0.0f) * im;
         const float lim = fmaf(2e-6f, fabsf(c0), thr);  // round-off of the expansion
         const int n = tg.n;

@@ -269,6 +269,16 @@ def test_records_that_change_from_time_to_time(change, nt, kind, d):
     _compare(_Records(rec, np.zeros(nb, bool), _positions(kind)), True)
 
 
+@pytest.mark.parametrize("curvature", [0.0, 1e-31, -1e-31, 1e-25])
+def test_records_whose_exponent_falls_along_the_run(curvature):
+    """An open box, chi = 25 - 1.5 k along a run: 25 at its first sensor, 2.5 at its
+    last, with a curvature at the edge of FP32's range or none."""
+    rec = _records(40, 70)
+    rec["x"][:] = np.array([30.0, 40.0]) * DX
+    rec["p"][:] = np.array([25.0 / (10 * DX) ** 2, -1.5 / (10 * DX * DX), curvature])
+    _compare(_Records(rec, np.ones(70, bool), _positions("run")), False)
+
+
 @pytest.mark.parametrize("compact", [False, True])
 @pytest.mark.parametrize("kind", ["line", "run", "short", "scattered"])
 def test_records_in_an_open_box(kind, compact):
