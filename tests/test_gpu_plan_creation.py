@@ -16,6 +16,7 @@ def test_a_plan_of_many_boxes_is_made_quickly():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     import beamax_b200 as bb
+    from beamax_b200 import _lib
 
     N = (65536,)
     wpt = bb.MSWPT(bb.DyadicDecomposition(3, N, (1024, 2048, 4096), (1,)), 2, "rectangular_mirror")
@@ -24,6 +25,8 @@ def test_a_plan_of_many_boxes_is_made_quickly():
     c = wpt.forward_device(x, scale=1.0, half_mask=False)  # the device and the libraries are up
     best = 1e9
     for _ in range(3):
+        for plan in wpt._plans.values():
+            _lib.lib().msgb_mswpt_destroy(plan)
         wpt._plans.clear()
         torch.cuda.synchronize()
         t = time.perf_counter()
