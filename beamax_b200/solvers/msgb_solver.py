@@ -774,6 +774,7 @@ class MSGBSolver:
             for tr, first, last in self._compact_integrate(pr, med, bs, lo, hi, domain, sensors, opts, dev, st,
                                                           status, keep=keep_last):
                 if first:
+                    ws = None  # the smaller buffer goes before the larger one is allocated
                     ws, nbytes = self._traj_workspace(dev, nbytes, self._limit_bytes(pr.nt, self._compact_widest))
                 with self._kernel_span("msgb_sum_fwd_f32_traj", cnt):
                     _lib.check(_lib.lib().msgb_sum_fwd_f32_traj(_lib.ref(pr), _lib.ref(bs), _lib.ref(tr),
